@@ -275,6 +275,41 @@ typedef struct PopePagedDecodeArgs {
   void* workspace; size_t workspace_bytes;
 } PopePagedDecodeArgs;
 
+/* ---- the embedding tables --------------------------------------------------------------------------
+ * Replaces the elementwise chains of PoPE.forward and AxialPoPE.forward, PoPE_pytorch/pope.py:125-147 and
+ * pope_nd.py:66-106, for integer lengths: positions of a sequence (axes = 1, dims[0] = its length) or of a
+ * row-major grid (dims[0] slowest; column 0 of `positions` holds the LAST, fastest dimension), each plus
+ * `offset`; freqs[p, c] = positions[p, axis(c)] * inv_freqs[axis(c)][c - first(axis)] where axis a owns
+ * width[a] consecutive features; bias_out = bias clamped to [-2 pi, 0].  All fp32, contiguous, written in one
+ * launch. */
+#define POPE_MAX_AXES 8
+#define POPE_BIAS_MIN -6.283185307179586f
+typedef struct PopeTableArgs {
+  uint32_t struct_bytes;
+  int32_t axes;                          /* 1 .. POPE_MAX_AXES */
+  int32_t dims[POPE_MAX_AXES];           /* grid sizes, product < 2^31 */
+  int32_t width[POPE_MAX_AXES];          /* features of position column a; their sum is r */
+  const float* inv_freqs[POPE_MAX_AXES]; /* width[a] values each */
+  float offset;
+  int32_t H;                             /* rows of bias */
+  const float* bias;                     /* (H, r), may be NULL */
+  float* positions;                      /* (n, axes) */
+  float* freqs;                          /* (n, r) */
+  float* inv_flat;                       /* (r), may be NULL together with axis_of */
+  int32_t* axis_of;                      /* (r) */
+  float* bias_out;                       /* (H, r), NULL with bias */
+} PopeTableArgs;
+
+/* Gradient of the clamp: grad_bias = grad where bias lies in [-2 pi, 0], else 0; n fp32 values. */
+typedef struct PopeClampBwdArgs {
+  uint32_t struct_bytes;
+  int32_t reserved0;
+  const float* bias;
+  const float* grad;
+  float* grad_bias;
+  int64_t n;
+} PopeClampBwdArgs;
+
 POPE_API int pope_b200_abi_version(void);
 POPE_API const char* pope_b200_status_str(int status);
 
@@ -310,6 +345,8 @@ POPE_API int pope_b200_apply_qk_fwd(const PopeApplyArgs* args, void* stream);
 POPE_API int pope_b200_apply_qk_bwd(const PopeApplyBwdArgs* args, void* stream);
 POPE_API int pope_b200_kv_append(const PopeKvAppendArgs* args, void* stream);
 POPE_API int pope_b200_attn_decode_paged(const PopePagedDecodeArgs* args, void* stream);
+POPE_API int pope_b200_table(const PopeTableArgs* args, void* stream);
+POPE_API int pope_b200_clamp_bwd(const PopeClampBwdArgs* args, void* stream);
 
 /* ---- attention forward for callers that cannot allocate -----------------------------------------
  * (No counterpart in the reference: its wrappers always allocate through torch.)

@@ -1,5 +1,6 @@
-"""ctypes binding of libpope_b200.so (the C ABI in include/pope_b200.h) and the autograd
-functions built on it.
+"""Binding of libpope_b200.so (the C ABI in include/pope_b200.h).  The operators and their autograd nodes are C++
+(csrc/torch_host.cpp, built as the extension module ``_host``), because their host time is what small calls cost;
+the ctypes mirror of the ABI serves the diagnostics and the allocation-free entry point.
 
 This is the seam where the reference re-points its two Triton imports
 (PoPE_pytorch/attention.py:21-26): ``similarity`` stands in for
@@ -110,9 +111,11 @@ class PagedDecodeArgs(C.Structure):
 EXPORTS = ("pope_b200_abi_version", "pope_b200_apply_qk_fwd", "pope_b200_apply_qk_bwd", "pope_b200_status_str", "pope_b200_last_path", "pope_b200_device_status",
            "pope_b200_clear_device_status", "pope_b200_selftest_bounded_wait",
            "pope_b200_workspace_bytes", "pope_b200_attn_fwd_noalloc", "pope_b200_kv_append", "pope_b200_attn_decode_paged",
+           "pope_b200_table", "pope_b200_clamp_bwd",
            "pope_b200_sim_fwd", "pope_b200_sim_bwd", "pope_b200_attn_fwd", "pope_b200_attn_bwd")
 
 _lib = None
+_host = None
 _load_error: Optional[str] = None
 
 
@@ -124,7 +127,8 @@ def _bind(lib):
     lib.pope_b200_workspace_bytes.restype = C.c_size_t
     lib.pope_b200_workspace_bytes.argtypes = [C.c_int, C.c_void_p]
     for name in ("pope_b200_sim_fwd", "pope_b200_sim_bwd", "pope_b200_attn_fwd", "pope_b200_attn_bwd",
-                 "pope_b200_apply_qk_fwd", "pope_b200_apply_qk_bwd", "pope_b200_kv_append", "pope_b200_attn_decode_paged"):
+                 "pope_b200_apply_qk_fwd", "pope_b200_apply_qk_bwd", "pope_b200_kv_append", "pope_b200_attn_decode_paged",
+                 "pope_b200_table", "pope_b200_clamp_bwd"):
         fn = getattr(lib, name)
         fn.restype = C.c_int
         fn.argtypes = [C.c_void_p, C.c_void_p]
@@ -141,7 +145,7 @@ def _bind(lib):
 
 def load_library():
     """dlopen the in-tree library once; raises RuntimeError when it is missing or stale."""
-    global _lib, _load_error
+    global _lib, _host, _load_error
     if _lib is not None:
         return _lib
     if not os.path.exists(LIB_PATH):
@@ -151,8 +155,20 @@ def load_library():
         lib = _bind(C.CDLL(LIB_PATH))
     except AttributeError as exc:     # a symbol of the current header is missing: the build is stale
         raise RuntimeError(f"{LIB_PATH} is stale ({exc}); rebuild it with `python -m pope_pytorch_b200.build`") from exc
-    _lib = lib
+    try:
+        from . import _host as host
+    except ImportError as exc:
+        raise RuntimeError(f"the extension module pope_pytorch_b200._host cannot be loaded ({exc}); "
+                           "rebuild it with `python -m pope_pytorch_b200.build`") from exc
+    _lib, _host = lib, host
     return lib
+
+
+def _ops():
+    """The extension module; raises RuntimeError when it or the library is missing."""
+    if _host is None:
+        load_library()
+    return _host
 
 
 def is_available() -> bool:
@@ -192,9 +208,8 @@ def _check(rc: int, what: str) -> None:
         raise RuntimeError(f"{what} failed: {msg} (status {rc})")
 
 
-# What a call costs on the host matters for the small shapes (a (2, 8, 1024, 64) forward is 29 us of GPU time): the
-# raw stream handle and the current device come from torch's C bindings directly, and the device guard is entered only
-# when the tensors live on another device than the current one.
+# For the calls that stay on ctypes: the raw stream handle and the current device come from torch's C bindings
+# directly, and the device guard is entered only when the tensors live on another device than the current one.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _get_device = getattr(torch._C, "_cuda_getDevice", None)
 
@@ -254,9 +269,14 @@ def _prep_embed(freqs: torch.Tensor, bias: torch.Tensor, nk: int, r: int):
     return freqs, bias
 
 
+def _attached(freqs):
+    """The factors riding on a table built by PoPE / AxialPoPE, unchecked (the binding looks at them)."""
+    return getattr(freqs, "_pope_factored", None)
+
+
 def _factors_of(freqs):
     """(positions, inv_freqs, axis_of) riding on a table built by PoPE / AxialPoPE, when usable as is."""
-    f = getattr(freqs, "_pope_factored", None)
+    f = _attached(freqs)
     if f is None or freqs.ndim != 2:
         return None
     pos, inv, axis = f
@@ -291,17 +311,16 @@ def _workspace(op: int, args, device) -> Optional[torch.Tensor]:
     return ws
 
 
-def _validate(q, k, freqs, bias):
-    if not (q.is_cuda and k.is_cuda):
-        raise RuntimeError("the native PoPE kernels need CUDA tensors")
-    if q.dtype not in _DTYPES or k.dtype != q.dtype:
-        raise TypeError(f"q and k must share a dtype among fp32/bf16/fp16, got {q.dtype}, {k.dtype}")
-    assert q.shape[1] % k.shape[1] == 0, "query heads must be a multiple of key heads"
-    assert q.shape[2] <= k.shape[2] and freqs.shape[-1] <= q.shape[-1]
+def _mask_u8(mask: Optional[torch.Tensor]):
+    if mask is None:
+        return None
+    m = mask if mask.dtype in (torch.bool, torch.uint8) else (mask != 0)
+    return m.view(torch.uint8) if m.dtype == torch.bool else m
 
 
 # ----------------------------------------------------------------------------------------------
-# the stand-alone transform
+# the operators (csrc/torch_host.cpp): head-first (b,h,n,d) tensors or views; with ``seq_first`` the
+# differentiable ones take (b,n,h,d)
 # ----------------------------------------------------------------------------------------------
 
 def apply_qk_supported(q, k, freqs, bias) -> bool:
@@ -313,191 +332,53 @@ def apply_qk_supported(q, k, freqs, bias) -> bool:
             and freqs.ndim in (2, 3, 4) and bias.ndim == 2 and is_available())
 
 
-class _ApplyQK(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, freqs, bias):
-        lib = load_library()
-        r = freqs.shape[-1]
-        qc, kc = _inner_contig(q), _inner_contig(k)
-        fr, bi = _prep_embed(freqs, bias, k.shape[2], r)
-        q_out = torch.empty(*q.shape[:-1], q.shape[-1] + r, dtype=torch.float32, device=q.device)
-        k_out = torch.empty(*k.shape[:-1], k.shape[-1] + r, dtype=torch.float32, device=q.device)
-        a = ApplyArgs(C.sizeof(ApplyArgs), 0, _shape(qc, kc, r), _embed_struct(fr, bi, r),
-                      qc.data_ptr(), _s3(qc), kc.data_ptr(), _s3(kc), q_out.data_ptr(), _s3(q_out), k_out.data_ptr(), _s3(k_out))
-        with _on_device(q.device):
-            _check(lib.pope_b200_apply_qk_fwd(C.addressof(a), _stream_ptr(q)), "pope_b200_apply_qk_fwd")
-        ctx.save_for_backward(qc, kc, fr, bi)
-        ctx.shapes = (freqs.shape, bias.shape, freqs.dtype, bias.dtype)
-        return q_out, k_out
-
-    @staticmethod
-    def backward(ctx, dq_out, dk_out):
-        lib = load_library()
-        q, k, freqs, bias = ctx.saved_tensors
-        r = freqs.shape[-1]
-        dq_out, dk_out = dq_out.contiguous().float(), dk_out.contiguous().float()
-        dq, dk = torch.empty_like(q), torch.empty_like(k)
-        need_df, need_db = ctx.needs_input_grad[2] and r > 0, ctx.needs_input_grad[3] and r > 0
-        dfreqs = torch.zeros(freqs.shape, dtype=torch.float32, device=q.device) if need_df else None
-        dbias = torch.zeros(bias.shape, dtype=torch.float32, device=q.device) if need_db else None
-        a = ApplyBwdArgs(C.sizeof(ApplyBwdArgs), 0, _shape(q, k, r), _embed_struct(freqs, bias, r),
-                         q.data_ptr(), _s3(q), k.data_ptr(), _s3(k), dq_out.data_ptr(), _s3(dq_out), dk_out.data_ptr(), _s3(dk_out),
-                         dq.data_ptr(), _s3(dq), dk.data_ptr(), _s3(dk),
-                         dfreqs.data_ptr() if dfreqs is not None else None,
-                         _freq_strides(dfreqs) if dfreqs is not None else Stride3(0, 0, 0),
-                         dbias.data_ptr() if dbias is not None else None, dbias.stride(0) if dbias is not None else 0)
-        with _on_device(q.device):
-            _check(lib.pope_b200_apply_qk_bwd(C.addressof(a), _stream_ptr(q)), "pope_b200_apply_qk_bwd")
-        fshape, bshape, fdt, bdt = ctx.shapes
-        if ctx.needs_input_grad[2] and dfreqs is None:
-            dfreqs = torch.zeros(fshape, dtype=fdt, device=q.device)
-        if ctx.needs_input_grad[3] and dbias is None:
-            dbias = torch.zeros(bshape, dtype=bdt, device=q.device)
-        return dq, dk, None if dfreqs is None else dfreqs.to(fdt), None if dbias is None else dbias.to(bdt)
-
-
 def apply_qk(q, k, freqs, bias):
     """Differentiable fused transform on head-first (b,h,n,d) tensors -> fp32 (q', k') in the
     reference's interleaved layout."""
-    return _ApplyQK.apply(q, k, freqs, bias)
+    return _ops().apply_qk(q, k, freqs, bias)
 
-
-# ----------------------------------------------------------------------------------------------
-# similarity
-# ----------------------------------------------------------------------------------------------
 
 def sim_forward(q, k, freqs, bias, allow_tf32=True, factors=None) -> torch.Tensor:
     """q (b,h,nq,d), k (b,hk,nk,d) head-first views -> sim (b,h,nq,nk) in q's dtype."""
-    lib = load_library()
-    r = freqs.shape[-1]
-    _validate(q, k, freqs, bias)
-    q, k = _inner_contig(q), _inner_contig(k)
-    factors = factors or _factors_of(freqs)
-    freqs, bias = _prep_embed(freqs, bias, k.shape[2], r)
-    sim = torch.empty(q.shape[0], q.shape[1], q.shape[2], k.shape[2], dtype=q.dtype, device=q.device)
-    a = SimArgs(C.sizeof(SimArgs), int(allow_tf32), _shape(q, k, r), _embed_struct(freqs, bias, r, factors),
-                q.data_ptr(), _s3(q), k.data_ptr(), _s3(k), sim.data_ptr(), _s3(sim), None, 0)
-    ws = _workspace(OP_SIM_FWD, a, q.device)
-    with _on_device(q.device):
-        _check(lib.pope_b200_sim_fwd(C.addressof(a), _stream_ptr(q)), "pope_b200_sim_fwd")
-    del ws
-    return sim
+    return _ops().sim_forward(q, k, freqs, bias, allow_tf32, factors or _attached(freqs))
 
 
 def sim_backward(dsim, q, k, freqs, bias, need_dfreqs, need_dbias, allow_tf32=True):
-    lib = load_library()
-    r = freqs.shape[-1]
-    q, k, dsim = _inner_contig(q), _inner_contig(k), _inner_contig(dsim)
-    freqs, bias = _prep_embed(freqs, bias, k.shape[2], r)
-    dq, dk = torch.empty_like(q), torch.empty_like(k)
-    dfreqs = torch.zeros(freqs.shape, dtype=torch.float32, device=q.device) if (need_dfreqs and r > 0) else None
-    dbias = torch.zeros(bias.shape, dtype=torch.float32, device=q.device) if (need_dbias and r > 0) else None
-    a = SimBwdArgs(C.sizeof(SimBwdArgs), int(allow_tf32), _shape(q, k, r), _embed_struct(freqs, bias, r),
-                   q.data_ptr(), _s3(q), k.data_ptr(), _s3(k), dsim.data_ptr(), _s3(dsim),
-                   dq.data_ptr(), _s3(dq), dk.data_ptr(), _s3(dk),
-                   dfreqs.data_ptr() if dfreqs is not None else None,
-                   _freq_strides(dfreqs) if dfreqs is not None else Stride3(0, 0, 0),
-                   dbias.data_ptr() if dbias is not None else None,
-                   dbias.stride(0) if dbias is not None else 0, None, 0)
-    ws = _workspace(OP_SIM_BWD, a, q.device)
-    with _on_device(q.device):
-        _check(lib.pope_b200_sim_bwd(C.addressof(a), _stream_ptr(q)), "pope_b200_sim_bwd")
-    del ws
-    if need_dfreqs and dfreqs is None:
-        dfreqs = torch.zeros_like(freqs)
-    if need_dbias and dbias is None:
-        dbias = torch.zeros_like(bias)
-    return dq, dk, dfreqs, dbias
+    return _ops().sim_backward(dsim, q, k, freqs, bias, need_dfreqs, need_dbias, allow_tf32)
 
 
-class _Similarity(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, freqs, bias, allow_tf32):
-        ctx.save_for_backward(q, k, freqs, bias)
-        ctx.allow_tf32 = allow_tf32
-        return sim_forward(q, k, freqs, bias, allow_tf32)
-
-    @staticmethod
-    def backward(ctx, dsim):
-        q, k, freqs, bias = ctx.saved_tensors
-        dq, dk, dfreqs, dbias = sim_backward(dsim.to(q.dtype), q, k, freqs, bias,
-                                             ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.allow_tf32)
-        if dfreqs is not None:
-            dfreqs = dfreqs.to(freqs.dtype)
-        if dbias is not None:
-            dbias = dbias.to(bias.dtype)
-        return dq, dk, dfreqs, dbias, None
-
-
-def similarity(q, k, freqs, bias, allow_tf32=True):
-    """Differentiable fused similarity on head-first tensors."""
-    return _Similarity.apply(q, k, freqs, bias, allow_tf32)
-
-
-# ----------------------------------------------------------------------------------------------
-# attention
-# ----------------------------------------------------------------------------------------------
-
-def _mask_u8(mask: Optional[torch.Tensor]):
-    if mask is None:
-        return None
-    m = mask if mask.dtype in (torch.bool, torch.uint8) else (mask != 0)
-    return m.view(torch.uint8) if m.dtype == torch.bool else m
+def similarity(q, k, freqs, bias, allow_tf32=True, seq_first=False):
+    """Differentiable fused similarity."""
+    return _ops().similarity(q, k, freqs, bias, allow_tf32, _attached(freqs), seq_first)
 
 
 def attn_forward(q, k, v, freqs, bias, mask, causal, scale, factors=None):
-    """Head-first VIEWS (b,h,n,d) of any stride with contiguous features -> (out, lse)."""
-    lib = load_library()
-    r = freqs.shape[-1]
-    _validate(q, k, freqs, bias)
-    q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
-    factors = factors or _factors_of(freqs)
-    freqs, bias = _prep_embed(freqs, bias, k.shape[2], r)
-    # the output takes the memory layout of q, so a (b,n,h,d) caller gets a (b,n,h,d)-contiguous result
-    out = torch.empty_like(q)
-    lse = torch.empty(q.shape[0], q.shape[1], q.shape[2], dtype=torch.float32, device=q.device)
-    m8 = _mask_u8(mask)
-    a = AttnArgs(C.sizeof(AttnArgs), int(causal), float(scale), 0, _shape(q, k, r), _embed_struct(freqs, bias, r, factors),
-                 q.data_ptr(), _s3(q), k.data_ptr(), _s3(k), v.data_ptr(), _s3(v), out.data_ptr(), _s3(out),
-                 lse.data_ptr(), m8.data_ptr() if m8 is not None else None,
-                 m8.stride(0) if m8 is not None else 0, m8.stride(1) if m8 is not None else 0, None, 0)
-    ws = _workspace(OP_ATTN_FWD, a, q.device)
-    with _on_device(q.device):
-        _check(lib.pope_b200_attn_fwd(C.addressof(a), _stream_ptr(q)), "pope_b200_attn_fwd")
-    del ws
-    return out, lse
+    """Head-first VIEWS (b,h,n,d) of any stride with contiguous features -> (out, lse).  The output takes the memory
+    layout of q, so a (b,n,h,d) caller gets a (b,n,h,d)-contiguous result."""
+    return _ops().attn_forward(q, k, v, freqs, bias, mask, causal, scale, factors or _attached(freqs))
 
 
 def attn_backward(dout, q, k, v, out, lse, freqs, bias, mask, causal, scale, need_dfreqs, need_dbias, factors=None):
-    lib = load_library()
-    r = freqs.shape[-1]
-    q, k, v, out, dout = (_inner_contig(t) for t in (q, k, v, out, dout))
-    factors = factors or _factors_of(freqs)
-    freqs, bias = _prep_embed(freqs, bias, k.shape[2], r)
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    dfreqs = torch.zeros(freqs.shape, dtype=torch.float32, device=q.device) if (need_dfreqs and r > 0) else None
-    dbias = torch.zeros(bias.shape, dtype=torch.float32, device=q.device) if (need_dbias and r > 0) else None
-    m8 = _mask_u8(mask)
-    a = AttnBwdArgs(C.sizeof(AttnBwdArgs), int(causal), float(scale), 0, _shape(q, k, r),
-                    _embed_struct(freqs, bias, r, factors),
-                    q.data_ptr(), _s3(q), k.data_ptr(), _s3(k), v.data_ptr(), _s3(v), out.data_ptr(), _s3(out),
-                    dout.data_ptr(), _s3(dout), lse.data_ptr(),
-                    m8.data_ptr() if m8 is not None else None,
-                    m8.stride(0) if m8 is not None else 0, m8.stride(1) if m8 is not None else 0,
-                    dq.data_ptr(), _s3(dq), dk.data_ptr(), _s3(dk), dv.data_ptr(), _s3(dv),
-                    dfreqs.data_ptr() if dfreqs is not None else None,
-                    _freq_strides(dfreqs) if dfreqs is not None else Stride3(0, 0, 0),
-                    dbias.data_ptr() if dbias is not None else None,
-                    dbias.stride(0) if dbias is not None else 0, None, 0)
-    ws = _workspace(OP_ATTN_BWD, a, q.device)
-    with _on_device(q.device):
-        _check(lib.pope_b200_attn_bwd(C.addressof(a), _stream_ptr(q)), "pope_b200_attn_bwd")
-    del ws
-    if need_dfreqs and dfreqs is None:
-        dfreqs = torch.zeros_like(freqs)
-    if need_dbias and dbias is None:
-        dbias = torch.zeros_like(bias)
-    return dq, dk, dv, dfreqs, dbias
+    return _ops().attn_backward(dout, q, k, v, out, lse, freqs, bias, mask, causal, scale, need_dfreqs, need_dbias,
+                                factors or _attached(freqs))
+
+
+def flash_attn(q, k, v, freqs=None, bias=None, mask=None, causal=False, softmax_scale=None, seq_first=False):
+    """Differentiable fused PoPE attention.  Without ``freqs`` / ``bias`` this is plain softmax attention, as the
+    seam it replaces behaves with ``HAS_POPE`` off (PoPE_pytorch/triton_pope_flash_attn.py:364-373): the kernels
+    run with zero rotated dims."""
+    scale = q.shape[-1] ** -0.5 if softmax_scale is None else softmax_scale
+    if freqs is None or bias is None:
+        head, row = (2, 1) if seq_first else (1, 2)
+        freqs = torch.empty(k.shape[row], 0, dtype=torch.float32, device=q.device)
+        bias = torch.empty(k.shape[head], 0, dtype=torch.float32, device=q.device)
+    return _ops().flash_attn(q, k, v, freqs, bias, mask, causal, scale, _attached(freqs), seq_first)
+
+
+def embed_table(bias, inv_freqs, dims, offset=0.0):
+    """(freqs, clamped bias, positions[, flat inverse frequencies, axis of a feature]) of the sequence or grid
+    ``dims`` in one launch, differentiable in ``bias``; None when the module's tensors are not plain fp32 CUDA ones."""
+    return _ops().table(bias, inv_freqs, dims, offset)
 
 
 NOALLOC_MAX_SCRATCH = 16 << 20
@@ -521,36 +402,3 @@ def attn_forward_noalloc(q, k, v, freqs, bias, mask, causal, scale, out, lse):
     with _on_device(q.device):
         _check(lib.pope_b200_attn_fwd_noalloc(C.addressof(a), _stream_ptr(q)), "pope_b200_attn_fwd_noalloc")
     return out, lse
-
-
-class _FlashAttn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, freqs, bias, mask, causal, scale):
-        ctx.factors = _factors_of(freqs)        # saved tensors come back as new objects: keep the factors here
-        out, lse = attn_forward(q, k, v, freqs, bias, mask, causal, scale, ctx.factors)
-        ctx.save_for_backward(q, k, v, freqs, bias, out, lse)
-        ctx.mask, ctx.causal, ctx.scale = mask, causal, scale
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        q, k, v, freqs, bias, out, lse = ctx.saved_tensors
-        dq, dk, dv, dfreqs, dbias = attn_backward(dout.to(q.dtype), q, k, v, out, lse, freqs, bias, ctx.mask,
-                                                  ctx.causal, ctx.scale,
-                                                  ctx.needs_input_grad[3], ctx.needs_input_grad[4], ctx.factors)
-        if dfreqs is not None:
-            dfreqs = dfreqs.to(freqs.dtype)
-        if dbias is not None:
-            dbias = dbias.to(bias.dtype)
-        return dq, dk, dv, dfreqs, dbias, None, None, None
-
-
-def flash_attn(q, k, v, freqs=None, bias=None, mask=None, causal=False, softmax_scale=None):
-    """Differentiable fused PoPE attention on head-first (b,h,n,d) views.  Without ``freqs`` /
-    ``bias`` this is plain softmax attention, as the seam it replaces behaves with ``HAS_POPE``
-    off (PoPE_pytorch/triton_pope_flash_attn.py:364-373): the kernels run with zero rotated dims."""
-    scale = q.shape[-1] ** -0.5 if softmax_scale is None else softmax_scale
-    if freqs is None or bias is None:
-        freqs = torch.empty(k.shape[2], 0, dtype=torch.float32, device=q.device)
-        bias = torch.empty(k.shape[1], 0, dtype=torch.float32, device=q.device)
-    return _FlashAttn.apply(q, k, v, freqs, bias, mask, causal, scale)

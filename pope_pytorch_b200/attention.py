@@ -49,8 +49,7 @@ def compute_attn_similarity(q, k, pope, allow_tf32=True, head_dimension_at_first
     assert head_dim in {32, 48, 64, 128, 256}, f"head_dim {head_dim} not in common sizes"
 
     if q.is_cuda and k.is_cuda and freqs.is_cuda and bias.is_cuda:
-        q, k = _head_first(q, head_dimension_at_first), _head_first(k, head_dimension_at_first)
-        return _native.similarity(q, k, freqs, bias, allow_tf32)
+        return _native.similarity(q, k, freqs, bias, allow_tf32, not head_dimension_at_first)
     return compute_attn_similarity_non_fused(q, k, pope, head_dimension_at_first=head_dimension_at_first)
 
 
@@ -67,9 +66,7 @@ def flash_attn_with_pope(q, k, v, pos_emb=None, mask=None, causal=False, softmax
     freqs, bias = pos_emb
 
     if fused:
-        qh, kh, vh = (_head_first(t, head_dimension_at_first) for t in (q, k, v))
-        out = _native.flash_attn(qh, kh, vh, freqs, bias, mask=mask, causal=causal, softmax_scale=softmax_scale)
-        return _head_first(out, head_dimension_at_first)
+        return _native.flash_attn(q, k, v, freqs, bias, mask, causal, softmax_scale, not head_dimension_at_first)
 
     # pure-PyTorch composition (reference: attention.py:106-145)
     qh, kh, vh = (_head_first(t, head_dimension_at_first) for t in (q, k, v))

@@ -257,4 +257,27 @@ int pope_b200_attn_decode_paged(const PopePagedDecodeArgs* a, void* stream) {
   return POPE_OK;
 }
 
+int pope_b200_table(const PopeTableArgs* a, void* stream) {
+  if (!a || a->struct_bytes != sizeof(PopeTableArgs) || a->axes < 1 || a->axes > POPE_MAX_AXES) return POPE_ERR_BAD_ARG;
+  int64_t n = 1, r = 0;
+  for (int i = 0; i < a->axes; ++i) {
+    if (a->dims[i] < 0 || a->width[i] < 0 || (a->width[i] > 0 && !a->inv_freqs[i])) return POPE_ERR_BAD_ARG;
+    n *= a->dims[i], r += a->width[i];
+    if (n > INT32_MAX) return POPE_ERR_UNSUPPORTED;
+  }
+  if (n * r > 0 && (!a->positions || !a->freqs)) return POPE_ERR_BAD_ARG;
+  if ((a->inv_flat != nullptr) != (a->axis_of != nullptr) || (a->bias && (!a->bias_out || a->H <= 0))) return POPE_ERR_BAD_ARG;
+  int rc = check_device();
+  if (rc != POPE_OK) return rc;
+  return pope::pope_table(*a, static_cast<cudaStream_t>(stream)) == cudaSuccess ? POPE_OK : POPE_ERR_CUDA;
+}
+
+int pope_b200_clamp_bwd(const PopeClampBwdArgs* a, void* stream) {
+  if (!a || a->struct_bytes != sizeof(PopeClampBwdArgs) || a->n < 0) return POPE_ERR_BAD_ARG;
+  if (a->n > 0 && (!a->bias || !a->grad || !a->grad_bias)) return POPE_ERR_BAD_ARG;
+  int rc = check_device();
+  if (rc != POPE_OK) return rc;
+  return pope::pope_clamp_bwd(*a, static_cast<cudaStream_t>(stream)) == cudaSuccess ? POPE_OK : POPE_ERR_CUDA;
+}
+
 }  // extern "C"

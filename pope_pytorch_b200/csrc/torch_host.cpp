@@ -1,0 +1,433 @@
+// torch binding of libpope_b200.so: output and workspace allocation, argument structs and the autograd nodes.
+//
+// What a call costs on the host decides the small shapes.  The same layer written in Python over ctypes took 45 us per
+// (2, 8, 1024, 64) forward whose kernels take 26 us and, with its backward in a Python autograd node on the engine's thread,
+// 351 us per (3, 8 / 2, 777, 64) training step whose kernels take 159 us; here they take 27 and 148 us.  The kernels themselves stay behind
+// the C ABI (include/pope_b200.h): this file only fills its structs.  No arithmetic happens here and nothing is kept from one
+// call to the next.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <cmath>
+#include <tuple>
+
+#include "../../include/pope_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using std::optional;
+
+namespace {
+
+using Factors = optional<std::tuple<Tensor, Tensor, optional<Tensor>>>;   // positions, inverse frequencies, axis of a feature
+
+[[noreturn]] void assertion(const char* what) {   // (the GIL is held: called from the binding layer only)
+  PyErr_SetString(PyExc_AssertionError, what);
+  throw py::error_already_set();
+}
+
+void check(int rc, const char* what) {
+  if (rc != POPE_OK) TORCH_CHECK(false, what, " failed: ", pope_b200_status_str(rc), " (status ", rc, ")");
+}
+
+int dtype_of(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return POPE_F32;
+    case at::kBFloat16: return POPE_BF16;
+    case at::kHalf: return POPE_F16;
+    default: return -1;
+  }
+}
+
+// (batch, head, row) strides of a (b, h, n, x) tensor or, with seq_first, of a (b, n, h, x) one; the innermost stride is 1
+PopeStride3 s3(const Tensor& t, bool seq_first = false) { return {t.stride(0), t.stride(seq_first ? 2 : 1), t.stride(seq_first ? 1 : 2)}; }
+
+Tensor inner_contig(const Tensor& t) { return t.size(-1) <= 1 || t.stride(-1) == 1 ? t : t.contiguous(); }
+
+Tensor fp32_rows(const Tensor& t) { return inner_contig(t.scalar_type() == at::kFloat ? t : t.to(at::kFloat)); }
+
+// (batch, head, row) strides with 0 = broadcast; a 4-D table is (b, h, n, r), as in apply_pope_to_qk and the reference's
+// similarity (PoPE_pytorch/pope.py:53-56, triton_pope.py:267-272)
+PopeStride3 freq_strides(const Tensor& f) {
+  switch (f.dim()) {
+    case 2: return {0, 0, f.stride(0)};
+    case 3: return {f.size(0) > 1 ? f.stride(0) : 0, 0, f.stride(1)};
+    case 4: return {f.size(0) > 1 ? f.stride(0) : 0, f.size(1) > 1 ? f.stride(1) : 0, f.stride(2)};
+    default: TORCH_CHECK_VALUE(false, "freqs must have 2, 3 or 4 dimensions");
+  }
+}
+
+// the factors of a table built by PoPE / AxialPoPE, when they are usable as they are
+bool factors_usable(const Factors& f, const Tensor& freqs) {
+  if (!f || freqs.dim() != 2) return false;
+  const auto& [pos, inv, axis] = *f;
+  return pos.device() == freqs.device() && inv.device() == freqs.device() && pos.scalar_type() == at::kFloat &&
+         inv.scalar_type() == at::kFloat && pos.size(0) == freqs.size(0) && inv.numel() == freqs.size(1) && pos.stride(-1) == 1 &&
+         inv.is_contiguous() &&
+         (!axis || (axis->device() == freqs.device() && axis->scalar_type() == at::kInt && axis->is_contiguous()));
+}
+
+PopeEmbed embed_of(const Tensor& freqs, const Tensor& bias, int r, const Factors& f = std::nullopt) {
+  PopeEmbed e = {};
+  if (r == 0) return e;
+  e.freqs = freqs.const_data_ptr<float>(), e.sf = freq_strides(freqs);
+  e.bias = bias.const_data_ptr<float>(), e.bias_stride_h = bias.stride(0);
+  if (factors_usable(f, freqs)) {
+    const auto& [pos, inv, axis] = *f;
+    e.positions = pos.const_data_ptr<float>(), e.pos_stride_n = pos.dim() == 2 ? pos.stride(0) : 1;
+    e.inv_freqs = inv.const_data_ptr<float>();
+    e.axis_of = axis ? axis->const_data_ptr<int32_t>() : nullptr;
+  }
+  return e;
+}
+
+PopeShape shape_of(const Tensor& q, const Tensor& k, int r, bool seq_first = false) {
+  const int h = seq_first ? 2 : 1, n = seq_first ? 1 : 2;
+  return {(int32_t)q.size(0), (int32_t)q.size(h), (int32_t)k.size(h), (int32_t)q.size(n), (int32_t)k.size(n), (int32_t)q.size(3), r, dtype_of(q)};
+}
+
+template <typename Args>
+Tensor workspace(int op, Args& a, const Tensor& like) {
+  const size_t need = pope_b200_workspace_bytes(op, &a);
+  if (need == 0) return Tensor();
+  Tensor ws = at::empty({(int64_t)need}, like.options().dtype(at::kByte));
+  a.workspace = ws.mutable_data_ptr(), a.workspace_bytes = need;
+  return ws;
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// the checks every operator makes on q, k and the pair (freqs, bias); GIL held
+void validate(const Tensor& q, const Tensor& k, const Tensor& freqs, bool seq_first) {
+  if (!(q.is_cuda() && k.is_cuda())) TORCH_CHECK(false, "the native PoPE kernels need CUDA tensors");
+  if (dtype_of(q) < 0 || k.scalar_type() != q.scalar_type())
+    TORCH_CHECK_TYPE(false, "q and k must share a dtype among fp32/bf16/fp16, got ", q.scalar_type(), ", ", k.scalar_type());
+  TORCH_CHECK(q.dim() == 4 && k.dim() == 4, "q and k must have 4 dimensions");
+  const int ha = seq_first ? 2 : 1, na = seq_first ? 1 : 2;
+  if (q.size(ha) % k.size(ha) != 0) assertion("query heads must be a multiple of key heads");
+  if (q.size(na) > k.size(na) || freqs.size(-1) > q.size(-1)) assertion("queries must not outnumber keys, nor rotated features the head dim");
+  if (freqs.dim() < 2 || (freqs.size(-2) != k.size(na) && freqs.size(-1) != 0)) assertion("freqs must have one row per key position");
+}
+
+// ---- attention -------------------------------------------------------------------------------------------------
+struct Mask {
+  Tensor keep;   // bool or uint8
+  explicit Mask(const optional<Tensor>& m) {
+    if (!m || !m->defined()) return;
+    keep = m->scalar_type() == at::kBool || m->scalar_type() == at::kByte ? *m : m->ne(0);
+  }
+  template <typename Args>
+  void put(Args& a) const {
+    if (!keep.defined()) return;
+    a.mask = static_cast<const uint8_t*>(keep.const_data_ptr()), a.mask_stride_b = keep.stride(0), a.mask_stride_n = keep.stride(1);
+  }
+};
+
+// tensors of any stride with contiguous features -> (out in q's memory layout, lse (b, h, n_q))
+std::tuple<Tensor, Tensor> attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& freqs_, const Tensor& bias_,
+                                        const optional<Tensor>& mask, bool causal, double scale, const Factors& factors, bool sf) {
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = inner_contig(q_), k = inner_contig(k_), v = inner_contig(v_), freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
+  Tensor out = at::empty_like(q), lse = at::empty({q.size(0), q.size(sf ? 2 : 1), q.size(sf ? 1 : 2)}, q.options().dtype(at::kFloat));
+  const int r = (int)freqs.size(-1);
+  const Mask m(mask);
+  PopeAttnArgs a = {};
+  a.struct_bytes = sizeof(a), a.causal = causal, a.softmax_scale = (float)scale;
+  a.shape = shape_of(q, k, r, sf), a.embed = embed_of(freqs, bias, r, factors);
+  a.q = q.const_data_ptr(), a.sq = s3(q, sf), a.k = k.const_data_ptr(), a.sk = s3(k, sf), a.v = v.const_data_ptr(), a.sv = s3(v, sf);
+  a.out = out.mutable_data_ptr(), a.so = s3(out, sf), a.lse = lse.mutable_data_ptr<float>();
+  m.put(a);
+  const Tensor ws = workspace(POPE_OP_ATTN_FWD, a, q);
+  check(pope_b200_attn_fwd(&a, stream_of(q)), "pope_b200_attn_fwd");
+  return {out, lse};
+}
+
+struct Grads {
+  Tensor dq, dk, dv, dfreqs, dbias;
+};
+
+template <typename Args>
+void put_phase_grads(Args& a, Grads& g, const Tensor& freqs, const Tensor& bias, bool need_df, bool need_db) {
+  // (accumulators of the kernels, and the result where nothing is rotated: zero-filled either way)
+  if (need_df) g.dfreqs = at::zeros(freqs.sizes(), freqs.options().dtype(at::kFloat));
+  if (need_db) g.dbias = at::zeros(bias.sizes(), bias.options().dtype(at::kFloat));
+  if (freqs.size(-1) == 0) return;
+  if (need_df) a.dfreqs = g.dfreqs.mutable_data_ptr<float>(), a.sdf = freq_strides(g.dfreqs);
+  if (need_db) a.dbias = g.dbias.mutable_data_ptr<float>(), a.dbias_stride_h = g.dbias.stride(0);
+}
+
+Grads attn_backward(const Tensor& dout_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& out_, const Tensor& lse,
+                    const Tensor& freqs_, const Tensor& bias_, const optional<Tensor>& mask, bool causal, double scale, bool need_df,
+                    bool need_db, const Factors& factors, bool sf) {
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = inner_contig(q_), k = inner_contig(k_), v = inner_contig(v_), out = inner_contig(out_), dout = inner_contig(dout_);
+  const Tensor freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
+  const int r = (int)freqs.size(-1);
+  Grads g{at::empty_like(q), at::empty_like(k), at::empty_like(v), Tensor(), Tensor()};
+  const Mask m(mask);
+  PopeAttnBwdArgs a = {};
+  a.struct_bytes = sizeof(a), a.causal = causal, a.softmax_scale = (float)scale;
+  a.shape = shape_of(q, k, r, sf), a.embed = embed_of(freqs, bias, r, factors);
+  a.q = q.const_data_ptr(), a.sq = s3(q, sf), a.k = k.const_data_ptr(), a.sk = s3(k, sf), a.v = v.const_data_ptr(), a.sv = s3(v, sf);
+  a.out = out.const_data_ptr(), a.so = s3(out, sf), a.dout = dout.const_data_ptr(), a.sdo = s3(dout, sf), a.lse = lse.const_data_ptr<float>();
+  a.dq = g.dq.mutable_data_ptr(), a.sdq = s3(g.dq, sf), a.dk = g.dk.mutable_data_ptr(), a.sdk = s3(g.dk, sf);
+  a.dv = g.dv.mutable_data_ptr(), a.sdv = s3(g.dv, sf);
+  m.put(a);
+  put_phase_grads(a, g, freqs, bias, need_df, need_db);
+  const Tensor ws = workspace(POPE_OP_ATTN_BWD, a, q);
+  check(pope_b200_attn_bwd(&a, stream_of(q)), "pope_b200_attn_bwd");
+  return g;
+}
+
+// What a backward node keeps beside its saved tensors.  (The factors and the mask are inputs without gradients that the
+// caller does not write to between the passes, as the phase table itself.)
+struct Kept : torch::CustomClassHolder {
+  Factors factors;
+  optional<Tensor> mask;
+  bool causal = false, seq_first = false;
+  double scale = 1.0;
+};
+
+Tensor to_dtype_of(const Tensor& g, const Tensor& like) { return g.defined() ? g.to(like.scalar_type()) : g; }
+
+struct FlashAttn : torch::autograd::Function<FlashAttn> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs,
+                        const Tensor& bias, const c10::intrusive_ptr<Kept>& kept) {
+    auto [out, lse] = attn_forward(q, k, v, freqs, bias, kept->mask, kept->causal, kept->scale, kept->factors, kept->seq_first);
+    ctx->save_for_backward({q, k, v, freqs, bias, out, lse});
+    ctx->saved_data["kept"] = c10::IValue::make_capsule(kept);
+    return out;
+  }
+  static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad) {
+    const auto s = ctx->get_saved_variables();
+    const auto kept = c10::static_intrusive_pointer_cast<Kept>(ctx->saved_data["kept"].toCapsule());
+    Grads g = attn_backward(grad[0].to(s[0].scalar_type()), s[0], s[1], s[2], s[5], s[6], s[3], s[4], kept->mask, kept->causal, kept->scale,
+                            ctx->needs_input_grad(3), ctx->needs_input_grad(4), kept->factors, kept->seq_first);
+    return {g.dq, g.dk, g.dv, to_dtype_of(g.dfreqs, s[3]), to_dtype_of(g.dbias, s[4]), Tensor()};
+  }
+};
+
+template <typename... Ts>
+bool wants_graph(const Ts&... ts) {
+  return at::GradMode::is_enabled() && (ts.requires_grad() || ...);
+}
+
+Tensor flash_attn(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask,
+                  bool causal, double scale, const Factors& factors, bool seq_first) {
+  validate(q, k, freqs, seq_first);
+  py::gil_scoped_release nogil;
+  if (!wants_graph(q, k, v, freqs, bias)) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return std::get<0>(attn_forward(q, k, v, freqs, bias, mask, causal, scale, factors, seq_first));
+  }
+  auto kept = c10::make_intrusive<Kept>();
+  kept->factors = factors, kept->mask = mask, kept->causal = causal, kept->seq_first = seq_first, kept->scale = scale;
+  return FlashAttn::apply(q, k, v, freqs, bias, kept);
+}
+
+// ---- similarity ------------------------------------------------------------------------------------------------
+Tensor sim_forward(const Tensor& q_, const Tensor& k_, const Tensor& freqs_, const Tensor& bias_, bool allow_tf32, const Factors& factors, bool sf) {
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = inner_contig(q_), k = inner_contig(k_), freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
+  const int r = (int)freqs.size(-1);
+  Tensor sim = at::empty({q.size(0), q.size(sf ? 2 : 1), q.size(sf ? 1 : 2), k.size(sf ? 1 : 2)}, q.options());
+  PopeSimArgs a = {};
+  a.struct_bytes = sizeof(a), a.allow_tf32 = allow_tf32;
+  a.shape = shape_of(q, k, r, sf), a.embed = embed_of(freqs, bias, r, factors);
+  a.q = q.const_data_ptr(), a.sq = s3(q, sf), a.k = k.const_data_ptr(), a.sk = s3(k, sf), a.sim = sim.mutable_data_ptr(), a.ss = s3(sim);
+  const Tensor ws = workspace(POPE_OP_SIM_FWD, a, q);
+  check(pope_b200_sim_fwd(&a, stream_of(q)), "pope_b200_sim_fwd");
+  return sim;
+}
+
+Grads sim_backward(const Tensor& dsim_, const Tensor& q_, const Tensor& k_, const Tensor& freqs_, const Tensor& bias_, bool need_df, bool need_db,
+                   bool allow_tf32, bool sf) {
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = inner_contig(q_), k = inner_contig(k_), dsim = inner_contig(dsim_), freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
+  const int r = (int)freqs.size(-1);
+  Grads g{at::empty_like(q), at::empty_like(k), Tensor(), Tensor(), Tensor()};
+  PopeSimBwdArgs a = {};
+  a.struct_bytes = sizeof(a), a.allow_tf32 = allow_tf32;
+  a.shape = shape_of(q, k, r, sf), a.embed = embed_of(freqs, bias, r);
+  a.q = q.const_data_ptr(), a.sq = s3(q, sf), a.k = k.const_data_ptr(), a.sk = s3(k, sf), a.dsim = dsim.const_data_ptr(), a.sds = s3(dsim);
+  a.dq = g.dq.mutable_data_ptr(), a.sdq = s3(g.dq, sf), a.dk = g.dk.mutable_data_ptr(), a.sdk = s3(g.dk, sf);
+  put_phase_grads(a, g, freqs, bias, need_df, need_db);
+  const Tensor ws = workspace(POPE_OP_SIM_BWD, a, q);
+  check(pope_b200_sim_bwd(&a, stream_of(q)), "pope_b200_sim_bwd");
+  return g;
+}
+
+struct Similarity : torch::autograd::Function<Similarity> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias,
+                        bool allow_tf32, bool seq_first, const Factors& factors) {
+    ctx->save_for_backward({q, k, freqs, bias});
+    ctx->saved_data["tf32"] = allow_tf32, ctx->saved_data["seq"] = seq_first;
+    return sim_forward(q, k, freqs, bias, allow_tf32, factors, seq_first);
+  }
+  static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad) {
+    const auto s = ctx->get_saved_variables();
+    Grads g = sim_backward(grad[0].to(s[0].scalar_type()), s[0], s[1], s[2], s[3], ctx->needs_input_grad(2), ctx->needs_input_grad(3),
+                           ctx->saved_data["tf32"].toBool(), ctx->saved_data["seq"].toBool());
+    return {g.dq, g.dk, to_dtype_of(g.dfreqs, s[2]), to_dtype_of(g.dbias, s[3]), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor similarity(const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias, bool allow_tf32, const Factors& factors,
+                  bool seq_first) {
+  validate(q, k, freqs, seq_first);
+  py::gil_scoped_release nogil;
+  if (!wants_graph(q, k, freqs, bias)) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return sim_forward(q, k, freqs, bias, allow_tf32, factors, seq_first);
+  }
+  return Similarity::apply(q, k, freqs, bias, allow_tf32, seq_first, factors);
+}
+
+// ---- the stand-alone transform -----------------------------------------------------------------------------------
+std::tuple<Tensor, Tensor> apply_forward(const Tensor& q_, const Tensor& k_, const Tensor& freqs_, const Tensor& bias_) {
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = inner_contig(q_), k = inner_contig(k_), freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
+  const int r = (int)freqs.size(-1);
+  const auto opt = q.options().dtype(at::kFloat);
+  Tensor q_out = at::empty({q.size(0), q.size(1), q.size(2), q.size(3) + r}, opt);
+  Tensor k_out = at::empty({k.size(0), k.size(1), k.size(2), k.size(3) + r}, opt);
+  PopeApplyArgs a = {};
+  a.struct_bytes = sizeof(a), a.shape = shape_of(q, k, r), a.embed = embed_of(freqs, bias, r);
+  a.q = q.const_data_ptr(), a.sq = s3(q), a.k = k.const_data_ptr(), a.sk = s3(k);
+  a.q_out = q_out.mutable_data_ptr<float>(), a.sqo = s3(q_out), a.k_out = k_out.mutable_data_ptr<float>(), a.sko = s3(k_out);
+  check(pope_b200_apply_qk_fwd(&a, stream_of(q)), "pope_b200_apply_qk_fwd");
+  return {q_out, k_out};
+}
+
+struct ApplyQK : torch::autograd::Function<ApplyQK> {
+  static torch::autograd::tensor_list forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& freqs,
+                                              const Tensor& bias) {
+    ctx->save_for_backward({q, k, freqs, bias});
+    auto [q_out, k_out] = apply_forward(q, k, freqs, bias);
+    return {q_out, k_out};
+  }
+  static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad) {
+    const auto s = ctx->get_saved_variables();
+    c10::cuda::OptionalCUDAGuard guard(s[0].device());
+    const Tensor q = inner_contig(s[0]), k = inner_contig(s[1]), freqs = fp32_rows(s[2]), bias = fp32_rows(s[3]);
+    const Tensor gq = grad[0].contiguous().to(at::kFloat), gk = grad[1].contiguous().to(at::kFloat);
+    const int r = (int)freqs.size(-1);
+    Grads g{at::empty_like(q), at::empty_like(k), Tensor(), Tensor(), Tensor()};
+    PopeApplyBwdArgs a = {};
+    a.struct_bytes = sizeof(a), a.shape = shape_of(q, k, r), a.embed = embed_of(freqs, bias, r);
+    a.q = q.const_data_ptr(), a.sq = s3(q), a.k = k.const_data_ptr(), a.sk = s3(k);
+    a.dq_out = gq.const_data_ptr<float>(), a.sdqo = s3(gq), a.dk_out = gk.const_data_ptr<float>(), a.sdko = s3(gk);
+    a.dq = g.dq.mutable_data_ptr(), a.sdq = s3(g.dq), a.dk = g.dk.mutable_data_ptr(), a.sdk = s3(g.dk);
+    put_phase_grads(a, g, freqs, bias, ctx->needs_input_grad(2), ctx->needs_input_grad(3));
+    check(pope_b200_apply_qk_bwd(&a, stream_of(q)), "pope_b200_apply_qk_bwd");
+    return {g.dq, g.dk, to_dtype_of(g.dfreqs, s[2]), to_dtype_of(g.dbias, s[3])};
+  }
+};
+
+std::tuple<Tensor, Tensor> apply_qk(const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias) {
+  if (freqs.size(-1) != 0 && freqs.size(-2) != k.size(2)) assertion("freqs must have one row per key position");
+  py::gil_scoped_release nogil;
+  if (!wants_graph(q, k, freqs, bias)) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return apply_forward(q, k, freqs, bias);
+  }
+  const auto out = ApplyQK::apply(q, k, freqs, bias);
+  return {out[0], out[1]};
+}
+
+// ---- the embedding tables ------------------------------------------------------------------------------------------
+// (freqs, clamped bias, positions, flat inverse frequencies, axis of a feature) of a sequence or a grid; a sequence has no
+// last two.  bias may carry a gradient, the frequencies do not (the Python modules see to that).
+struct Table : torch::autograd::Function<Table> {
+  static torch::autograd::tensor_list forward(torch::autograd::AutogradContext* ctx, const Tensor& bias, const std::vector<Tensor>* inv,
+                                              const std::vector<int64_t>* dims, double offset) {
+    c10::cuda::OptionalCUDAGuard guard(bias.device());
+    PopeTableArgs a = {};
+    a.struct_bytes = sizeof(a), a.axes = (int32_t)dims->size(), a.offset = (float)offset;
+    int64_t n = 1, r = 0;
+    for (int i = 0; i < a.axes; ++i) {
+      a.dims[i] = (int32_t)(*dims)[i], a.width[i] = (int32_t)(*inv)[i].numel(), a.inv_freqs[i] = (*inv)[i].const_data_ptr<float>();
+      n *= a.dims[i], r += a.width[i];
+    }
+    const bool grid = a.axes > 1;
+    const auto opt = bias.options();
+    Tensor freqs = at::empty({n, r}, opt), clamped = at::empty({bias.size(0), bias.size(1)}, opt);
+    Tensor pos = grid ? at::empty({n, a.axes}, opt) : at::empty({n}, opt), inv_flat, axis_of;
+    if (grid) inv_flat = at::empty({r}, opt), axis_of = at::empty({r}, opt.dtype(at::kInt));
+    a.H = (int32_t)bias.size(0), a.bias = bias.const_data_ptr<float>(), a.bias_out = clamped.mutable_data_ptr<float>();
+    a.positions = pos.mutable_data_ptr<float>(), a.freqs = freqs.mutable_data_ptr<float>();
+    if (grid) a.inv_flat = inv_flat.mutable_data_ptr<float>(), a.axis_of = axis_of.mutable_data_ptr<int32_t>();
+    check(pope_b200_table(&a, stream_of(bias)), "pope_b200_table");
+    ctx->save_for_backward({bias});
+    ctx->set_materialize_grads(false);
+    torch::autograd::tensor_list out = {freqs, clamped, pos};
+    if (grid) out.insert(out.end(), {inv_flat, axis_of});
+    torch::autograd::tensor_list constant = out;
+    constant.erase(constant.begin() + 1);
+    ctx->mark_non_differentiable(constant);
+    return out;
+  }
+  static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad) {
+    if (!grad[1].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
+    const Tensor bias = ctx->get_saved_variables()[0], g = grad[1].contiguous();
+    c10::cuda::OptionalCUDAGuard guard(bias.device());
+    Tensor out = at::empty_like(bias);
+    PopeClampBwdArgs a = {};
+    a.struct_bytes = sizeof(a), a.n = bias.numel();
+    a.bias = bias.const_data_ptr<float>(), a.grad = g.const_data_ptr<float>(), a.grad_bias = out.mutable_data_ptr<float>();
+    check(pope_b200_clamp_bwd(&a, stream_of(bias)), "pope_b200_clamp_bwd");
+    return {out, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// None when the module's tensors are not what the kernel takes (another type or device, frequencies that train, ...)
+optional<std::vector<Tensor>> table(const Tensor& bias, const std::vector<Tensor>& inv, const std::vector<int64_t>& dims, double offset) {
+  auto plain = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous(); };
+  if (inv.empty() || inv.size() != dims.size() || inv.size() > POPE_MAX_AXES || bias.dim() != 2 || !plain(bias)) return std::nullopt;
+  int64_t n = 1, r = 0;
+  for (const int64_t d : dims) {
+    if (d <= 0 || d > INT32_MAX || n * d > INT32_MAX) return std::nullopt;
+    n *= d;
+  }
+  for (const Tensor& t : inv) {
+    if (!plain(t) || t.device() != bias.device() || t.requires_grad() || t.numel() == 0) return std::nullopt;
+    r += t.numel();
+  }
+  if (bias.size(1) != r || bias.size(0) == 0) return std::nullopt;
+  py::gil_scoped_release nogil;
+  return Table::apply(bias, &inv, &dims, offset);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("flash_attn", &flash_attn);
+  m.def("similarity", &similarity);
+  m.def("apply_qk", &apply_qk);
+  m.def("table", &table);
+  m.def("attn_forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask,
+                           bool causal, double scale, const Factors& factors) {
+    validate(q, k, freqs, false);
+    at::NoGradGuard off;
+    return attn_forward(q, k, v, freqs, bias, mask, causal, scale, factors, false);
+  });
+  m.def("attn_backward", [](const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
+                            const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask, bool causal, double scale, bool need_df,
+                            bool need_db, const Factors& factors) {
+    at::NoGradGuard off;
+    Grads g = attn_backward(dout, q, k, v, out, lse, freqs, bias, mask, causal, scale, need_df, need_db, factors, false);
+    return std::make_tuple(g.dq, g.dk, g.dv, need_df ? optional<Tensor>(g.dfreqs) : std::nullopt, need_db ? optional<Tensor>(g.dbias) : std::nullopt);
+  });
+  m.def("sim_forward", [](const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias, bool allow_tf32, const Factors& factors) {
+    validate(q, k, freqs, false);
+    at::NoGradGuard off;
+    return sim_forward(q, k, freqs, bias, allow_tf32, factors, false);
+  });
+  m.def("sim_backward", [](const Tensor& dsim, const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias, bool need_df, bool need_db,
+                           bool allow_tf32) {
+    at::NoGradGuard off;
+    Grads g = sim_backward(dsim, q, k, freqs, bias, need_df, need_db, allow_tf32, false);
+    return std::make_tuple(g.dq, g.dk, need_df ? optional<Tensor>(g.dfreqs) : std::nullopt, need_db ? optional<Tensor>(g.dbias) : std::nullopt);
+  });
+}

@@ -42,7 +42,6 @@ def _interleave_polar(magnitude: Tensor, phase: Tensor) -> Tensor:
     return pair.reshape(*pair.shape[:-2], -1)
 
 
-@torch.autocast("cuda", enabled=False)
 def apply_pope_to_qk(pope, q: Tensor, k: Tensor, to_magnitude=F.softplus, return_complex: bool = False):
     """Expand head-first q (b,h,i,d) and k (b,hk,j,d) to their polar form of width 2r + (d - r).
 
@@ -59,7 +58,12 @@ def apply_pope_to_qk(pope, q: Tensor, k: Tensor, to_magnitude=F.softplus, return
         from . import _native          # CUDA tensors: one fused pass in the native library (no fallback when it is present)
         if _native.apply_qk_supported(q, k, freqs, bias):
             return _native.apply_qk(q, k, freqs, bias)
+    return _apply_pope_to_qk_torch(freqs, bias, q, k, to_magnitude, return_complex)
 
+
+@torch.autocast("cuda", enabled=False)
+def _apply_pope_to_qk_torch(freqs, bias, q, k, to_magnitude, return_complex):
+    n_q, r, d = q.shape[-2], freqs.shape[-1], q.shape[-1]
     if freqs.ndim == 3:                       # (b, n, r) -> (b, 1, n, r)
         freqs = freqs.unsqueeze(1)
     key_phase = freqs + bias.unsqueeze(-2)    # (.., h, n, r)
@@ -106,8 +110,17 @@ class PoPE(nn.Module):
     def device(self):
         return self.inv_freqs.device
 
-    @torch.autocast("cuda", enabled=False)
     def forward(self, pos_or_seq_len: Union[Tensor, int], offset=0) -> PolarEmbedReturn:
+        if self.bias.is_cuda and isinstance(pos_or_seq_len, int) and isinstance(offset, (int, float)):
+            from . import _native          # one launch instead of a chain of elementwise kernels
+            made = _native.embed_table(self.bias, [self.inv_freqs], [pos_or_seq_len], offset)
+            if made is not None:
+                freqs, bias, positions = made
+                return FactoredPolarEmbed(freqs, bias, positions, self.inv_freqs)
+        return self._forward_torch(pos_or_seq_len, offset)
+
+    @torch.autocast("cuda", enabled=False)
+    def _forward_torch(self, pos_or_seq_len, offset) -> PolarEmbedReturn:
         if torch.is_tensor(pos_or_seq_len):
             positions = pos_or_seq_len
         else:

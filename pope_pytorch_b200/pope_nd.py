@@ -43,8 +43,17 @@ class AxialPoPE(nn.Module):
             coords = coords.unsqueeze(-1)
         return coords.flip(-1)
 
-    @torch.autocast("cuda", enabled=False)
     def forward(self, pos_or_dims: Union[Tensor, Tuple[int, ...]]) -> PolarEmbedReturn:
+        if self.bias.is_cuda and isinstance(pos_or_dims, tuple) and len(pos_or_dims) == len(self.axial_dims) > 1:
+            from . import _native          # one launch instead of a chain of elementwise kernels
+            made = _native.embed_table(self.bias, list(self.inv_freqs), list(pos_or_dims))
+            if made is not None:
+                freqs, bias, positions, inv_flat, axis_of = made
+                return FactoredPolarEmbed(freqs, bias, positions, inv_flat, axis_of)
+        return self._forward_torch(pos_or_dims)
+
+    @torch.autocast("cuda", enabled=False)
+    def _forward_torch(self, pos_or_dims) -> PolarEmbedReturn:
         positions = self.get_grid_positions(*pos_or_dims, device=self.device) \
             if isinstance(pos_or_dims, tuple) else pos_or_dims
         assert positions.shape[-1] == len(self.axial_dims)
