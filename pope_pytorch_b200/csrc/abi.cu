@@ -160,7 +160,7 @@ int pope_b200_attn_fwd(const PopeAttnArgs* a, void* stream) {
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const cudaError_t e = tc ? pope::attn_fwd_tc(*a, st) : dec ? pope::decode_stream(*a, st) : pope::attn_fwd_simt(*a, st);
   if (e != cudaSuccess) return POPE_ERR_CUDA;
-  g_last_path = tc ? "tcgen05" : dec ? "decode_stream" : "simt";
+  g_last_path = tc ? "tcgen05" : dec && !pope::decode_is_exact(*a) ? "decode_stream" : "simt";
   return POPE_OK;
 }
 

@@ -30,17 +30,20 @@ namespace pope {
 
 
 struct DecodeStreamP {
-  int H, Hk, Nk, r, nsplit, split_len, nstages, HDP;
+  int H, Hk, Nk, r, nsplit, nstages, head_blocks;   // head_blocks: groups of G query heads per key head
   int k_rows_contiguous, v_rows_contiguous;
   float scale_log2;
   const void *q, *k, *v;
-  Strides sq, sk, sv;
+  Strides sq, sk, sv, so;
+  void* out;
+  float* lse;
   const float *freqs, *bias;
   int64_t sfn, bias_sh;
   const __half *ch, *sh;     // fp16 cos / sin of freqs, [Nk][r]
   const uint8_t* mask;
   int64_t msb, msn;
-  float *part_o, *part_ml;
+  float *part_o, *part_ml;   // [unit][split][G][D] and [unit][split][G][max (log2 units), sum]
+  unsigned int* done;        // [unit] CTAs of the unit that have written their partials; zero when the kernel starts
   unsigned int* status;
   // paged cache (page_table != nullptr): k / v point at the page pools, sk.h / sv.h = page_size * d, sk.n = sv.n = d
   const int32_t* page_table;
@@ -49,65 +52,118 @@ struct DecodeStreamP {
   int64_t page_stride;       // elements per page
 };
 
-template <typename T> __device__ __forceinline__ void unpack8(const uint4& w, float (&x)[8]) {
-  const uint32_t u[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float2 v = unpack2<T>(u[e]);
-    x[2 * e] = v.x, x[2 * e + 1] = v.y;
-  }
+// two fp32 lanes per instruction (the kernel is bound by instruction issue, not by FMA throughput)
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, z, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nmov.b64 z, {%6, %7};\nfma.rn.f32x2 w, x, y, z;\n"
+      "mov.b64 {%0, %1}, w;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nmul.rn.f32x2 w, x, y;\nmov.b64 {%0, %1}, w;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nadd.rn.f32x2 w, x, y;\nmov.b64 {%0, %1}, w;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+// softplus(x) / ln 2 = max(y, 0) + log2(1 + 2^-|y|), y = x log2(e): the accuracy of softplus_fast; the factor ln 2 is
+// part of the query's coordinates
+__device__ __forceinline__ float2 softplus2_log2(float2 x) {
+  const float2 y = mul2(x, make_float2(LOG2E, LOG2E));
+  const float2 t = add2(make_float2(ex2_approx(-fabsf(y.x)), ex2_approx(-fabsf(y.y))), make_float2(1.f, 1.f));
+  return add2(make_float2(lg2_approx(t.x), lg2_approx(t.y)), make_float2(fmaxf(y.x, 0.f), fmaxf(y.y, 0.f)));
 }
 
-// D: head dim (64, 96, 128); LPK: lanes per key (4 or 8); KPL: keys per lane and tile; NW: worker warps (+ 1 loader
-// warp); MINB: CTAs per SM the register allocation must allow.  A tile is NW * KPL * 32 / LPK keys.
-template <typename T, int D, int LPK, int KPL, int NW, int MINB>
-__global__ void __launch_bounds__(32 * (NW + 1), MINB) attn_decode_stream_kernel(DecodeStreamP p) {
-  constexpr int DS_WORKERS = NW;
-  constexpr int KPW = 32 / LPK;                 // keys per warp and pass
-  constexpr int TILE = DS_WORKERS * KPW * KPL;  // keys per tile
-  constexpr int NCH = D / 8;                    // 16-byte chunks per key row
-  constexpr int NI = NCH / LPK;                 // chunks per lane
-  static_assert(NCH % LPK == 0, "chunks must divide over the lanes of a key");
-  constexpr int FPL = 4;                        // output features per lane in the P V step
-  constexpr int OLANES = D / FPL;               // lanes that own output features
-  constexpr bool SWZ = (LPK == 4) && (D % 64 == 0);   // see the bank note below
+template <typename T, int N2> __device__ __forceinline__ void unpack_words(const void* src, float2 (&x)[N2]) {
+  uint32_t u[N2];
+  if constexpr (N2 == 4) {
+    const uint4 w = *reinterpret_cast<const uint4*>(src);
+    u[0] = w.x, u[1] = w.y, u[2] = w.z, u[3] = w.w;
+  } else {
+    const uint2 w = *reinterpret_cast<const uint2*>(src);
+    u[0] = w.x, u[1] = w.y;
+  }
+#pragma unroll
+  for (int e = 0; e < N2; ++e) x[e] = unpack2<T>(u[e]);
+}
+
+// every thread of every CTA of the cluster
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p in the shared memory of CTA `rank` of this cluster
+__device__ __forceinline__ float dsmem_ld(const float* p, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+constexpr int DS_EXACT_KEYS = 1024;   // shorter contiguous key ranges keep fp32 phases
+constexpr int DS_TILE = 64;       // keys per tile
+constexpr int DS_MAX_SPLIT = 64;  // key ranges per unit
+
+// D: head dim (64, 96, 128); G: query heads of one key head that a CTA serves (1, 2, 4) -- each key is transformed once for
+// all of them; LPK: lanes per key; E: features of one piece of a key row (8 = 16-byte loads, 4 = 8-byte loads), a lane
+// takes pieces t, t + LPK, ...: with half of the features rotated every lane then has as many rotated as plain ones.
+// NW: worker warps (+ 1 loader warp): 8, two CTAs per SM; with four heads 16 in one CTA, whose coordinates then are read from
+// shared memory (91 against 102 us for 8 warps with everything in registers at (2, 32 / 8, 32768, 128)).
+// SHORT: a call of few tiles per CTA, where launches and latency are the cost: the ring brings the fp32 phases themselves and
+// the lanes take their cosines and sines (no table kernel), and the splits of a unit form one cluster that merges through
+// distributed shared memory (no partials in global memory, no counters).
+template <typename T, int D, int G, int LPK, int E, int NW, bool SHORT>
+__global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_stream_kernel(DecodeStreamP p) {
+  constexpr int TILE = DS_TILE;
+  constexpr int KPW = 32 / LPK;                   // keys per warp and pass
+  constexpr int WK = TILE / NW;           // keys per warp and tile
+  constexpr int KPL = WK / KPW;                   // keys per lane and tile
+  constexpr int NI = D / (LPK * E);               // pieces per lane
+  constexpr int E2 = E / 2;
+  constexpr bool QREG = G < 4;                    // the lane's slice of the queries: registers, or read from shared memory per tile
+  static_assert(NI * LPK * E == D && KPL * KPW == WK, "pieces must divide over the lanes of a key");
+  constexpr int PL = D == 64 ? 8 : 16;            // lanes per row of V, 8 features each
+  constexpr int KV = 32 / PL;                     // rows of V per warp and pass
+  constexpr int NV = G * KPL, DUP = LPK / NV;     // scores of a lane group; lanes that end up with the same one
+  static_assert(NV * DUP == LPK, "the scores of a lane group must divide over its lanes");
 
   extern __shared__ __align__(128) uint8_t smem[];
-  const int r = p.r, RC = r >> 3;
+  const int r = p.r;
   const int kbytes = TILE * D * 2, tbytes = TILE * r * 2;
   const int stage_bytes = 2 * kbytes + 2 * tbytes;
-  float* qcs = reinterpret_cast<float*>(smem + (size_t)p.nstages * stage_bytes);   // [D] Qc / pass-through q, then [D] Qs
-  float* red_o = qcs + 2 * D;                                                       // [DS_WORKERS][D]
-  float* red_ml = red_o + DS_WORKERS * D;                                           // [DS_WORKERS][2]
-  uint64_t* full = reinterpret_cast<uint64_t*>(red_ml + 2 * DS_WORKERS);            // [nstages] tile landed
+  float* qcs = reinterpret_cast<float*>(smem + (size_t)p.nstages * stage_bytes);   // [G][2][D] Qc / pass-through q, Qs
+  float* red_o = qcs + G * 2 * D;                                                   // [NW][G][D]
+  float* red_ml = red_o + NW * G * D;                                       // [NW][G][2]
+  float* wgt = red_ml + NW * G * 2;                                         // [G][DS_MAX_SPLIT] weights of the splits
+  uint64_t* full = reinterpret_cast<uint64_t*>(wgt + G * DS_MAX_SPLIT);             // [nstages] tile landed
   uint64_t* empty = full + p.nstages;                                               // [nstages] all workers done with it
-  int* pages_s = reinterpret_cast<int*>(empty + p.nstages);                         // [npg_smem] pages of this CTA's key range
+  unsigned int* last_s = reinterpret_cast<unsigned int*>(empty + p.nstages);        // whether this CTA finished last of its unit
+  int* pages_s = reinterpret_cast<int*>(last_s + 2);                                // [npg_smem] pages of this CTA's key range
 
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int u = blockIdx.y, b = u / p.H, h = u % p.H, hk = h % p.Hk;
+  const int u = blockIdx.y, hb = u % p.head_blocks, bk = u / p.head_blocks, hk = bk % p.Hk, b = bk / p.Hk;
+  auto head = [&](int g) { return hk + (hb * G + g) * p.Hk; };   // query head h reads key head h % Hk
   const T* kbase = (const T*)p.k + b * p.sk.b + hk * p.sk.h;
   const T* vbase = (const T*)p.v + b * p.sv.b + hk * p.sv.h;
-  // keys of this sequence (paged cache: its own length, at most the bound the split was planned for)
+  // keys of this sequence (paged cache: its own length, at most the bound the split was planned for), cut evenly
   const int nk = p.seq_lens ? max(0, min(p.seq_lens[b], p.Nk)) : p.Nk;
-  const int kb = blockIdx.x * p.split_len, ke = min(nk, kb + p.split_len);
+  const int tiles_all = (nk + TILE - 1) / TILE;
+  const int kb = (int)((int64_t)tiles_all * blockIdx.x / p.nsplit) * TILE;
+  const int ke = min(nk, (int)((int64_t)tiles_all * (blockIdx.x + 1) / p.nsplit) * TILE);
   const int T_tiles = ke > kb ? (ke - kb + TILE - 1) / TILE : 0;
 
   if (tid == 0) {
-    for (int s = 0; s < p.nstages; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], DS_WORKERS);
+    for (int s = 0; s < p.nstages; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], NW);
     mbar_init_fence();
-  }
-  // the query's polar coordinates with the key-side bias folded in (exact transform: one row per CTA)
-  if (tid < D) {
-    const T* qrow = (const T*)p.q + b * p.sq.b + h * p.sq.h;
-    const float x = to_f32<T>(qrow[tid]);
-    float c = x, s = 0.f;
-    if (tid < r) {
-      float sn, cs;
-      sincosf(p.freqs[(int64_t)(max(nk, 1) - 1) * p.sfn + tid] - p.bias[hk * p.bias_sh + tid], &sn, &cs);
-      const float a = softplus_f(x);
-      c = a * cs, s = a * sn;
-    }
-    qcs[tid] = c, qcs[D + tid] = s;
   }
   if (p.page_table) {
     // page indices of [kb, ke); an index outside the pool is never dereferenced (clamped, status bit 1)
@@ -124,15 +180,11 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) attn_decode_stream_kernel
   __syncthreads();
   bool failed = false;
 
-  if (w == DS_WORKERS) {
+  if (w == NW) {
     // =============================== loader =====================================================
-    pdl_trigger();   // the split combine behind this kernel may set itself up
-    pdl_wait();      // the fp16 phase table (the kernel before this one) is complete
-    for (int jt = 0; jt < T_tiles && !failed; ++jt) {
-      const int s = jt % p.nstages, key0 = kb + jt * TILE, n = min(TILE, ke - key0);
+    auto load_kv = [&](int jt, int s) {
+      const int key0 = kb + jt * TILE, n = min(TILE, ke - key0);
       uint8_t* st = smem + (size_t)s * stage_bytes;
-      if (jt >= p.nstages) failed = !mbar_wait(&empty[s], ((jt / p.nstages) - 1) & 1, WAIT_LIMIT);
-      if (failed) { drain_copies(full, p.nstages, jt - p.nstages, jt); break; }
       if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)(2 * n * D * 2 + 2 * n * r * 2));
       __syncwarp();
       const T *kt = kbase + (int64_t)key0 * p.sk.n, *vt = vbase + (int64_t)key0 * p.sv.n;
@@ -151,139 +203,401 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB) attn_decode_stream_kernel
       } else {
         for (int i = lane; i < n; i += 32) bulk_load(st + kbytes + i * D * 2, vt + (int64_t)i * p.sv.n, D * 2, &full[s]);
       }
-      if (r > 0) {
-        if (lane == 2) bulk_load(st + 2 * kbytes, p.ch + (int64_t)key0 * r, n * r * 2, &full[s]);
-        if (lane == 3) bulk_load(st + 2 * kbytes + tbytes, p.sh + (int64_t)key0 * r, n * r * 2, &full[s]);
+    };
+    auto load_phases = [&](int jt, int s) {
+      const int key0 = kb + jt * TILE, n = min(TILE, ke - key0);
+      uint8_t* st = smem + (size_t)s * stage_bytes + 2 * kbytes;
+      if constexpr (SHORT) {   // rows of the phase table itself: as many bytes as the two fp16 rows
+        if (r > 0 && lane == 2) bulk_load(st, p.freqs + (int64_t)key0 * r, n * r * 4, &full[s]);
+        return;
       }
+      if (r > 0 && lane == 2) bulk_load(st, p.ch + (int64_t)key0 * r, n * r * 2, &full[s]);
+      if (r > 0 && lane == 3) bulk_load(st + tbytes, p.sh + (int64_t)key0 * r, n * r * 2, &full[s]);
+    };
+    // the first ring of K and V does not depend on the phase table, which the kernel before this one may still be writing
+    const int pre = min(T_tiles, p.nstages);
+    for (int jt = 0; jt < pre; ++jt) load_kv(jt, jt);
+    if (!SHORT) pdl_wait();
+    for (int jt = 0; jt < pre; ++jt) load_phases(jt, jt);
+    int s = 0;
+    uint32_t par = 0;
+    for (int jt = pre; jt < T_tiles; ++jt) {
+      failed = !mbar_wait(&empty[s], par, WAIT_LIMIT);
+      if (failed) { drain_copies(full, p.nstages, jt - p.nstages, jt); break; }
+      load_kv(jt, s), load_phases(jt, s);
+      if (++s == p.nstages) s = 0, par ^= 1;
     }
     if (failed && lane == 0) atomicOr(p.status, 1u);
+    if (SHORT && p.nsplit > 1) cluster_sync(), cluster_sync();
     return;   // nothing below is a block-wide barrier; the workers finish on their own
   }
 
   // =============================== workers ======================================================
+  auto worker_sync = []() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); };
+  // the queries' polar coordinates with the key-side bias folded in (exact transform: one row per head and CTA)
+  for (int i = tid; i < G * D; i += 32 * NW) {
+    const int g = i / D, c = i - g * D;
+    const T* qrow = (const T*)p.q + b * p.sq.b + head(g) * p.sq.h;
+    const float x = to_f32<T>(qrow[c]);
+    float qc = x, qs = 0.f;
+    if (c < r) {
+      float sn, cs;
+      sincosf(p.freqs[(int64_t)(max(nk, 1) - 1) * p.sfn + c] - p.bias[hk * p.bias_sh + c], &sn, &cs);
+      const float a = softplus_f(x) * LN2;   // (the keys' magnitudes come in units of ln 2)
+      qc = a * cs, qs = a * sn;
+    }
+    qcs[g * 2 * D + c] = qc, qcs[g * 2 * D + D + c] = qs;
+  }
+  worker_sync();
+
   const int kw = lane / LPK, t = lane % LPK;        // key of the warp's group, lane within the key
-  const int krow0 = w * KPW * KPL + kw;             // first row of the tile this lane works on; the others KPW apart
-  // Bank note: with 4 lanes per key a quarter-warp covers two keys; when the row stride is a multiple of 128 bytes
-  // both rows start on the same bank, so odd rows walk their chunk groups in the swapped order (i ^ 1).
-  const int swz = SWZ ? (krow0 & 1) : 0;            // KPW is even for LPK = 4: all rows of a lane share the parity
-  // this lane's slice of the query, in the order it visits its chunks
-  float qc[NI][8], qs[NI][8];
+  const int krow0 = w * WK + kw;                    // first row of the tile this lane works on; the others KPW apart
+  float2 qc[QREG ? G : 1][NI][E2], qs[QREG ? G : 1][NI][E2];   // this lane's slice of the queries
+  if constexpr (QREG) {
 #pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const int c = t + LPK * (i ^ swz);
+    for (int g = 0; g < G; ++g)
 #pragma unroll
-    for (int e = 0; e < 8; ++e) qc[i][e] = qcs[c * 8 + e], qs[i][e] = qcs[D + c * 8 + e];
+      for (int i = 0; i < NI; ++i)
+#pragma unroll
+        for (int e = 0; e < E2; ++e) {
+          const int c = (t + LPK * i) * E + 2 * e;
+          qc[g][i][e] = *reinterpret_cast<const float2*>(qcs + g * 2 * D + c);
+          qs[g][i][e] = *reinterpret_cast<const float2*>(qcs + g * 2 * D + D + c);
+        }
   }
   const uint8_t* maskb = p.mask ? p.mask + b * p.msb : nullptr;
-  float mrun = -CUDART_INF_F, lrun = 0.f, o[FPL] = {0.f, 0.f, 0.f, 0.f};
+  const int vg = lane / PL, vf = (lane % PL) * 8;   // row group and first feature of this lane in the P V step
+  // After the reduction over its group a lane holds one score: head my_g, key my_kq of its group.
+  const int my_g = t / DUP / KPL, my_kq = t / DUP % KPL;
+  auto holder = [](int g, int kq, int kw_) { return kw_ * LPK + (g * KPL + kq) * DUP; };   // first lane with that score
+  float m_run = -CUDART_INF_F, l_run = 0.f;         // of head my_g: the warp's maximum, the sum over the lane's own keys
+  float2 o[G][4];
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[g][e] = make_float2(0.f, 0.f);
 
+  int s = 0;
+  uint32_t par = 0;
   for (int jt = 0; jt < T_tiles; ++jt) {
-    const int s = jt % p.nstages, key0 = kb + jt * TILE;
+    const int key0 = kb + jt * TILE;
     const uint8_t* st = smem + (size_t)s * stage_bytes;
-    if (!failed) failed = !mbar_wait(&full[s], (jt / p.nstages) & 1, WAIT_LIMIT);
+    const int my_key = key0 + krow0 + my_kq * KPW;
+    const bool valid = my_key < ke && (!maskb || maskb[(int64_t)my_key * p.msn] != 0);
+    if (!failed) failed = !mbar_wait(&full[s], par, WAIT_LIMIT);
     if (failed) break;
-    float part[KPL];
-    bool valid[KPL];
+    // (rows past the end of the range hold stale bytes: their scores are dropped by `valid`)
+    float2 part[G][KPL];
 #pragma unroll
-    for (int kq = 0; kq < KPL; ++kq) {
-      const int krow = krow0 + kq * KPW, key = key0 + krow;
-      valid[kq] = key < ke && (!maskb || maskb[(int64_t)key * p.msn] != 0);
-      part[kq] = 0.f;
-      if (key < ke) {
-        const uint8_t* krow_p = st + krow * (D * 2);
-        const uint8_t* crow_p = st + 2 * kbytes + krow * (r * 2);
-        const uint8_t* srow_p = crow_p + tbytes;
+    for (int g = 0; g < G; ++g)
 #pragma unroll
-        for (int i = 0; i < NI; ++i) {
-          const int c = t + LPK * (i ^ swz);
-          float x[8];
-          unpack8<T>(*reinterpret_cast<const uint4*>(krow_p + c * 16), x);
-          if (c < RC) {
-            float co[8], si[8];
-            unpack8<__half>(*reinterpret_cast<const uint4*>(crow_p + c * 16), co);
-            unpack8<__half>(*reinterpret_cast<const uint4*>(srow_p + c * 16), si);
+      for (int kq = 0; kq < KPL; ++kq) part[g][kq] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float a = softplus_fast(x[e]);
-              part[kq] = fmaf(a, fmaf(qc[i][e], co[e], qs[i][e] * si[e]), part[kq]);
+    for (int i = 0; i < NI; ++i) {
+      const int c = (t + LPK * i) * E;
+      const bool rot = c < r;
+      // keys transformed together: one where the queries sit in registers, all where each piece of them is loaded once per tile
+      constexpr int KB = QREG ? 1 : KPL;
+#pragma unroll
+      for (int k0 = 0; k0 < KPL; k0 += KB) {
+        float2 kc[KB][E2], ks[KB][E2];   // polar coordinates of the lane's keys (in units of ln 2), or the plain features
+#pragma unroll
+        for (int m = 0; m < KB; ++m) {
+          const int kq = k0 + m;
+          const int krow = krow0 + kq * KPW;
+          unpack_words<T>(st + krow * (D * 2) + c * 2, kc[m]);
+          if (rot) {
+            const uint8_t* crow_p = st + 2 * kbytes + krow * (r * (SHORT ? 4 : 2));
+            float2 co[E2], si[E2];
+            if constexpr (SHORT) {
+#pragma unroll
+              for (int e = 0; e < E2; ++e) {
+                const float2 f = *reinterpret_cast<const float2*>(crow_p + c * 4 + e * 8);
+                sincos_reduced(f.x, &si[e].x, &co[e].x), sincos_reduced(f.y, &si[e].y, &co[e].y);
+              }
+            } else {
+              unpack_words<__half>(crow_p + c * 2, co);
+              unpack_words<__half>(crow_p + tbytes + c * 2, si);
             }
-          } else {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) part[kq] = fmaf(qc[i][e], x[e], part[kq]);
+            for (int e = 0; e < E2; ++e) {
+              const float2 a = softplus2_log2(kc[m][e]);
+              if constexpr (G == 1) {
+                part[0][kq] = fma2(a, fma2(qc[0][i][e], co[e], mul2(qs[0][i][e], si[e])), part[0][kq]);
+              } else {
+                kc[m][e] = mul2(a, co[e]), ks[m][e] = mul2(a, si[e]);
+              }
+            }
+          } else if constexpr (G == 1) {
+#pragma unroll
+            for (int e = 0; e < E2; ++e) part[0][kq] = fma2(qc[0][i][e], kc[m][e], part[0][kq]);
+          }
+        }
+        if constexpr (G > 1) {
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            float2 qv[E2], qw[E2];
+#pragma unroll
+            for (int e = 0; e < E2; ++e) {
+              if constexpr (QREG) qv[e] = qc[g][i][e], qw[e] = qs[g][i][e];
+              else qv[e] = *reinterpret_cast<const float2*>(qcs + g * 2 * D + c + 2 * e);
+            }
+#pragma unroll
+            for (int m = 0; m < KB; ++m)
+#pragma unroll
+              for (int e = 0; e < E2; ++e) part[g][k0 + m] = fma2(qv[e], kc[m][e], part[g][k0 + m]);
+            if (rot) {
+              if constexpr (!QREG) {
+#pragma unroll
+                for (int e = 0; e < E2; ++e) qw[e] = *reinterpret_cast<const float2*>(qcs + g * 2 * D + D + c + 2 * e);
+              }
+#pragma unroll
+              for (int m = 0; m < KB; ++m)
+#pragma unroll
+                for (int e = 0; e < E2; ++e) part[g][k0 + m] = fma2(qw[e], ks[m][e], part[g][k0 + m]);
+            }
           }
         }
       }
     }
-    float sc[KPL], mloc = -CUDART_INF_F;
+    // Sum over the lanes of a key, halving the values a lane still carries with every step: NV - 1 + log2(DUP) shuffles for
+    // NV scores, and everything that follows is done once per score instead of once per lane.
+    float v[NV];
 #pragma unroll
-    for (int kq = 0; kq < KPL; ++kq) {
+    for (int i = 0; i < NV; ++i) v[i] = part[i / KPL][i % KPL].x + part[i / KPL][i % KPL].y;
 #pragma unroll
-      for (int off = 1; off < LPK; off <<= 1) part[kq] += __shfl_xor_sync(0xffffffffu, part[kq], off);
-      sc[kq] = valid[kq] ? part[kq] * p.scale_log2 : -CUDART_INF_F;     // log2 units
-      mloc = fmaxf(mloc, sc[kq]);
+    for (int n = NV / 2; n >= 1; n /= 2) {
+      const int off = n * DUP;
+      const bool hi = (t & off) != 0;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float give = hi ? v[i] : v[i + n], keep = hi ? v[i + n] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+      }
     }
-    const float mnew = fmaxf(mrun, warp_max(mloc));
-    if (mnew != -CUDART_INF_F) {   // warp-uniform
-      const float alpha = ex2_approx(mrun - mnew);    // exp2(-inf) = 0 on the first visible tile
-      float pj[KPL], psum = 0.f;
 #pragma unroll
-      for (int kq = 0; kq < KPL; ++kq) pj[kq] = ex2_approx(sc[kq] - mnew), psum += pj[kq];   // 0 for masked keys
-      lrun = lrun * alpha + warp_sum(t == 0 ? psum : 0.f);
-      mrun = mnew;
+    for (int off = DUP / 2; off >= 1; off /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    const float sc = valid ? v[0] * p.scale_log2 : -CUDART_INF_F;     // log2 units
+    // the maximum may lag by 2^8: most tiles then need neither a warp reduction nor a rescale
+    if (__any_sync(0xffffffffu, sc > m_run + 8.f)) {
 #pragma unroll
-      for (int e = 0; e < FPL; ++e) o[e] *= alpha;
-      const uint8_t* vt = st + kbytes + (w * KPW * KPL) * (D * 2) + lane * (FPL * 2);
+      for (int g = 0; g < G; ++g) {
+        const float old = __shfl_sync(0xffffffffu, m_run, holder(g, 0, 0));
+        const float mx = warp_max(my_g == g ? fmaxf(m_run, sc) : -CUDART_INF_F);
+        const float alpha = mx == -CUDART_INF_F ? 1.f : ex2_approx(old - mx);    // exp2(-inf) = 0 on the first visible tile
+        if (my_g == g) m_run = mx, l_run *= alpha;
 #pragma unroll
-      for (int kq = 0; kq < KPL; ++kq)
+        for (int e = 0; e < 4; ++e) o[g][e] = mul2(o[g][e], make_float2(alpha, alpha));
+      }
+    }
+    const float pj = ex2_approx(sc - (m_run == -CUDART_INF_F ? 0.f : m_run));   // 0 for masked keys
+    l_run += pj;
+    const uint8_t* vt = st + kbytes + (w * WK + vg) * (D * 2) + vf * 2;
+    const bool clean = !maskb && key0 + TILE <= ke;   // every row of the tile is a key
 #pragma unroll
-        for (int kk = 0; kk < KPW; ++kk) {
-          const float pk = __shfl_sync(0xffffffffu, pj[kq], kk * LPK);
-          if (pk != 0.f && lane < OLANES) {   // masked / out-of-range rows may hold stale bytes: never touch them
-            const uint2 vv = *reinterpret_cast<const uint2*>(vt + (kq * KPW + kk) * (D * 2));
-            const float2 v01 = unpack2<T>(vv.x), v23 = unpack2<T>(vv.y);
-            o[0] = fmaf(pk, v01.x, o[0]), o[1] = fmaf(pk, v01.y, o[1]);
-            o[2] = fmaf(pk, v23.x, o[2]), o[3] = fmaf(pk, v23.y, o[3]);
-          }
-        }
+    for (int vk = 0; vk < WK / KV; ++vk) {
+      // row vk * KV + vg of the warp = key (row % KPW) of the lane groups, row / KPW of a lane's keys
+      float pk[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) pk[g] = __shfl_sync(0xffffffffu, pj, holder(g, vk * KV / KPW, vk * KV % KPW + vg));
+      bool any = clean;
+      if (!clean) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) any |= pk[g] != 0.f;
+      }
+      if (any && (D % 64 == 0 || vf < D)) {   // masked / out-of-range rows may hold stale bytes: never touch them
+        float2 vv[4];
+        unpack_words<T>(vt + vk * KV * (D * 2), vv);
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[g][e] = fma2(make_float2(pk[g], pk[g]), vv[e], o[g][e]);
+      }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
+    if (++s == p.nstages) s = 0, par ^= 1;
   }
   if (failed && lane == 0) atomicOr(p.status, 1u);
 
-  // merge the worker warps of the CTA, then hand the partial to the cross-split combine (natural-log units)
-  if (lane < OLANES) {
+  // merge the lanes of the warp, then the warps of the CTA
 #pragma unroll
-    for (int e = 0; e < FPL; ++e) red_o[w * D + lane * FPL + e] = o[e];
-  }
-  if (lane == 0) red_ml[2 * w] = mrun, red_ml[2 * w + 1] = lrun;
-  asm volatile("bar.sync 1, %0;" ::"n"(32 * DS_WORKERS) : "memory");
-  float M = -CUDART_INF_F;
+  for (int g = 0; g < G; ++g) {
 #pragma unroll
-  for (int ww = 0; ww < DS_WORKERS; ++ww) M = fmaxf(M, red_ml[2 * ww]);
-  const int64_t slot = (int64_t)u * p.nsplit + blockIdx.x;     // one query row per unit
-  for (int c = tid; c < p.HDP; c += 32 * DS_WORKERS) {
-    float acc = 0.f;
-    if (c < D) {
+    for (int e = 0; e < 4; ++e)
 #pragma unroll
-      for (int ww = 0; ww < DS_WORKERS; ++ww)
-        acc += red_ml[2 * ww] == -CUDART_INF_F ? 0.f : red_o[ww * D + c] * ex2_approx(red_ml[2 * ww] - M);
+      for (int off = PL; off < 32; off <<= 1) {
+        o[g][e].x += __shfl_xor_sync(0xffffffffu, o[g][e].x, off);
+        o[g][e].y += __shfl_xor_sync(0xffffffffu, o[g][e].y, off);
+      }
+    const float mg = __shfl_sync(0xffffffffu, m_run, holder(g, 0, 0));
+    const float lg = warp_sum(my_g == g && t % DUP == 0 ? l_run : 0.f);
+    if (lane < PL && vf < D) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(red_o + (w * G + g) * D + vf + 2 * e) = o[g][e];
     }
-    p.part_o[slot * p.HDP + c] = acc;
+    if (lane == 0) red_ml[(w * G + g) * 2] = mg, red_ml[(w * G + g) * 2 + 1] = lg;
   }
-  if (tid == 0) {
+  worker_sync();
+  float* fin = reinterpret_cast<float*>(smem);
+  const int64_t slot = ((int64_t)u * p.nsplit + blockIdx.x) * G;
+  auto cta_max = [&](int g) {
+    float M = -CUDART_INF_F;
+#pragma unroll
+    for (int ww = 0; ww < NW; ++ww) M = fmaxf(M, red_ml[(ww * G + g) * 2]);
+    return M;
+  };
+  auto cta_sum = [&](int g, float M) {
     float L = 0.f;
 #pragma unroll
-    for (int ww = 0; ww < DS_WORKERS; ++ww)
-      L += red_ml[2 * ww] == -CUDART_INF_F ? 0.f : red_ml[2 * ww + 1] * ex2_approx(red_ml[2 * ww] - M);
-    p.part_ml[slot * 2] = M * LN2, p.part_ml[slot * 2 + 1] = L;
+    for (int ww = 0; ww < NW; ++ww)
+      L += red_ml[(ww * G + g) * 2] == -CUDART_INF_F ? 0.f : red_ml[(ww * G + g) * 2 + 1] * ex2_approx(red_ml[(ww * G + g) * 2] - M);
+    return L;
+  };
+  auto write_out = [&](int g, int c, float acc, float L) {
+    T* orow = (T*)p.out + b * p.so.b + head(g) * p.so.h;
+    orow[c] = from_f32<T>(L > 0.f ? acc / L : 0.f);
+  };
+  auto write_lse = [&](int g, float M, float L) {
+    p.lse[(int64_t)b * p.H + head(g)] = L > 0.f ? M * LN2 + logf(L) : -CUDART_INF_F;
+  };
+  for (int i = tid; i < G * D; i += 32 * NW) {
+    const int g = i / D, c = i - g * D;
+    const float M = cta_max(g);
+    float acc = 0.f;
+#pragma unroll
+    for (int ww = 0; ww < NW; ++ww)
+      acc += red_ml[(ww * G + g) * 2] == -CUDART_INF_F ? 0.f : red_o[(ww * G + g) * D + c] * ex2_approx(red_ml[(ww * G + g) * 2] - M);
+    if (p.nsplit == 1) {
+      const float L = cta_sum(g, M);
+      write_out(g, c, acc, L);
+      if (c == 0) write_lse(g, M, L);
+    } else if (SHORT) {   // (every ring stage has been read: the first one takes the CTA's result)
+      fin[i] = acc;
+      if (c == 0) fin[G * D + 2 * g] = M, fin[G * D + 2 * g + 1] = cta_sum(g, M);
+    } else {
+      p.part_o[slot * D + i] = acc;
+      if (c == 0) p.part_ml[(slot + g) * 2] = M, p.part_ml[(slot + g) * 2 + 1] = cta_sum(g, M);
+    }
+  }
+  if (p.nsplit == 1) return;
+  if constexpr (SHORT) {
+    // CTA i of the cluster merges every nsplit-th element from the shared memory of all of them
+    __syncwarp();
+    cluster_sync();
+    for (int i = tid * p.nsplit + (int)blockIdx.x; i < G * D; i += 32 * NW * p.nsplit) {
+      const int g = i / D, c = i - g * D;
+      float m2[8], l2[8], a2[8], M = -CUDART_INF_F, L = 0.f, acc = 0.f;
+#pragma unroll
+      for (int sp = 0; sp < 8; ++sp) {
+        m2[sp] = -CUDART_INF_F, l2[sp] = a2[sp] = 0.f;
+        if (sp < p.nsplit) {
+          a2[sp] = dsmem_ld(fin + i, sp), m2[sp] = dsmem_ld(fin + G * D + 2 * g, sp), l2[sp] = dsmem_ld(fin + G * D + 2 * g + 1, sp);
+        }
+        M = fmaxf(M, m2[sp]);
+      }
+#pragma unroll
+      for (int sp = 0; sp < 8; ++sp) {
+        const float wt = m2[sp] == -CUDART_INF_F ? 0.f : ex2_approx(m2[sp] - M);
+        L = fmaf(wt, l2[sp], L), acc = fmaf(wt, a2[sp], acc);
+      }
+      write_out(g, c, acc, L);
+      if (c == 0) write_lse(g, M, L);
+    }
+    __syncwarp();
+    cluster_sync();   // nobody leaves while its shared memory is read
+    return;
+  }
+  // The CTA that finishes last merges the splits of its unit (one launch less than a kernel of its own, and no wait for the
+  // slowest unit of the grid).
+  __threadfence();
+  worker_sync();
+  if (tid == 0) {
+    pdl_wait();   // the counters were zeroed by the kernel before this one
+    *last_s = atomicAdd(p.done + u, 1u) == (unsigned)p.nsplit - 1u;
+  }
+  worker_sync();
+  if (!*last_s) return;
+  __threadfence();
+  const int64_t slot0 = (int64_t)u * p.nsplit * G;
+  if (w < G) {   // warp g: the weights of head g's splits, relative to their sum
+    float m2[DS_MAX_SPLIT / 32], l2[DS_MAX_SPLIT / 32], M = -CUDART_INF_F, L = 0.f;
+#pragma unroll
+    for (int i = 0; i < DS_MAX_SPLIT / 32; ++i) {
+      const int sp = lane + 32 * i;
+      const float2 ml = sp < p.nsplit ? __ldcg(reinterpret_cast<const float2*>(p.part_ml + (slot0 + (int64_t)sp * G + w) * 2))
+                                      : make_float2(-CUDART_INF_F, 0.f);
+      m2[i] = ml.x, l2[i] = ml.y, M = fmaxf(M, ml.x);
+    }
+    M = warp_max(M);
+#pragma unroll
+    for (int i = 0; i < DS_MAX_SPLIT / 32; ++i) {
+      m2[i] = m2[i] == -CUDART_INF_F ? 0.f : ex2_approx(m2[i] - M);
+      L += m2[i] * l2[i];
+    }
+    L = warp_sum(L);
+#pragma unroll
+    for (int i = 0; i < DS_MAX_SPLIT / 32; ++i) wgt[w * DS_MAX_SPLIT + lane + 32 * i] = m2[i];
+    if (lane == 0) red_ml[w] = L, write_lse(w, M, L);
+  }
+  worker_sync();
+  for (int i = tid; i < G * D; i += 32 * NW) {
+    const int g = i / D, c = i - g * D;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int sp = 0; sp < p.nsplit; ++sp) acc = fmaf(wgt[g * DS_MAX_SPLIT + sp], __ldcg(p.part_o + (slot0 + (int64_t)sp * G) * D + i), acc);
+    write_out(g, c, acc, red_ml[g]);
   }
 }
 
 // ---- host side -----------------------------------------------------------------------------------
+// Query heads per CTA: as many of the heads that share a key head as the registers hold (their coordinates live there), so
+// that K and V are read and transformed once for all of them.
+static int decode_heads(const PopeShape& s) {
+  const int groups = s.H / s.Hk;
+  return groups % 4 == 0 && s.d != 96 ? 4 : groups % 2 == 0 ? 2 : 1;
+}
+
+// CTAs resident at a time: two per SM with 8 worker warps, one with 16 (four heads per CTA)
+static int64_t decode_slots(const PopeShape& s) { return (decode_heads(s) == 4 ? 1 : 2) * 148; }
+
+// Key ranges per unit.  The time of a grid in units of one 64-key tile: whole waves of resident CTAs times the tiles of a CTA
+// plus what a CTA costs beside its tiles (start, ring fill, merge: about four tiles' time); the smallest wins.  SHORT: at
+// most a cluster of eight.
+static int decode_stream_split(const PopeShape& s, bool shrt) {
+  const int tiles = (s.Nk + DS_TILE - 1) / DS_TILE, g = decode_heads(s);
+  const int64_t units = (int64_t)s.B * s.H / g, slots = decode_slots(s);
+  const int most = std::min(tiles, shrt ? 8 : DS_MAX_SPLIT);
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int n = 1; n <= most; ++n) {
+    const int64_t cost = (units * n + slots - 1) / slots * ((tiles + n - 1) / n + 4);
+    if (cost < best_cost) best = n, best_cost = cost;
+  }
+  return best;
+}
+
+// The SHORT flavour saves a launch and the trip of the partials through L2, about 2 us, and pays for its own cosines and sines
+// with every tile of a CTA, the less the more heads share them: (2, 16, 4000, 128) with 8 tiles per CTA takes 21.6 us
+// against 18.9, (4, 32 / 8, 2000, 128) with 8 tiles of four heads 19.9 against 20.7, (2, 16 / 4, 777, 128) 10.0 against 11.8.
+// It copies rows of the phase table, which therefore has to be contiguous.  Below DS_EXACT_KEYS keys every call takes it: those
+// calls are promised fp32 phases (they belong to the exact-arithmetic family; a call without a usable table goes to its
+// other kernels).
+static bool decode_short_possible(const PopeShape& s, const PopeEmbed& e) {
+  return s.r == 0 || (e.sf.n == s.r && (reinterpret_cast<uintptr_t>(e.freqs) & 15) == 0);
+}
+static bool decode_short(const PopeShape& s, const PopeEmbed& e) {
+  if (!decode_short_possible(s, e)) return false;
+  if (s.Nk < DS_EXACT_KEYS) return true;
+  const int tiles = (s.Nk + DS_TILE - 1) / DS_TILE, n = decode_stream_split(s, true), g = decode_heads(s);
+  const int64_t ctas = (int64_t)s.B * s.H / g * n, slots = decode_slots(s);
+  return (ctas + slots - 1) / slots * ((tiles + n - 1) / n) <= 4 + g;
+}
+
 bool decode_stream_supported(const PopeAttnArgs& a) {
   const PopeShape& s = a.shape;
-  if (s.Nq != 1 || a.causal || s.Nk < 1024) return false;
+  if (s.Nq != 1 || a.causal) return false;
+  if (s.Nk < DS_EXACT_KEYS && !decode_short_possible(s, a.embed)) return false;
   if (s.dtype != POPE_BF16 && s.dtype != POPE_F16) return false;
   if (s.d != 64 && s.d != 96 && s.d != 128) return false;
   if (s.r % 8 != 0) return false;
@@ -296,102 +610,111 @@ bool decode_stream_supported(const PopeAttnArgs& a) {
   return true;
 }
 
-static int decode_tile(int) { return 64; }   // keys per tile of every instantiation below (8 warps x 32 / LPK x KPL)   // keys per tile: 4 lanes per key at d = 96, else 8
-
-// Split the keys so that the grid fills whole waves of one CTA pair per SM; every split keeps at least 8 tiles.
-static void decode_stream_plan(const PopeShape& s, int& nsplit, int& split_len) {
-  const int tile = decode_tile(s.d);
-  const int64_t units = (int64_t)s.B * s.H;
-  const int slots = 2 * 148;
-  const int max_split = std::max(1, s.Nk / (8 * tile));
-  int best = 1;
-  double best_eff = 0.0;
-  for (int n = 1; n <= max_split && n <= 64; ++n) {
-    const int64_t ctas = units * n;
-    const double eff = (double)ctas / (double)(((ctas + slots - 1) / slots) * slots);
-    if (eff > best_eff + 1e-9) best = n, best_eff = eff;
-    if (eff >= 0.95 && ctas >= 2 * slots) break;
-  }
-  nsplit = best;
-  split_len = ((s.Nk + nsplit - 1) / nsplit + tile - 1) / tile * tile;
-  nsplit = (s.Nk + split_len - 1) / split_len;
+// workspace: [counters][partial outputs][partial max, sum][fp16 cos / sin tables]
+struct DecodeWs {
+  size_t done, part_o, part_ml, table, total;
+};
+static DecodeWs decode_ws(const PopeShape& s) {
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t slots = (size_t)s.B * s.H * decode_stream_split(s, false);   // (unit, split, head of the unit)
+  DecodeWs w;
+  w.done = 0;
+  w.part_o = up((size_t)s.B * s.H * sizeof(unsigned int));
+  w.part_ml = w.part_o + up(slots * s.d * sizeof(float));
+  w.table = w.part_ml + up(slots * 2 * sizeof(float));
+  w.total = w.table + up((size_t)s.Nk * s.r * 4);
+  return w;
 }
 
-static size_t decode_partials_bytes(const PopeShape& s, int nsplit) {
-  const int HDP = simt_dch(s.d) * 32;
-  return ((size_t)s.B * s.H * nsplit * (HDP + 2) * sizeof(float) + 255) / 256 * 256;
-}
+size_t decode_stream_workspace(const PopeAttnArgs& a) { return decode_short(a.shape, a.embed) ? 0 : decode_ws(a.shape).total; }
 
-size_t decode_stream_workspace(const PopeAttnArgs& a) {
-  int ns, sl;
-  decode_stream_plan(a.shape, ns, sl);
-  return decode_partials_bytes(a.shape, ns) + (((size_t)a.shape.Nk * a.shape.r * 4 + 255) & ~(size_t)255);
-}
-
-cudaError_t launch_split_combine(const PopeAttnArgs& a, int nsplit, float* part_o, float* part_ml, cudaStream_t st);
-
-template <typename T, int D, int LPK, int KPL, int NW, int MINB>
+template <typename T, int D, int G, int LPK, int E, int NW, bool SHORT>
 static cudaError_t launch_decode_stream(const PopeAttnArgs& a, cudaStream_t st, const PopePagedKV* kv) {
-  constexpr int DS_WORKERS = NW, DS_THREADS = 32 * (NW + 1);
   const PopeShape& s = a.shape;
   DecodeStreamP p = {};
   p.H = s.H, p.Hk = s.Hk, p.Nk = s.Nk, p.r = s.r;
-  decode_stream_plan(s, p.nsplit, p.split_len);
-  p.HDP = simt_dch(s.d) * 32;
+  p.nsplit = decode_stream_split(s, SHORT), p.head_blocks = s.H / s.Hk / G;
   p.scale_log2 = a.softmax_scale * LOG2E;
   p.q = a.q, p.k = a.k, p.v = a.v, p.sq = a.sq, p.sk = a.sk, p.sv = a.sv;
+  p.out = a.out, p.so = a.so, p.lse = a.lse;
   p.k_rows_contiguous = a.sk.n == s.d, p.v_rows_contiguous = a.sv.n == s.d;
   p.freqs = a.embed.freqs, p.bias = a.embed.bias, p.sfn = a.embed.sf.n, p.bias_sh = a.embed.bias_stride_h;
   p.mask = a.mask, p.msb = a.mask_stride_b, p.msn = a.mask_stride_n;
+  const int tiles = (s.Nk + DS_TILE - 1) / DS_TILE;
   if (kv) {
     p.page_table = kv->page_table, p.seq_lens = kv->seq_lens;
     p.page_size = kv->page_size, p.max_pages = kv->max_pages_per_seq, p.num_pages = kv->num_pages;
     p.page_stride = (int64_t)s.Hk * kv->page_size * s.d;
-    p.npg_smem = p.split_len / kv->page_size + 2;
+    p.npg_smem = (tiles + p.nsplit - 1) / p.nsplit * DS_TILE / kv->page_size + 2;
   }
-  const size_t slots = (size_t)s.B * s.H * p.nsplit;
-  p.part_o = static_cast<float*>(a.workspace);
-  p.part_ml = p.part_o + slots * p.HDP;
-  __half* ch = reinterpret_cast<__half*>(static_cast<uint8_t*>(a.workspace) + decode_partials_bytes(s, p.nsplit));
+  const DecodeWs ws = decode_ws(s);
+  uint8_t* base = static_cast<uint8_t*>(a.workspace);
+  p.done = reinterpret_cast<unsigned int*>(base + ws.done);
+  p.part_o = reinterpret_cast<float*>(base + ws.part_o), p.part_ml = reinterpret_cast<float*>(base + ws.part_ml);
+  __half* ch = reinterpret_cast<__half*>(base + ws.table);
   __half* sh = ch + (size_t)s.Nk * s.r;
   p.ch = ch, p.sh = sh;
   p.status = tc_status_ptr();
   if (!p.status) return cudaErrorInvalidSymbol;
-  cudaError_t e;
-  if (s.r > 0 && (e = launch_trig_tables(a.embed, s.Nk, s.r, nullptr, nullptr, ch, sh, st)) != cudaSuccess) return e;
-  constexpr int TILE = DS_WORKERS * KPL * 32 / LPK;
-  const size_t stage = (size_t)TILE * (2 * D * 2 + 2 * s.r * 2);
-  const size_t fixed = (2 * D + DS_WORKERS * D + 2 * DS_WORKERS) * sizeof(float) + 2 * 8 * 8 + 64 + (size_t)p.npg_smem * sizeof(int);
+  const size_t stage = (size_t)DS_TILE * (2 * D * 2 + 2 * s.r * 2);
+  const size_t fixed = ((2 + NW) * G * D + NW * G * 2 + G * DS_MAX_SPLIT) * sizeof(float) + 2 * 3 * 8 + 64 +
+                       (size_t)p.npg_smem * sizeof(int);
   // two CTAs per SM: the ring of each takes what half of the shared memory leaves, at most 3 stages
-  // Measured on B200 (8 x 32 x 32768 x 128, r = 64): two keys per lane and two resident CTAs per SM reach 4.67 TB/s;
-  // a deeper ring in one CTA per SM is slower (2.06 ms against 0.92 ms): the workers, not the copies, need the overlap.
-  int nst = (int)((110 * 1024 - fixed) / stage);
-  if (nst < 2) nst = (int)((kMaxDynamicSmem - 1024 - fixed) / stage);   // wide rotations (r = d = 128): one CTA per SM
+  int nst = (int)(((NW == 8 ? 112 : 224) * 1024 - (int64_t)fixed) / (int64_t)stage);
+  if (nst < 2) nst = (int)((kMaxDynamicSmem - 1024 - (int64_t)fixed) / (int64_t)stage);   // wide rotations (r = d = 128): one CTA per SM
   nst = nst > 3 ? 3 : nst;
   if (nst < 2) return cudaErrorInvalidValue;
   p.nstages = nst;
   const size_t smem = nst * stage + fixed;
-  if ((e = ensure_max_smem<attn_decode_stream_kernel<T, D, LPK, KPL, NW, MINB>>()) != cudaSuccess) return e;
-  // behind the table kernel the decode kernel starts as its programmatic dependent (its loader waits for the table);
+  const auto kernel = attn_decode_stream_kernel<T, D, G, LPK, E, NW, SHORT>;
+  cudaError_t e;
+  if ((e = ensure_max_smem<attn_decode_stream_kernel<T, D, G, LPK, E, NW, SHORT>>()) != cudaSuccess) return e;
+  const unsigned units = (unsigned)(s.B * s.H / G);
+  const dim3 grid((unsigned)p.nsplit, units), block(32 * (NW + 1));
+  if constexpr (SHORT) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.nsplit, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+  }
+  // behind the table kernel, which also zeroes the counters, the decode kernel starts as its programmatic dependent;
   // without rotated features it is the first launch of the call and an ordinary one
   if (s.r > 0) {
-    e = launch_dependent(attn_decode_stream_kernel<T, D, LPK, KPL, NW, MINB>, dim3(p.nsplit, s.B * s.H), dim3(DS_THREADS), smem, st, p);
-  } else {
-    attn_decode_stream_kernel<T, D, LPK, KPL, NW, MINB><<<dim3(p.nsplit, s.B * s.H), DS_THREADS, smem, st>>>(p);
-    e = cudaGetLastError();
+    if ((e = launch_trig_tables(a.embed, s.Nk, s.r, nullptr, nullptr, ch, sh, st, 1, 1, p.done, (int)units)) != cudaSuccess) return e;
+    return launch_dependent(kernel, grid, block, smem, st, p);
   }
-  if (e != cudaSuccess) return e;
-  return launch_split_combine(a, p.nsplit, p.part_o, p.part_ml, st);
+  if (p.nsplit > 1 && (e = cudaMemsetAsync(p.done, 0, units * sizeof(unsigned int), st)) != cudaSuccess) return e;
+  kernel<<<grid, block, smem, st>>>(p);
+  return cudaGetLastError();
+}
+
+// LPK and E: 8-byte pieces (E = 4) leave a lane few coordinates of many heads, 16-byte ones (E = 8) fewer loads for one head
+template <typename T, bool SHORT>
+static cudaError_t decode_stream_g(const PopeAttnArgs& a, cudaStream_t st, const PopePagedKV* kv) {
+  const int g = decode_heads(a.shape);
+  switch (a.shape.d) {
+    case 64:
+      return g == 4   ? launch_decode_stream<T, 64, 4, 8, 4, 16, SHORT>(a, st, kv)
+             : g == 2 ? launch_decode_stream<T, 64, 2, 8, 4, 8, SHORT>(a, st, kv)
+                      : launch_decode_stream<T, 64, 1, 8, 4, 8, SHORT>(a, st, kv);
+    case 96:
+      return g == 2 ? launch_decode_stream<T, 96, 2, 8, 4, 8, SHORT>(a, st, kv) : launch_decode_stream<T, 96, 1, 8, 4, 8, SHORT>(a, st, kv);
+    default:
+      return g == 4   ? launch_decode_stream<T, 128, 4, 16, 4, 16, SHORT>(a, st, kv)
+             : g == 2 ? launch_decode_stream<T, 128, 2, 16, 4, 8, SHORT>(a, st, kv)
+                      : launch_decode_stream<T, 128, 1, 8, 8, 8, SHORT>(a, st, kv);
+  }
 }
 
 template <typename T>
 static cudaError_t decode_stream_d(const PopeAttnArgs& a, cudaStream_t st, const PopePagedKV* kv) {
-  switch (a.shape.d) {
-    case 64: return launch_decode_stream<T, 64, 8, 2, 8, 1>(a, st, kv);
-    case 96: return launch_decode_stream<T, 96, 4, 1, 8, 1>(a, st, kv);
-    default: return launch_decode_stream<T, 128, 8, 2, 8, 1>(a, st, kv);
-  }
+  return decode_short(a.shape, a.embed) ? decode_stream_g<T, true>(a, st, kv) : decode_stream_g<T, false>(a, st, kv);
 }
+
+bool decode_is_exact(const PopeAttnArgs& a) { return a.shape.Nk < DS_EXACT_KEYS; }
 
 cudaError_t decode_stream(const PopeAttnArgs& a, cudaStream_t st) {
   return a.shape.dtype == POPE_BF16 ? decode_stream_d<__nv_bfloat16>(a, st, nullptr) : decode_stream_d<__half>(a, st, nullptr);

@@ -156,9 +156,9 @@ inline PhaseSrc phase_src(const PopeEmbed& e) {
 }
 cudaError_t launch_trig_table_f32(const PopeEmbed& e, int n, int r, float* ctab, float* stab, cudaStream_t st);
 // `slices` tables of n x r entries, slice = batch index x tab_heads + head index of a batched caller table (1 slice for a
-// plain (n, r) table); every output pointer may be null
+// plain (n, r) table); every output pointer may be null.  The launch also zeroes `nzero` counters at `zero`.
 cudaError_t launch_trig_tables(const PopeEmbed& e, int n, int r, float* ctab, float* stab, void* ch, void* sh, cudaStream_t st,
-                               int slices = 1, int tab_heads = 1);
+                               int slices = 1, int tab_heads = 1, unsigned int* zero = nullptr, int nzero = 0);
 // slices of the phase table an attention call needs: one per batch entry and / or head that the caller's table tells apart
 inline int table_heads(const PopeEmbed& e, int heads) { return e.sf.h != 0 ? heads : 1; }
 inline int table_slices(const PopeEmbed& e, int batch, int heads) { return (e.sf.b != 0 ? batch : 1) * table_heads(e, heads); }

@@ -55,9 +55,13 @@ constexpr int SIM_THREADS = 320;
 // ch / sh (may be null): the same tables rounded to fp16 (cos and sin lie in [-1, 1]: 2^-12 absolute error), read by
 // the operand-image pre-pass, whose result is rounded to 8 or 11 bits anyway.
 // grid.y = table slice (batch entry x head of a batched caller table)
-__global__ void pope_trig_table_f32_kernel(PhaseSrc src, int n, int r, float* ctab, float* stab, __half* ch, __half* sh) {
+// `zero` (may be null): nzero counters that the kernel behind this one wants to find at 0
+__global__ void pope_trig_table_f32_kernel(PhaseSrc src, int n, int r, float* ctab, float* stab, __half* ch, __half* sh, unsigned int* zero,
+                                           int nzero) {
   pdl_trigger();   // the kernel behind this one may set itself up; it waits for this grid before it reads the tables
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (zero && blockIdx.y == 0)
+    for (int64_t i = idx; i < nzero; i += (int64_t)gridDim.x * blockDim.x) zero[i] = 0u;
   if (idx >= (int64_t)n * r) return;
   const int pos = idx / r, c = idx % r, slice = blockIdx.y;
   if (!src.pos) src.freqs += (slice / src.tab_heads) * src.sfb + (slice % src.tab_heads) * src.sfh;
@@ -69,12 +73,12 @@ __global__ void pope_trig_table_f32_kernel(PhaseSrc src, int n, int r, float* ct
 }
 
 cudaError_t launch_trig_tables(const PopeEmbed& e, int n, int r, float* ctab, float* stab, void* ch, void* sh, cudaStream_t st,
-                               int slices, int tab_heads) {
+                               int slices, int tab_heads, unsigned int* zero, int nzero) {
   const int64_t total = (int64_t)n * r;
   PhaseSrc src = phase_src(e);
   src.tab_heads = tab_heads;
   pope_trig_table_f32_kernel<<<dim3((unsigned)((total + 255) / 256), (unsigned)slices), 256, 0, st>>>(
-      src, n, r, ctab, stab, static_cast<__half*>(ch), static_cast<__half*>(sh));
+      src, n, r, ctab, stab, static_cast<__half*>(ch), static_cast<__half*>(sh), zero, nzero);
   return cudaGetLastError();
 }
 cudaError_t launch_trig_table_f32(const PopeEmbed& e, int n, int r, float* ctab, float* stab, cudaStream_t st) {
