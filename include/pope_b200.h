@@ -244,7 +244,7 @@ typedef struct PopePagedKV {
 
 /* Append n_new rows per sequence: k, v (B, Hk, n_new, d) with element strides, written at positions
  * [seq_lens[b], seq_lens[b] + n_new) of sequence b; the table must already map those positions.  With
- * `advance` nonzero seq_lens[b] += n_new afterwards (a second tiny launch on the same stream). */
+ * `advance` nonzero seq_lens[b] += n_new afterwards (on the same stream; a launch of its own for long inputs). */
 typedef struct PopeKvAppendArgs {
   uint32_t struct_bytes;
   int32_t dtype;               /* PopeDtype: POPE_BF16 or POPE_F16 */
@@ -254,6 +254,18 @@ typedef struct PopeKvAppendArgs {
   const void* k; PopeStride3 sk;
   const void* v; PopeStride3 sv;
 } PopeKvAppendArgs;
+
+/* Host bookkeeping -> device: n assignments that travel as kernel parameters (no copy, no synchronisation).  index and
+ * value are HOST arrays: index[i] >= 0 sets page_table[index[i]] = value[i], index[i] < 0 sets
+ * seq_lens[-1 - index[i]] = value[i]. */
+typedef struct PopeKvMapArgs {
+  uint32_t struct_bytes;
+  int32_t n, B, max_pages_per_seq;   /* indices lie in [-B, B * max_pages_per_seq) */
+  int32_t* page_table;
+  int32_t* seq_lens;
+  const int32_t* index;
+  const int32_t* value;
+} PopeKvMapArgs;
 
 /* One query row per (batch, head) against the cached keys of its sequence: out = softmax(q' K'^T scale) V
  * with the query at the LAST cached position, seq_lens[b] - 1 (PoPE_pytorch/pope.py:64 and
@@ -344,6 +356,7 @@ POPE_API int pope_b200_attn_bwd(const PopeAttnBwdArgs* args, void* stream);
 POPE_API int pope_b200_apply_qk_fwd(const PopeApplyArgs* args, void* stream);
 POPE_API int pope_b200_apply_qk_bwd(const PopeApplyBwdArgs* args, void* stream);
 POPE_API int pope_b200_kv_append(const PopeKvAppendArgs* args, void* stream);
+POPE_API int pope_b200_kv_map(const PopeKvMapArgs* args, void* stream);
 POPE_API int pope_b200_attn_decode_paged(const PopePagedDecodeArgs* args, void* stream);
 POPE_API int pope_b200_table(const PopeTableArgs* args, void* stream);
 POPE_API int pope_b200_clamp_bwd(const PopeClampBwdArgs* args, void* stream);

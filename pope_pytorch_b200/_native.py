@@ -111,7 +111,7 @@ class PagedDecodeArgs(C.Structure):
 EXPORTS = ("pope_b200_abi_version", "pope_b200_apply_qk_fwd", "pope_b200_apply_qk_bwd", "pope_b200_status_str", "pope_b200_last_path", "pope_b200_device_status",
            "pope_b200_clear_device_status", "pope_b200_selftest_bounded_wait",
            "pope_b200_workspace_bytes", "pope_b200_attn_fwd_noalloc", "pope_b200_kv_append", "pope_b200_attn_decode_paged",
-           "pope_b200_table", "pope_b200_clamp_bwd",
+           "pope_b200_table", "pope_b200_clamp_bwd", "pope_b200_kv_map",
            "pope_b200_sim_fwd", "pope_b200_sim_bwd", "pope_b200_attn_fwd", "pope_b200_attn_bwd")
 
 _lib = None
@@ -128,7 +128,7 @@ def _bind(lib):
     lib.pope_b200_workspace_bytes.argtypes = [C.c_int, C.c_void_p]
     for name in ("pope_b200_sim_fwd", "pope_b200_sim_bwd", "pope_b200_attn_fwd", "pope_b200_attn_bwd",
                  "pope_b200_apply_qk_fwd", "pope_b200_apply_qk_bwd", "pope_b200_kv_append", "pope_b200_attn_decode_paged",
-                 "pope_b200_table", "pope_b200_clamp_bwd"):
+                 "pope_b200_table", "pope_b200_clamp_bwd", "pope_b200_kv_map"):
         fn = getattr(lib, name)
         fn.restype = C.c_int
         fn.argtypes = [C.c_void_p, C.c_void_p]

@@ -240,6 +240,16 @@ int pope_b200_kv_append(const PopeKvAppendArgs* a, void* stream) {
   return POPE_OK;
 }
 
+int pope_b200_kv_map(const PopeKvMapArgs* a, void* stream) {
+  if (!a || a->struct_bytes != sizeof(PopeKvMapArgs) || a->n < 0 || a->B <= 0 || a->max_pages_per_seq <= 0) return POPE_ERR_BAD_ARG;
+  if (!a->page_table || !a->seq_lens || (a->n > 0 && (!a->index || !a->value))) return POPE_ERR_BAD_ARG;
+  for (int i = 0; i < a->n; ++i)
+    if (a->index[i] < -a->B || a->index[i] >= (int64_t)a->B * a->max_pages_per_seq) return POPE_ERR_BAD_ARG;
+  const int rc = check_device();
+  if (rc != POPE_OK) return rc;
+  return pope::kv_map(*a, static_cast<cudaStream_t>(stream)) == cudaSuccess ? POPE_OK : POPE_ERR_CUDA;
+}
+
 int pope_b200_attn_decode_paged(const PopePagedDecodeArgs* a, void* stream) {
   if (!a || a->struct_bytes != sizeof(PopePagedDecodeArgs)) return POPE_ERR_BAD_ARG;
   int rc = check_shape(a->shape);

@@ -154,6 +154,11 @@ __global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_st
   auto head = [&](int g) { return hk + (hb * G + g) * p.Hk; };   // query head h reads key head h % Hk
   const T* kbase = (const T*)p.k + b * p.sk.b + hk * p.sk.h;
   const T* vbase = (const T*)p.v + b * p.sv.b + hk * p.sv.h;
+  if (tid == 0) {
+    for (int s = 0; s < p.nstages; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], NW);
+    mbar_init_fence();
+  }
+  if (SHORT) pdl_wait();   // (first kernel of its call: nothing in global memory may be touched earlier)
   // keys of this sequence (paged cache: its own length, at most the bound the split was planned for), cut evenly
   const int nk = p.seq_lens ? max(0, min(p.seq_lens[b], p.Nk)) : p.Nk;
   const int tiles_all = (nk + TILE - 1) / TILE;
@@ -161,10 +166,6 @@ __global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_st
   const int ke = min(nk, (int)((int64_t)tiles_all * (blockIdx.x + 1) / p.nsplit) * TILE);
   const int T_tiles = ke > kb ? (ke - kb + TILE - 1) / TILE : 0;
 
-  if (tid == 0) {
-    for (int s = 0; s < p.nstages; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], NW);
-    mbar_init_fence();
-  }
   if (p.page_table) {
     // page indices of [kb, ke); an index outside the pool is never dereferenced (clamped, status bit 1)
     for (int i = tid; i < p.npg_smem; i += blockDim.x) {
@@ -674,10 +675,12 @@ static cudaError_t launch_decode_stream(const PopeAttnArgs& a, cudaStream_t st, 
   if constexpr (SHORT) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)p.nsplit, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr, cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr, cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, p);
   }
   // behind the table kernel, which also zeroes the counters, the decode kernel starts as its programmatic dependent;
@@ -773,12 +776,8 @@ struct KvAppendP {
 // One thread per 16 bytes of a new row of k and of v.  A position past the table or a page index outside the pool is
 // skipped and reported through status bit 1.
 template <typename T>
-__global__ void __launch_bounds__(256) kv_append_kernel(KvAppendP p) {
-  const int cpr = p.d >> 3;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= p.n_new * cpr) return;
-  const int i = idx / cpr, c = idx - i * cpr, hk = blockIdx.y, b = blockIdx.z;
-  const int pos = p.seq_lens[b] + i, lp = pos / p.page_size;
+__device__ __forceinline__ void append_group(const KvAppendP& p, int b, int hk, int i, int c, int len) {
+  const int pos = len + i, lp = pos / p.page_size;
   if (pos < 0 || lp >= p.max_pages) { atomicOr(p.status, 2u); return; }
   const int pg = p.page_table[(int64_t)b * p.max_pages + lp];
   if (pg < 0 || pg >= p.num_pages) { atomicOr(p.status, 2u); return; }
@@ -787,6 +786,29 @@ __global__ void __launch_bounds__(256) kv_append_kernel(KvAppendP p) {
   const T* vrow = static_cast<const T*>(p.v) + b * p.sv.b + hk * p.sv.h + (int64_t)i * p.sv.n + c * 8;
   *reinterpret_cast<uint4*>(static_cast<T*>(p.k_pages) + dst) = __ldg(reinterpret_cast<const uint4*>(krow));
   *reinterpret_cast<uint4*>(static_cast<T*>(p.v_pages) + dst) = __ldg(reinterpret_cast<const uint4*>(vrow));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) kv_append_kernel(KvAppendP p) {
+  const int cpr = p.d >> 3;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= p.n_new * cpr) return;
+  append_group<T>(p, blockIdx.z, blockIdx.y, idx / cpr, idx % cpr, p.seq_lens[blockIdx.z]);
+}
+
+// The rows of a few tokens (a decode step): one CTA per sequence, which therefore may advance the length itself when all
+// of its threads have read it -- a decode step is bound by its launches.
+constexpr int KV_STEP_GROUPS = 4096;   // 16-byte groups of k per sequence that one CTA still copies in a few microseconds
+template <typename T>
+__global__ void __launch_bounds__(256) kv_append_step_kernel(KvAppendP p, int advance) {
+  pdl_wait();
+  const int cpr = p.d >> 3, b = blockIdx.x, len = p.seq_lens[b];
+  for (int idx = threadIdx.x; idx < p.Hk * p.n_new * cpr; idx += 256) {
+    const int row = idx / cpr;
+    append_group<T>(p, b, row / p.n_new, row % p.n_new, idx % cpr, len);
+  }
+  __syncthreads();
+  if (advance && threadIdx.x == 0) p.seq_lens[b] = len + p.n_new;
 }
 
 __global__ void kv_advance_kernel(int32_t* seq_lens, int B, int n_new) {
@@ -803,8 +825,11 @@ cudaError_t kv_append(const PopeKvAppendArgs& g, cudaStream_t st) {
   p.k_pages = g.kv.k_pages, p.v_pages = g.kv.v_pages, p.page_table = g.kv.page_table, p.seq_lens = g.kv.seq_lens;
   p.status = tc_status_ptr();
   if (!p.status) return cudaErrorInvalidSymbol;
-  const dim3 grid((unsigned)((g.n_new * (g.d / 8) + 255) / 256), (unsigned)g.Hk, (unsigned)g.B);
   // (both 16-bit types move as raw 16-byte groups)
+  if ((int64_t)g.Hk * g.n_new * (g.d / 8) <= KV_STEP_GROUPS) {
+    return launch_dependent(kv_append_step_kernel<__nv_bfloat16>, dim3(g.B), dim3(256), 0, st, p, (int)g.advance);
+  }
+  const dim3 grid((unsigned)((g.n_new * (g.d / 8) + 255) / 256), (unsigned)g.Hk, (unsigned)g.B);
   kv_append_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -813,6 +838,29 @@ cudaError_t kv_append(const PopeKvAppendArgs& g, cudaStream_t st) {
     e = cudaGetLastError();
   }
   return e;
+}
+
+constexpr int KV_MAP_BATCH = 128;
+struct KvMapBatch {
+  int32_t n, index[KV_MAP_BATCH], value[KV_MAP_BATCH];
+};
+__global__ void kv_map_kernel(const __grid_constant__ KvMapBatch m, int32_t* page_table, int32_t* seq_lens) {
+  const int i = threadIdx.x;
+  pdl_wait();
+  if (i >= m.n) return;
+  if (m.index[i] >= 0) page_table[m.index[i]] = m.value[i];
+  else seq_lens[-1 - m.index[i]] = m.value[i];
+}
+
+cudaError_t kv_map(const PopeKvMapArgs& a, cudaStream_t st) {
+  for (int first = 0; first < a.n; first += KV_MAP_BATCH) {
+    KvMapBatch m;
+    m.n = std::min(a.n - first, KV_MAP_BATCH);
+    std::copy_n(a.index + first, m.n, m.index), std::copy_n(a.value + first, m.n, m.value);
+    const cudaError_t e = launch_dependent(kv_map_kernel, dim3(1), dim3(KV_MAP_BATCH), 0, st, m, a.page_table, a.seq_lens);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace pope

@@ -31,6 +31,7 @@ bool decode_paged_supported(const PopePagedDecodeArgs& a);
 size_t decode_paged_workspace(const PopePagedDecodeArgs& a);
 cudaError_t decode_paged(const PopePagedDecodeArgs& a, cudaStream_t st);
 cudaError_t kv_append(const PopeKvAppendArgs& a, cudaStream_t st);
+cudaError_t kv_map(const PopeKvMapArgs& a, cudaStream_t st);
 // phase table, clamped bias and the clamp's gradient
 cudaError_t pope_table(const PopeTableArgs& a, cudaStream_t st);
 cudaError_t pope_clamp_bwd(const PopeClampBwdArgs& a, cudaStream_t st);

@@ -399,6 +399,63 @@ optional<std::vector<Tensor>> table(const Tensor& bias, const std::vector<Tensor
   return Table::apply(bias, &inv, &dims, offset);
 }
 
+// ---- paged key / value cache ---------------------------------------------------------------------------------------
+// The cache's tensors; `row` > 0 = the view that starts at sequence `row` (a batch of one)
+struct Pages {
+  Tensor k, v, table, lens;
+  PopePagedKV view(int64_t row = 0) const {
+    PopePagedKV kv = {};
+    kv.k_pages = k.mutable_data_ptr(), kv.v_pages = v.mutable_data_ptr();
+    kv.page_table = table.const_data_ptr<int32_t>() + row * table.size(1), kv.seq_lens = lens.mutable_data_ptr<int32_t>() + row;
+    kv.num_pages = (int32_t)k.size(0), kv.page_size = (int32_t)k.size(2), kv.max_pages_per_seq = (int32_t)table.size(1);
+    return kv;
+  }
+};
+
+void kv_map(const Pages& p, const std::vector<int32_t>& index, const std::vector<int32_t>& value) {
+  py::gil_scoped_release nogil;
+  c10::cuda::OptionalCUDAGuard guard(p.k.device());
+  PopeKvMapArgs a = {};
+  a.struct_bytes = sizeof(a), a.n = (int32_t)index.size(), a.B = (int32_t)p.lens.size(0), a.max_pages_per_seq = (int32_t)p.table.size(1);
+  a.page_table = p.table.mutable_data_ptr<int32_t>(), a.seq_lens = p.lens.mutable_data_ptr<int32_t>();
+  a.index = index.data(), a.value = value.data();
+  check(pope_b200_kv_map(&a, stream_of(p.k)), "pope_b200_kv_map");
+}
+
+// k, v (b, hk, n, d), or (hk, n, d) for sequence `row` alone
+void kv_append(const Pages& p, const Tensor& k_, const Tensor& v_, int64_t row) {
+  py::gil_scoped_release nogil;
+  c10::cuda::OptionalCUDAGuard guard(p.k.device());
+  at::NoGradGuard off;
+  const Tensor k = inner_contig(k_), v = inner_contig(v_);
+  const bool one = k.dim() == 3;
+  const int64_t h = one ? 0 : 1;
+  TORCH_CHECK_INDEX(row >= 0 && row + (one ? 1 : k.size(0)) <= p.lens.size(0), "sequence ", row, " is not in the cache");
+  PopeKvAppendArgs a = {};
+  a.struct_bytes = sizeof(a), a.dtype = dtype_of(k), a.B = one ? 1 : (int32_t)k.size(0), a.Hk = (int32_t)k.size(h), a.d = (int32_t)k.size(h + 2);
+  a.n_new = (int32_t)k.size(h + 1), a.advance = 1, a.kv = p.view(row);
+  a.k = k.const_data_ptr(), a.sk = {one ? 0 : k.stride(0), k.stride(h), k.stride(h + 1)};
+  a.v = v.const_data_ptr(), a.sv = {one ? 0 : v.stride(0), v.stride(h), v.stride(h + 1)};
+  check(pope_b200_kv_append(&a, stream_of(k)), "pope_b200_kv_append");
+}
+
+std::tuple<Tensor, Tensor> kv_decode(const Pages& p, const Tensor& q_, const Tensor& freqs_, const Tensor& bias_, double scale, int64_t nk) {
+  py::gil_scoped_release nogil;
+  c10::cuda::OptionalCUDAGuard guard(p.k.device());
+  at::NoGradGuard off;
+  const Tensor q = inner_contig(q_), freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
+  const int r = (int)freqs.size(-1);
+  Tensor out = at::empty_like(q), lse = at::empty({q.size(0), q.size(1)}, q.options().dtype(at::kFloat));
+  PopePagedDecodeArgs a = {};
+  a.struct_bytes = sizeof(a), a.softmax_scale = (float)scale;
+  a.shape = {(int32_t)q.size(0), (int32_t)q.size(1), (int32_t)p.k.size(1), 1, (int32_t)nk, (int32_t)q.size(3), r, dtype_of(q)};
+  a.embed = embed_of(freqs, bias, r), a.kv = p.view();
+  a.q = q.const_data_ptr(), a.sq = s3(q), a.out = out.mutable_data_ptr(), a.so = s3(out), a.lse = lse.mutable_data_ptr<float>();
+  const Tensor ws = workspace(POPE_OP_DECODE_PAGED, a, q);
+  check(pope_b200_attn_decode_paged(&a, stream_of(q)), "pope_b200_attn_decode_paged");
+  return {out, lse};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -406,6 +463,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("similarity", &similarity);
   m.def("apply_qk", &apply_qk);
   m.def("table", &table);
+  py::class_<Pages>(m, "Pages").def(py::init([](Tensor k, Tensor v, Tensor table, Tensor lens) { return Pages{k, v, table, lens}; }));
+  m.def("kv_map", &kv_map);
+  m.def("kv_append", &kv_append);
+  m.def("kv_decode", &kv_decode);
   m.def("attn_forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask,
                            bool causal, double scale, const Factors& factors) {
     validate(q, k, freqs, false);

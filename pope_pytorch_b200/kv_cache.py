@@ -13,7 +13,6 @@ in the CUDA library; there is no fallback.
 """
 from __future__ import annotations
 
-import ctypes as C
 from typing import List, Optional, Sequence
 
 import torch
@@ -42,7 +41,10 @@ class PageAllocator:
         """Map the pages that ``n_new`` more keys per sequence need; returns the new (b, logical, physical) entries.
         Raises (and changes nothing) when the pool or a sequence's table is too small."""
         rows = range(self.batch) if rows is None else rows
-        want = [(b, self.pages_needed(b, n_new)) for b in rows]
+        lens, table, size = self.lens, self.table, self.page_size
+        want = [(b, n) for b in rows if (n := -(-(lens[b] + n_new) // size) - len(table[b])) > 0]
+        if not want:      # nearly every step of a decode loop
+            return []
         if sum(n for _, n in want) > len(self.free):
             raise RuntimeError("paged KV cache: out of pages")
         for b, n in want:
@@ -90,6 +92,7 @@ class PagedKVCache:
         self.device = self.k_pages.device   # with its index
         self.page_table = torch.zeros(batch, max_pages, dtype=torch.int32, device=self.device)
         self.seq_lens = torch.zeros(batch, dtype=torch.int32, device=self.device)
+        self._held = None
 
     # ---- bookkeeping -------------------------------------------------------------------------------
     @property
@@ -104,28 +107,27 @@ class PagedKVCache:
     def max_len(self) -> int:
         return max(self.alloc.lens)
 
-    def _kv_struct(self, row: int = 0) -> N.PagedKV:
-        """The cache as the C ABI sees it; ``row`` > 0 = the view that starts at sequence ``row`` (a batch of one)."""
-        return N.PagedKV(self.k_pages.data_ptr(), self.v_pages.data_ptr(),
-                         self.page_table.data_ptr() + 4 * row * self.alloc.max_pages_per_seq, self.seq_lens.data_ptr() + 4 * row,
-                         self.alloc.num_pages, self.alloc.page_size, self.alloc.max_pages_per_seq, 0)
+    def _pages(self):
+        """The cache's tensors as the binding takes them (they are fixed for the life of the cache)."""
+        held = self._held
+        if held is None or held[0] is not self.k_pages or held[1] is not self.v_pages or held[2] is not self.page_table or held[3] is not self.seq_lens:
+            tensors = (self.k_pages, self.v_pages, self.page_table, self.seq_lens)
+            self._held = held = (*tensors, N._ops().Pages(*tensors))
+        return held[4]
 
     def _push_table(self, new_entries) -> None:
-        if not new_entries:
-            return
-        idx = torch.tensor([[b, lp] for b, lp, _ in new_entries], dtype=torch.long)
-        val = torch.tensor([pg for _, _, pg in new_entries], dtype=torch.int32)
-        self.page_table[idx[:, 0].to(self.device), idx[:, 1].to(self.device)] = val.to(self.device)
+        if new_entries:
+            width = self.alloc.max_pages_per_seq
+            N._ops().kv_map(self._pages(), [b * width + lp for b, lp, _ in new_entries], [pg for _, _, pg in new_entries])
 
     def release(self, b: int) -> None:
         """Forget sequence ``b`` and free its pages."""
         self.alloc.release(b)
-        self.seq_lens[b] = 0
+        N._ops().kv_map(self._pages(), [-1 - (b % self.batch)], [0])
 
     # ---- the two operators -------------------------------------------------------------------------
     def append(self, k: torch.Tensor, v: torch.Tensor) -> None:
         """k, v: (batch, kv_heads, n_new, head_dim) views with contiguous features; every sequence grows by n_new."""
-        lib = N.load_library()
         if k.shape != v.shape or k.ndim != 4 or k.shape[0] != self.batch or k.shape[1] != self.kv_heads or k.shape[3] != self.head_dim:
             raise ValueError("k and v must be (batch, kv_heads, n_new, head_dim)")
         if k.dtype != self.dtype or v.dtype != self.dtype or k.device != self.device or v.device != self.device:
@@ -133,17 +135,12 @@ class PagedKVCache:
         n_new = k.shape[2]
         if n_new == 0:
             return
-        k, v = N._inner_contig(k), N._inner_contig(v)
         self._push_table(self.alloc.reserve(n_new))
-        a = N.KvAppendArgs(C.sizeof(N.KvAppendArgs), N._DTYPES[self.dtype], self.batch, self.kv_heads, self.head_dim, n_new, 1, 0,
-                           self._kv_struct(), k.data_ptr(), N._s3(k), v.data_ptr(), N._s3(v))
-        with N._on_device(self.device):
-            N._check(lib.pope_b200_kv_append(C.addressof(a), N._stream_ptr(k)), "pope_b200_kv_append")
+        N._ops().kv_append(self._pages(), k, v, 0)
         self.alloc.advance(n_new)
 
     def append_to(self, b: int, k: torch.Tensor, v: torch.Tensor) -> None:
         """k, v: (kv_heads, n_new, head_dim) appended to sequence ``b`` only (ragged prompts)."""
-        lib = N.load_library()
         if k.shape != v.shape or k.ndim != 3 or k.shape[0] != self.kv_heads or k.shape[2] != self.head_dim:
             raise ValueError("k and v must be (kv_heads, n_new, head_dim)")
         if k.dtype != self.dtype or v.dtype != self.dtype or k.device != self.device or v.device != self.device:
@@ -151,18 +148,13 @@ class PagedKVCache:
         n_new = k.shape[1]
         if n_new == 0:
             return
-        k, v = N._inner_contig(k).unsqueeze(0), N._inner_contig(v).unsqueeze(0)
         self._push_table(self.alloc.reserve(n_new, rows=[b]))
-        a = N.KvAppendArgs(C.sizeof(N.KvAppendArgs), N._DTYPES[self.dtype], 1, self.kv_heads, self.head_dim, n_new, 1, 0,
-                           self._kv_struct(b), k.data_ptr(), N._s3(k), v.data_ptr(), N._s3(v))
-        with N._on_device(self.device):
-            N._check(lib.pope_b200_kv_append(C.addressof(a), N._stream_ptr(k)), "pope_b200_kv_append")
+        N._ops().kv_append(self._pages(), k, v, b)
         self.alloc.advance(n_new, rows=[b])
 
     def decode(self, q: torch.Tensor, pos_emb, softmax_scale: Optional[float] = None, return_lse: bool = False):
         """q: (batch, heads, 1, head_dim); pos_emb: (freqs, bias) with at least ``max_len`` rows of freqs.
         Returns out (batch, heads, 1, head_dim) in q's dtype (and lse (batch, heads) on request)."""
-        lib = N.load_library()
         freqs, bias = pos_emb
         if q.ndim != 4 or q.shape[0] != self.batch or q.shape[2] != 1 or q.shape[3] != self.head_dim or q.shape[1] % self.kv_heads != 0:
             raise ValueError("q must be (batch, heads, 1, head_dim) with heads a multiple of kv_heads")
@@ -173,18 +165,8 @@ class PagedKVCache:
             raise ValueError("the paged decode takes a (positions, rotate_dim) table")
         if r > 0 and freqs.shape[0] < nk:
             raise ValueError("freqs must cover every cached position")
-        q = N._inner_contig(q)
-        freqs, bias = N._prep_embed(freqs[:nk] if r > 0 else freqs, bias, nk, r)
-        out = torch.empty_like(q)
-        lse = torch.empty(q.shape[0], q.shape[1], dtype=torch.float32, device=self.device)
         scale = self.head_dim ** -0.5 if softmax_scale is None else softmax_scale
-        shape = N.Shape(self.batch, q.shape[1], self.kv_heads, 1, nk, self.head_dim, r, N._DTYPES[self.dtype])
-        a = N.PagedDecodeArgs(C.sizeof(N.PagedDecodeArgs), float(scale), shape, N._embed_struct(freqs, bias, r), self._kv_struct(),
-                              q.data_ptr(), N._s3(q), out.data_ptr(), N._s3(out), lse.data_ptr(), None, 0)
-        ws = N._workspace(N.OP_DECODE_PAGED, a, self.device)
-        with N._on_device(self.device):
-            N._check(lib.pope_b200_attn_decode_paged(C.addressof(a), N._stream_ptr(q)), "pope_b200_attn_decode_paged")
-        del ws
+        out, lse = N._ops().kv_decode(self._pages(), q, freqs, bias, scale, nk)
         return (out, lse) if return_lse else out
 
     # ---- for tests and debugging -------------------------------------------------------------------
