@@ -94,13 +94,13 @@ size_t pope_b200_workspace_bytes(int op, const void* args) {
       if (a.struct_bytes != sizeof(PopeAttnArgs) || check_shape(a.shape) != POPE_OK) return 0;
       if (!force_simt() && pope::attn_fwd_tc_supported(a)) return pope::attn_fwd_tc_workspace(a);
       if (!force_simt() && pope::decode_stream_supported(a)) return pope::decode_stream_workspace(a);
-      return pope::attn_fwd_simt_workspace(a);
+      return pope::attn_fwd_tiled_supported(a.shape) ? pope::attn_fwd_tiled_workspace(a.shape) : pope::attn_fwd_simt_workspace(a);
     }
     case POPE_OP_ATTN_BWD: {
       const PopeAttnBwdArgs& a = *static_cast<const PopeAttnBwdArgs*>(args);
       if (a.struct_bytes != sizeof(PopeAttnBwdArgs) || check_shape(a.shape) != POPE_OK) return 0;
       if (!force_simt() && pope::attn_bwd_tc_supported(a)) return pope::attn_bwd_tc_workspace(a);
-      return pope::attn_bwd_simt_workspace(a);
+      return pope::attn_bwd_tiled_supported(a.shape) ? pope::attn_bwd_tiled_workspace(a.shape) : pope::attn_bwd_simt_workspace(a);
     }
     case POPE_OP_DECODE_PAGED: {
       const PopePagedDecodeArgs& a = *static_cast<const PopePagedDecodeArgs*>(args);
@@ -153,12 +153,21 @@ int pope_b200_attn_fwd(const PopeAttnArgs* a, void* stream) {
   if (a->shape.d > 256) return POPE_ERR_UNSUPPORTED;
   const bool tc = !force_simt() && pope::attn_fwd_tc_supported(*a);
   const bool dec = !tc && !force_simt() && pope::decode_stream_supported(*a);
-  const size_t need = tc ? pope::attn_fwd_tc_workspace(*a) : dec ? pope::decode_stream_workspace(*a) : pope::attn_fwd_simt_workspace(*a);
+  // (a caller that passes no workspace, as the exact family once needed none, gets the kernels that work without)
+  const bool tiled = !tc && !dec && pope::attn_fwd_tiled_supported(a->shape) && a->workspace &&
+                     a->workspace_bytes >= pope::attn_fwd_tiled_workspace(a->shape);
+  const size_t need = tc      ? pope::attn_fwd_tc_workspace(*a)
+                      : dec   ? pope::decode_stream_workspace(*a)
+                      : tiled ? pope::attn_fwd_tiled_workspace(a->shape)
+                              : pope::attn_fwd_simt_workspace(*a);
   if (need > 0 && (!a->workspace || a->workspace_bytes < need)) return POPE_ERR_WORKSPACE;
   if (need > 0 && (reinterpret_cast<uintptr_t>(a->workspace) & 15) != 0) return POPE_ERR_MISALIGNED;
   if ((rc = check_device()) != POPE_OK) return rc;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const cudaError_t e = tc ? pope::attn_fwd_tc(*a, st) : dec ? pope::decode_stream(*a, st) : pope::attn_fwd_simt(*a, st);
+  const cudaError_t e = tc      ? pope::attn_fwd_tc(*a, st)
+                        : dec   ? pope::decode_stream(*a, st)
+                        : tiled ? pope::attn_fwd_tiled(*a, st)
+                                : pope::attn_fwd_simt(*a, st);
   if (e != cudaSuccess) return POPE_ERR_CUDA;
   g_last_path = tc ? "tcgen05" : dec && !pope::decode_is_exact(*a) ? "decode_stream" : "simt";
   return POPE_OK;
@@ -172,12 +181,13 @@ int pope_b200_attn_bwd(const PopeAttnBwdArgs* a, void* stream) {
   if (!a->q || !a->k || !a->v || !a->out || !a->dout || !a->lse || !a->dq || !a->dk || !a->dv) return POPE_ERR_BAD_ARG;
   if (a->shape.d > 256) return POPE_ERR_UNSUPPORTED;
   const bool tc = !force_simt() && pope::attn_bwd_tc_supported(*a);
-  const size_t need = tc ? pope::attn_bwd_tc_workspace(*a) : pope::attn_bwd_simt_workspace(*a);
+  const bool tiled = !tc && pope::attn_bwd_tiled_supported(a->shape) && a->workspace && a->workspace_bytes >= pope::attn_bwd_tiled_workspace(a->shape);
+  const size_t need = tc ? pope::attn_bwd_tc_workspace(*a) : tiled ? pope::attn_bwd_tiled_workspace(a->shape) : pope::attn_bwd_simt_workspace(*a);
   if (!a->workspace || a->workspace_bytes < need) return POPE_ERR_WORKSPACE;
   if ((reinterpret_cast<uintptr_t>(a->workspace) & 15) != 0) return POPE_ERR_MISALIGNED;
   if ((rc = check_device()) != POPE_OK) return rc;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if ((tc ? pope::attn_bwd_tc(*a, st) : pope::attn_bwd_simt(*a, st)) != cudaSuccess) return POPE_ERR_CUDA;
+  if ((tc ? pope::attn_bwd_tc(*a, st) : tiled ? pope::attn_bwd_tiled(*a, st) : pope::attn_bwd_simt(*a, st)) != cudaSuccess) return POPE_ERR_CUDA;
   g_last_path = tc ? "tcgen05" : "simt";
   return POPE_OK;
 }

@@ -5,13 +5,14 @@
 // work between them are the whole cost (a training step at (2, 8, 2048, 96) spent 0.25 of its 0.53 ms there).  One kernel
 // writes everything: positions, freqs[p][c] = positions[p][axis(c)] * inv_freqs[c] (one fp32 multiply, as the module does
 // it), the flat inverse frequencies and axis numbers that the factored form needs, and the clamped bias.
-#include "common.cuh"
 #include "kernels.h"
+#include "tc_common.cuh"
 
 namespace pope {
 
 // One thread per (position, feature); the threads behind the table take the bias and the small vectors.
 __global__ void __launch_bounds__(256) pope_table_kernel(PopeTableArgs p, int n, int r) {
+  pdl_wait();
   const int64_t total = (int64_t)n * r, bias_n = p.bias ? (int64_t)p.H * r : 0;
   int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (idx < total) {
@@ -41,20 +42,19 @@ cudaError_t pope_table(const PopeTableArgs& p, cudaStream_t st) {
   for (int a = 0; a < p.axes; ++a) n *= p.dims[a], r += p.width[a];
   const int64_t work = n * r + (p.bias ? (int64_t)p.H * r : 0);
   if (work == 0) return cudaSuccess;
-  pope_table_kernel<<<(unsigned)((work + 255) / 256), 256, 0, st>>>(p, (int)n, r);
-  return cudaGetLastError();
+  return launch_dependent(pope_table_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), 0, st, p, (int)n, r);
 }
 
 __global__ void __launch_bounds__(256) pope_clamp_bwd_kernel(const float* __restrict__ bias, const float* __restrict__ grad,
                                                              float* __restrict__ out, int64_t n) {
+  pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i < n) out[i] = (bias[i] >= POPE_BIAS_MIN && bias[i] <= 0.f) ? grad[i] : 0.f;
 }
 
 cudaError_t pope_clamp_bwd(const PopeClampBwdArgs& p, cudaStream_t st) {
   if (p.n == 0) return cudaSuccess;
-  pope_clamp_bwd_kernel<<<(unsigned)((p.n + 255) / 256), 256, 0, st>>>(p.bias, p.grad, p.grad_bias, p.n);
-  return cudaGetLastError();
+  return launch_dependent(pope_clamp_bwd_kernel, dim3((unsigned)((p.n + 255) / 256)), dim3(256), 0, st, p.bias, p.grad, p.grad_bias, p.n);
 }
 
 }  // namespace pope

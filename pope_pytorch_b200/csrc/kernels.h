@@ -14,6 +14,14 @@ cudaError_t attn_fwd_simt(const PopeAttnArgs& a, cudaStream_t st);
 size_t attn_bwd_simt_workspace(const PopeAttnBwdArgs& a);
 cudaError_t attn_bwd_simt(const PopeAttnBwdArgs& a, cudaStream_t st);
 
+// the same arithmetic in 64 x 64 tiles over operands transformed once per call: Nq >= 32, d + r <= 256 (backward: d <= 128)
+bool attn_fwd_tiled_supported(const PopeShape& s);
+bool attn_bwd_tiled_supported(const PopeShape& s);
+size_t attn_fwd_tiled_workspace(const PopeShape& s);
+size_t attn_bwd_tiled_workspace(const PopeShape& s);
+cudaError_t attn_fwd_tiled(const PopeAttnArgs& a, cudaStream_t st);
+cudaError_t attn_bwd_tiled(const PopeAttnBwdArgs& a, cudaStream_t st);
+
 // tensor-core (tcgen05 + TMEM) family: bf16 / fp16, d in {64, 96, 128}, r % 16 == 0, 2-D freqs
 bool attn_fwd_tc_supported(const PopeAttnArgs& a);
 size_t attn_fwd_tc_workspace(const PopeAttnArgs& a);

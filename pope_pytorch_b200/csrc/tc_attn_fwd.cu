@@ -572,9 +572,9 @@ static cudaError_t launch_fwd_tc(const PopeAttnArgs& a, cudaStream_t st) {
   jobs.job[0] = expand_job(a.k, a.sk, s.B, s.Hk, s.Nk, s.r, 0, a.embed.bias, a.embed.bias_stride_h, kimg, s.Nk, by_batch, tab_heads);
   jobs.job[0].tile128 = 1;
   if (s.r > 0 && (e = launch_trig_tables(a.embed, s.Nk, s.r, nullptr, nullptr, tt.ch, tt.sh, st, slices, tab_heads)) != cudaSuccess) return e;
-  // tables -> images -> attention: the second and third kernel start as programmatic dependents of the one before (each
-  // waits for it before its first read of that kernel's output); the first launch of the chain is an ordinary one
-  if ((e = launch_expand_images(jobs, 1, s.d, bf16, tt.ch, tt.sh, st, s.r > 0)) != cudaSuccess) return e;
+  // tables -> images -> attention, each a programmatic dependent of the kernel before it; the first of them waits for the
+  // work before the call and lets the next one go only then
+  if ((e = launch_expand_images(jobs, 1, s.d, bf16, tt.ch, tt.sh, st)) != cudaSuccess) return e;
   dim3 grid((s.Nq + TQ - 1) / TQ, s.B * s.H);
   return launch_dependent(attn_fwd_tc_kernel<D, T>, grid, dim3(FW_THREADS), smem, st, p, tmap_v);
 }

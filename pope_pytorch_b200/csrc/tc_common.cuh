@@ -114,10 +114,8 @@ bool make_wide_tmap(CUtensorMap* out, const void* base, bool is_bf16, int d, int
 // an operand image as (1 KB run, tile, chunk): box = (1 KB, 2 tiles, all chunks) = one resident 128-row operand
 bool make_image_tmap(CUtensorMap* out, const void* img, int64_t ntiles, int chunks);
 // ch / sh = fp16 cos / sin of the phase table, [positions][r].  All jobs share d and the dtype; one launch.
-// `dependent`: launch it as a programmatic dependent of the kernel before it on the stream (only when that kernel is one
-// of this library's: the kernel waits for it before its first read)
 cudaError_t launch_expand_images(const ExpandJobs& jobs, int njobs, int d, bool is_bf16, const void* ch, const void* sh,
-                                 cudaStream_t st, bool dependent = false);
+                                 cudaStream_t st);
 
 // Launch `kernel` so that its CTAs may start while the previous kernel on `st` still runs (programmatic stream
 // serialization); the kernel calls pdl_wait() before it reads what that kernel wrote.  A kernel that waits before its first

@@ -58,7 +58,8 @@ constexpr int SIM_THREADS = 320;
 // `zero` (may be null): nzero counters that the kernel behind this one wants to find at 0
 __global__ void pope_trig_table_f32_kernel(PhaseSrc src, int n, int r, float* ctab, float* stab, __half* ch, __half* sh, unsigned int* zero,
                                            int nzero) {
-  pdl_trigger();   // the kernel behind this one may set itself up; it waits for this grid before it reads the tables
+  pdl_wait();      // usually the first kernel of its call; only behind this wait is the work before the call complete, so the
+  pdl_trigger();   // next kernel, which may read the caller's inputs before its own wait, is let go after it
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (zero && blockIdx.y == 0)
     for (int64_t i = idx; i < nzero; i += (int64_t)gridDim.x * blockDim.x) zero[i] = 0u;
@@ -77,9 +78,8 @@ cudaError_t launch_trig_tables(const PopeEmbed& e, int n, int r, float* ctab, fl
   const int64_t total = (int64_t)n * r;
   PhaseSrc src = phase_src(e);
   src.tab_heads = tab_heads;
-  pope_trig_table_f32_kernel<<<dim3((unsigned)((total + 255) / 256), (unsigned)slices), 256, 0, st>>>(
-      src, n, r, ctab, stab, static_cast<__half*>(ch), static_cast<__half*>(sh), zero, nzero);
-  return cudaGetLastError();
+  return launch_dependent(pope_trig_table_f32_kernel, dim3((unsigned)((total + 255) / 256), (unsigned)slices), dim3(256), 0, st, src, n, r,
+                          ctab, stab, static_cast<__half*>(ch), static_cast<__half*>(sh), zero, nzero);
 }
 cudaError_t launch_trig_table_f32(const PopeEmbed& e, int n, int r, float* ctab, float* stab, cudaStream_t st) {
   return launch_trig_tables(e, n, r, ctab, stab, nullptr, nullptr, st);
@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(256) sim_prepass_kernel(const T* __restrict__ 
                                                           int Nk, int d, int r, int qtiles, int ktiles, int tile_rows,
                                                           uint8_t* __restrict__ qimg, uint8_t* __restrict__ kimg) {
   const int tid = threadIdx.x, u = blockIdx.y;
-  pdl_trigger();   // the similarity kernel behind this one may set itself up; it waits for this grid before it reads the images
+  pdl_wait();      // the work before this call is complete ...
+  pdl_trigger();   // ... before the similarity kernel behind this one may start (it waits for this grid before it reads the images)
   const int bpt = tile_rows / 32;   // blocks per tile
   const bool is_q = (int)blockIdx.x < bpt * qtiles;
   const int blk = is_q ? blockIdx.x : blockIdx.x - bpt * qtiles, tile = blk / bpt, quarter = blk % bpt;
@@ -448,23 +449,16 @@ cudaError_t sim_launch_prepass(const PopeShape& s, const PopeEmbed& e, const voi
                                const PopeStride3& sk, uint8_t* qimg, uint8_t* kimg, int tile_rows, cudaStream_t st) {
   const int qtiles = (s.Nq + tile_rows - 1) / tile_rows, ktiles = (s.Nk + tile_rows - 1) / tile_rows;
   const dim3 grid((tile_rows / 32) * (qtiles + ktiles), s.B * s.H);
+  auto go = [&](auto kernel, auto tag) {
+    using T = decltype(tag);
+    return launch_dependent(kernel, grid, dim3(256), 0, st, static_cast<const T*>(q), Strides(sq), static_cast<const T*>(k), Strides(sk),
+                            phase_src(e), e.bias, e.bias_stride_h, s.B, s.H, s.Hk, s.Nq, s.Nk, s.d, s.r, qtiles, ktiles, tile_rows, qimg, kimg);
+  };
   switch (s.dtype) {
-    case POPE_F32:
-      sim_prepass_kernel<float, true><<<grid, 256, 0, st>>>(static_cast<const float*>(q), Strides(sq), static_cast<const float*>(k),
-                                                            Strides(sk), phase_src(e), e.bias, e.bias_stride_h, s.B, s.H, s.Hk,
-                                                            s.Nq, s.Nk, s.d, s.r, qtiles, ktiles, tile_rows, qimg, kimg);
-      break;
-    case POPE_BF16:
-      sim_prepass_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(q), Strides(sq), static_cast<const __nv_bfloat16*>(k), Strides(sk), phase_src(e), e.bias,
-          e.bias_stride_h, s.B, s.H, s.Hk, s.Nq, s.Nk, s.d, s.r, qtiles, ktiles, tile_rows, qimg, kimg);
-      break;
-    default:
-      sim_prepass_kernel<__half, false><<<grid, 256, 0, st>>>(static_cast<const __half*>(q), Strides(sq), static_cast<const __half*>(k),
-                                                              Strides(sk), phase_src(e), e.bias, e.bias_stride_h, s.B, s.H, s.Hk,
-                                                              s.Nq, s.Nk, s.d, s.r, qtiles, ktiles, tile_rows, qimg, kimg);
+    case POPE_F32: return go(sim_prepass_kernel<float, true>, float());
+    case POPE_BF16: return go(sim_prepass_kernel<__nv_bfloat16, false>, __nv_bfloat16());
+    default: return go(sim_prepass_kernel<__half, false>, __half());
   }
-  return cudaGetLastError();
 }
 
 template <typename T, bool SPLIT, int MT, int NKB>
