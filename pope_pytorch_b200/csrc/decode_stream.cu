@@ -96,19 +96,6 @@ template <typename T, int N2> __device__ __forceinline__ void unpack_words(const
   for (int e = 0; e < N2; ++e) x[e] = unpack2<T>(u[e]);
 }
 
-// every thread of every CTA of the cluster
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// *p in the shared memory of CTA `rank` of this cluster
-__device__ __forceinline__ float dsmem_ld(const float* p, uint32_t rank) {
-  uint32_t a;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
-
 constexpr int DS_EXACT_KEYS = 1024;   // shorter contiguous key ranges keep fp32 phases
 constexpr int DS_TILE = 64;       // keys per tile
 constexpr int DS_MAX_SPLIT = 64;  // key ranges per unit
@@ -673,15 +660,7 @@ static cudaError_t launch_decode_stream(const PopeAttnArgs& a, cudaStream_t st, 
   const unsigned units = (unsigned)(s.B * s.H / G);
   const dim3 grid((unsigned)p.nsplit, units), block(32 * (NW + 1));
   if constexpr (SHORT) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)p.nsplit, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr, cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
+    return launch_clusters(kernel, p.nsplit, grid, block, smem, st, p);
   }
   // behind the table kernel, which also zeroes the counters, the decode kernel starts as its programmatic dependent;
   // without rotated features it is the first launch of the call and an ordinary one

@@ -9,8 +9,12 @@
 //     permuted by  group ^ (feature / 4 mod 16).  That one layout feeds both kinds of product without bank conflicts: with the
 //     features as the contraction index (scores: four rows of both operands per feature) and with the rows as the contraction
 //     index (gradients and P V: four keys of a feature at a time).
-//   * a thread owns a 4 x 4 piece of the score tile and 4 rows x (columns / 16) of the accumulators: two 16-byte shared loads
-//     per 16 FMAs, a quarter of what one row x one key per lane needed.
+//   * a thread owns 4 rows x 8 columns of the score tile (4 x 4 where the accumulators are wide) and a warp 16 rows x 64
+//     columns, 4 x 8 lanes: of the three 16-byte loads per 32 FMAs the lanes of a half-warp share addresses, six
+//     wavefronts in eight clocks of the FMA pipe.  (4 x 4 per thread and 2 x 16 lanes: six wavefronts in four clocks, and
+//     shared memory set the pace.)
+//   * small grids are cut along the streamed operand: a cluster of 2 or 4 CTAs shares a tile, each takes a part of the
+//     stream, and the partial accumulators meet in distributed shared memory.
 // Measured at (1, 8, 1024, 64), r = 64, causal, fp32: see the table at the launch functions.
 //
 // Semantics: PoPE_pytorch/triton_pope_flash_attn.py:23-218 (top-left causal mask, bottom-right positions, mask True = keep,
@@ -25,11 +29,23 @@
 namespace pope {
 
 constexpr int ST_ROWS = 64;        // rows of a tile
-constexpr int ST_THREADS = 256;    // 16 x 16 threads, 4 x 4 scores each
+
+// Thread layout: TX = 8: 128 threads, 4 x 8 scores each; TX = 16: 256 threads, 4 x 4.  Rows 4 ty + i; column (or feature) j of
+// a thread is 4 tx + j % 4 + 4 TX (j / 4).
+template <int TX> struct Lay {
+  static constexpr int THREADS = 16 * TX, CS = 64 / TX;
+  int tx, ty;
+  __device__ __forceinline__ Lay() {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    tx = (lane & 7) + (TX == 16 ? (w & 1) * 8 : 0), ty = (TX == 16 ? w >> 1 : w) * 4 + (lane >> 3);
+  }
+  __device__ __forceinline__ int col(int j) const { return tx * 4 + (j & 3) + 4 * TX * (j >> 2); }
+};
 
 struct TiledP {
   int H, Hk, Nq, Nk, d, r, KD;     // KD = d + r rounded up to 8: features of a Q' / K' tile
   int qt, kt, causal, dtype;       // tiles per unit
+  int split;                       // CTAs of a cluster that share a tile
   float scale, scale_log2;
   const float *qimg, *kimg, *vimg, *gimg;   // [unit][tile][KD | DP][64]: Q', K', V, dO
   int DP;                          // features of a V / dO tile: d rounded up to 8
@@ -113,49 +129,62 @@ static cudaError_t launch_tile_images(const TileJobs& jobs, int njobs, const Pop
 }
 
 // ---- tile products ---------------------------------------------------------------------------------------------------
-// c[i][j] += sum over features k < n of A[k][4 ty + i] B[k][4 tx + j], both feature-major tiles
-__device__ __forceinline__ void mm_features(float (&c)[4][4], const float* A, const float* B, int n, int ty, int tx) {
+// c[i][j] += sum over features k < n of A[k][row(i)] B[k][col(j)], both feature-major tiles
+template <int TX>
+__device__ __forceinline__ void mm_features(float (&c)[4][64 / TX], const float* A, const float* B, int n, Lay<TX> L) {
+  constexpr int CS = 64 / TX;
 #pragma unroll 2
   for (int k4 = 0; k4 < n; k4 += 4) {
     const int sw = (k4 >> 2) & 15;
-    const float* a = A + k4 * ST_ROWS + ((ty ^ sw) << 2);
-    const float* b = B + k4 * ST_ROWS + ((tx ^ sw) << 2);
+    const float* a = A + k4 * ST_ROWS + ((L.ty ^ sw) << 2);
+    const float* b[CS / 4];
+#pragma unroll
+    for (int q = 0; q < CS / 4; ++q) b[q] = B + k4 * ST_ROWS + (((L.tx + TX * q) ^ sw) << 2);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float4 av = *reinterpret_cast<const float4*>(a + k * ST_ROWS), bv = *reinterpret_cast<const float4*>(b + k * ST_ROWS);
-      const float x[4] = {av.x, av.y, av.z, av.w}, y[4] = {bv.x, bv.y, bv.z, bv.w};
+      const float4 av = *reinterpret_cast<const float4*>(a + k * ST_ROWS);
+      const float x[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int q = 0; q < CS / 4; ++q) {
+        const float4 bv = *reinterpret_cast<const float4*>(b[q] + k * ST_ROWS);
+        const float y[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) c[i][j] = fmaf(x[i], y[j], c[i][j]);
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) c[i][q * 4 + j] = fmaf(x[i], y[j], c[i][q * 4 + j]);
+      }
     }
   }
 }
 
-// c[i][m] += sum over the 64 tile rows t of S[4 ty + i][t] B[feature(m)][t]: S is a row-major score tile (put_scores), B a
-// feature-major tile; feature(m) = 4 tx + m % 4 + 64 (m / 4)
-template <int NC>
-__device__ __forceinline__ void mm_rows(float (&c)[4][NC], const float* S, const float* B, int ty, int tx) {
-  const float* s = S + ty * 4 * ST_ROWS;
-  const float* b = B + tx * 4 * ST_ROWS;
+// c[i][m] += sum over the 64 tile rows t of S[row(i)][t] B[col(m)][t]: S is a row-major score tile (put_scores), B a
+// feature-major tile
+template <int TX, int NC>
+__device__ __forceinline__ void mm_rows(float (&c)[4][NC], const float* S, const float* B, Lay<TX> L) {
+  const float* s = S + L.ty * 4 * ST_ROWS;
+  const float* b = B + L.tx * 4 * ST_ROWS;
 #pragma unroll 2
   for (int g = 0; g < 16; ++g) {
     float4 x[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(s + i * ST_ROWS + ((g ^ ty) << 2));
+    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(s + i * ST_ROWS + ((g ^ L.ty) << 2));
 #pragma unroll
     for (int m = 0; m < NC; ++m) {
-      const float4 y = *reinterpret_cast<const float4*>(b + ((m >> 2) * 64 + (m & 3)) * ST_ROWS + ((g ^ tx) << 2));
+      const float4 y = *reinterpret_cast<const float4*>(b + ((m >> 2) * 4 * TX + (m & 3)) * ST_ROWS + ((g ^ ((L.tx + TX * (m >> 2)) & 15)) << 2));
 #pragma unroll
       for (int i = 0; i < 4; ++i) c[i][m] = fmaf(x[i].w, y.w, fmaf(x[i].z, y.z, fmaf(x[i].y, y.y, fmaf(x[i].x, y.x, c[i][m]))));
     }
   }
 }
 
-__device__ __forceinline__ void put_scores(float* S, const float (&v)[4][4], int ty, int tx) {
+template <int TX>
+__device__ __forceinline__ void put_scores(float* S, const float (&v)[4][64 / TX], Lay<TX> L) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    *reinterpret_cast<float4*>(S + (ty * 4 + i) * ST_ROWS + ((tx ^ ty) << 2)) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+#pragma unroll
+    for (int q = 0; q < 64 / TX / 4; ++q)
+      *reinterpret_cast<float4*>(S + (L.ty * 4 + i) * ST_ROWS + (((L.tx + TX * q) ^ L.ty) << 2)) =
+          make_float4(v[i][q * 4], v[i][q * 4 + 1], v[i][q * 4 + 2], v[i][q * 4 + 3]);
 }
 
 template <int N> __device__ __forceinline__ void zero(float (&c)[4][N]) {
@@ -163,6 +192,18 @@ template <int N> __device__ __forceinline__ void zero(float (&c)[4][N]) {
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) c[i][j] = 0.f;
+}
+
+// the sum of *p over the CTAs that share a tile
+__device__ __forceinline__ float over_split(const float* p, int split) {
+  if (split == 1) return *p;
+  float v = 0.f;
+  for (int r = 0; r < split; ++r) v += dsmem_ld(p, r);
+  return v;
+}
+__device__ __forceinline__ void split_sync(int split) {
+  if (split == 1) __syncthreads();
+  else __syncwarp(), cluster_sync();
 }
 
 // one image tile by bulk copy; a thread of the CTA calls it after every thread is done with the buffer
@@ -174,108 +215,152 @@ __device__ __forceinline__ void fetch(float* dst, const float* img, int feats, u
 // ---- forward ---------------------------------------------------------------------------------------------------------
 // Shared memory: Q' tile, K' tile, V tile, P.  The K' buffer is free once the scores are in registers and refilled behind
 // the softmax and P V, the V buffer is refilled behind the next scores; where two CTAs fit an SM they cover the rest.
+// ND: output features per thread.
 template <int ND>
-__global__ void __launch_bounds__(ST_THREADS, ND == 4 ? 2 : 1) attn_fwd_tiled_kernel(TiledP p) {
+__global__ void __launch_bounds__(128, ND == 8 ? 2 : 1) attn_fwd_tiled_kernel(TiledP p) {
+  constexpr int TX = 8, CS = 8;
   extern __shared__ __align__(128) float st_smem[];
-  const int QF = p.KD * ST_ROWS, VF = ND * 16 * ST_ROWS;
-  float *Qs = st_smem, *Ks = Qs + QF, *Vs = Ks + QF, *Ps = Vs + VF;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(Ps + ST_ROWS * ST_ROWS);   // Q', K', V landed
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int QF = p.KD * ST_ROWS, VF = ND * TX * ST_ROWS;
+  float *Qs = st_smem, *Ks = Qs + QF, *Vs = Ks + QF, *Ps = Vs + VF, *ml = Ps + ST_ROWS * ST_ROWS;   // ml: [64] maxima, [64] sums
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ml + 2 * ST_ROWS);   // Q', K', V landed
+  const int tid = threadIdx.x;
+  const Lay<TX> L;
   const int u = blockIdx.y, b = u / p.H, h = u % p.H, hk = h % p.Hk, uk = b * p.Hk + hk;
-  const int qtile = gridDim.x - 1 - blockIdx.x, i0 = qtile * ST_ROWS;   // heavy (late) row blocks first
+  const int rank = blockIdx.x % p.split, qtile = p.qt - 1 - blockIdx.x / p.split, i0 = qtile * ST_ROWS;   // heavy (late) row blocks first
   int n_end = p.Nk;
   if (p.causal) n_end = min(n_end, min(i0 + ST_ROWS, p.Nq));
-  const int T = (n_end + ST_ROWS - 1) / ST_ROWS;
-  const float* kimg = p.kimg + (int64_t)uk * p.kt * QF;
-  const float* vimg = p.vimg + (int64_t)uk * p.kt * p.DP * ST_ROWS;
+  const int tiles = (n_end + ST_ROWS - 1) / ST_ROWS, t0 = tiles * rank / p.split, T = tiles * (rank + 1) / p.split - t0;
+  const float* kimg = p.kimg + ((int64_t)uk * p.kt + t0) * QF;
+  const float* vimg = p.vimg + ((int64_t)uk * p.kt + t0) * p.DP * ST_ROWS;
   const uint8_t* mask = p.mask ? p.mask + b * p.msb : nullptr;
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
     mbar_init_fence();
     pdl_wait();
-    fetch(Qs, p.qimg + ((int64_t)u * p.qt + qtile) * QF, p.KD, &bars[0]);
-    fetch(Ks, kimg, p.KD, &bars[1]);
-    fetch(Vs, vimg, p.DP, &bars[2]);
+    if (T > 0) {
+      fetch(Qs, p.qimg + ((int64_t)u * p.qt + qtile) * QF, p.KD, &bars[0]);
+      fetch(Ks, kimg, p.KD, &bars[1]);
+      fetch(Vs, vimg, p.DP, &bars[2]);
+    }
   }
   __syncthreads();
-  bool failed = !mbar_wait(&bars[0], 0, WAIT_LIMIT);
+  bool failed = T > 0 && !mbar_wait(&bars[0], 0, WAIT_LIMIT);
   float m[4], l[4], o[4][ND];
 #pragma unroll
   for (int i = 0; i < 4; ++i) m[i] = -CUDART_INF_F, l[i] = 0.f;
   zero(o);
   for (int t = 0; t < T; ++t) {
-    const int n0 = t * ST_ROWS;
-    float s[4][4];
+    const int n0 = (t0 + t) * ST_ROWS;
+    float s[4][CS];
     zero(s);
-    if (!failed) failed = !mbar_wait(&bars[1], t & 1, WAIT_LIMIT);
-    mm_features(s, Qs, Ks, p.KD, ty, tx);
-    const int j0 = n0 + tx * 4;
-    bool ok[4];
+    uint32_t ok = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ok[j] = j0 + j < p.Nk && (!mask || mask[(int64_t)(j0 + j) * p.msn] != 0);
+    for (int j = 0; j < CS; ++j) {
+      const int key = n0 + L.col(j);
+      ok |= (uint32_t)(key < p.Nk && (!mask || mask[(int64_t)key * p.msn] != 0)) << j;
+    }
+    if (!failed) failed = !mbar_wait(&bars[1], t & 1, WAIT_LIMIT);
+    mm_features<TX>(s, Qs, Ks, p.KD, L);
     __syncthreads();   // the K' tile and (from the last round) P have been read
     if (tid == 0 && t + 1 < T) fetch(Ks, kimg + (int64_t)(t + 1) * QF, p.KD, &bars[1]);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int gi = i0 + ty * 4 + i;
+      const int gi = i0 + L.ty * 4 + i;
       float mx = -CUDART_INF_F;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        s[i][j] = ok[j] && (!p.causal || j0 + j <= gi) ? s[i][j] * p.scale_log2 : -CUDART_INF_F;
+      for (int j = 0; j < CS; ++j) {
+        s[i][j] = ((ok >> j) & 1u) && (!p.causal || n0 + L.col(j) <= gi) ? s[i][j] * p.scale_log2 : -CUDART_INF_F;
         mx = fmaxf(mx, s[i][j]);
       }
 #pragma unroll
-      for (int off = 8; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      for (int off = 4; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       const float m_new = fmaxf(m[i], mx), m_use = m_new == -CUDART_INF_F ? 0.f : m_new;
       const float alpha = exp2f(m[i] - m_use);   // 0 on the first visible tile
       m[i] = m_new;
       float sum = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = exp2f(s[i][j] - m_use), sum += s[i][j];
+      for (int j = 0; j < CS; ++j) s[i][j] = exp2f(s[i][j] - m_use), sum += s[i][j];
       l[i] = l[i] * alpha + sum;                 // this lane's columns; the lanes of a row are summed at the end
 #pragma unroll
       for (int c = 0; c < ND; ++c) o[i][c] *= alpha;
     }
-    put_scores(Ps, s, ty, tx);
+    put_scores<TX>(Ps, s, L);
     __syncthreads();
     if (!failed) failed = !mbar_wait(&bars[2], t & 1, WAIT_LIMIT);
-    mm_rows<ND>(o, Ps, Vs, ty, tx);
+    mm_rows<TX, ND>(o, Ps, Vs, L);
     if (t + 1 < T) {
       __syncthreads();   // the V tile has been read
       if (tid == 0) fetch(Vs, vimg + (int64_t)(t + 1) * p.DP * ST_ROWS, p.DP, &bars[2]);
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gi = i0 + ty * 4 + i;
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int off = 8; off >= 1; off >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
-    if (gi >= p.Nq) continue;
-    const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
-    const int64_t base = b * p.so.b + h * p.so.h + (int64_t)gi * p.so.n;
+    for (int off = 4; off >= 1; off >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
+  if (p.split == 1) {
 #pragma unroll
-    for (int c = 0; c < ND; ++c) {
-      const int col = tx * 4 + (c & 3) + 64 * (c >> 2);
-      if (col < p.d) put(p.o, base + col, o[i][c] * inv, p.dtype);
+    for (int i = 0; i < 4; ++i) {
+      const int gi = i0 + L.ty * 4 + i;
+      if (gi >= p.Nq) continue;
+      const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+      const int64_t base = b * p.so.b + h * p.so.h + (int64_t)gi * p.so.n;
+#pragma unroll
+      for (int c = 0; c < ND; ++c)
+        if (L.col(c) < p.d) put(p.o, base + L.col(c), o[i][c] * inv, p.dtype);
+      if (L.tx == 0) p.lse[(int64_t)u * p.Nq + gi] = l[i] > 0.f ? m[i] * LN2 + logf(l[i]) : -CUDART_INF_F;
     }
-    if (tx == 0) p.lse[(int64_t)u * p.Nq + gi] = l[i] > 0.f ? m[i] * LN2 + logf(l[i]) : -CUDART_INF_F;
+  } else {
+    // the parts of the key range meet: (max, sum, output) of every CTA in its own shared memory, each CTA finishes its
+    // share of the rows
+    float* os = Vs;   // [64][ND * TX]; V and P are dead
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = L.ty * 4 + i;
+#pragma unroll
+      for (int c = 0; c < ND; ++c) os[row * (ND * TX) + L.col(c)] = o[i][c];
+      if (L.tx == 0) ml[row] = m[i], ml[ST_ROWS + row] = l[i];
+    }
+    split_sync(p.split);
+    const int r0 = ST_ROWS * rank / p.split, r1 = ST_ROWS * (rank + 1) / p.split;
+    for (int row = r0 + (tid >> 5); row < r1 && i0 + row < p.Nq; row += 4) {
+      float M = -CUDART_INF_F, sum = 0.f, w[4];
+      for (int r = 0; r < p.split; ++r) M = fmaxf(M, dsmem_ld(ml + row, r));
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        w[r] = r < p.split && M != -CUDART_INF_F ? exp2f(dsmem_ld(ml + row, r) - M) : 0.f;
+        if (r < p.split) sum += w[r] * dsmem_ld(ml + ST_ROWS + row, r);
+      }
+      const float inv = sum > 0.f ? 1.f / sum : 0.f;
+      const int64_t base = b * p.so.b + h * p.so.h + (int64_t)(i0 + row) * p.so.n;
+      for (int c = tid & 31; c < p.d; c += 32) {
+        float v = 0.f;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (r < p.split) v = fmaf(w[r], dsmem_ld(os + row * (ND * TX) + c, r), v);
+        put(p.o, base + c, v * inv, p.dtype);
+      }
+      if ((tid & 31) == 0) p.lse[(int64_t)u * p.Nq + i0 + row] = sum > 0.f ? M * LN2 + logf(sum) : -CUDART_INF_F;
+    }
+    split_sync(p.split);   // nobody leaves while its shared memory is read
   }
   if (failed) atomicOr(p.status, 1u);
 }
 
 // ---- backward ----------------------------------------------------------------------------------------------------------
-// Epilogue: X' gradients of 64 rows in `acc` [64][ASTR] -> dx, dphase.  Everything the chain rule needs is in the resident
+// Epilogue: X' gradients of rows [r0, r1) of a tile, staged as [64][astr] by every CTA that shares it -> dx, dphase.  Everything the chain rule needs is in the resident
 // image tile: with xc = a cos, xs = a sin,  a = sqrt(xc^2 + xs^2),  sigmoid(x) = 1 - exp(-a),
 //   dx = (gc xc + gs xs) / a * sigmoid(x),  dphase = gs xc - gc xs.
 __device__ __forceinline__ void chain_rule(const TiledP& p, const float* acc, int astr, const float* X, int row0, int rows, void* dx, int64_t base,
-                                           int64_t sn, float* df, int64_t sfn, int pos0, float* dbias) {
+                                           int64_t sn, float* df, int64_t sfn, int pos0, float* dbias, int rank) {
+  const int r0 = ST_ROWS * rank / p.split, r1 = ST_ROWS * (rank + 1) / p.split;
   for (int c = threadIdx.x & 63; c < p.d; c += 64) {
     float sum = 0.f;
-    for (int row = threadIdx.x >> 6; row < ST_ROWS && row0 + row < rows; row += 4) {
-      float g = acc[row * astr + c];
+    for (int row = r0 + (threadIdx.x >> 6); row < r1 && row0 + row < rows; row += blockDim.x >> 6) {
+      float g = over_split(acc + row * astr + c, p.split);
       if (c < p.r) {
         const int grp = row >> 2, e = row & 3;
-        const float gs = acc[row * astr + p.d + c];
+        const float gs = over_split(acc + row * astr + p.d + c, p.split);
         const float xc = X[c * ST_ROWS + (((grp ^ (c >> 2)) & 15) << 2) + e];
         const float xs = X[(p.d + c) * ST_ROWS + (((grp ^ ((p.d + c) >> 2)) & 15) << 2) + e];
         const float a = sqrtf(xc * xc + xs * xs), dph = gs * xc - g * xs;
@@ -290,40 +375,39 @@ __device__ __forceinline__ void chain_rule(const TiledP& p, const float* acc, in
 }
 
 // accumulator columns -> row-major staging tile
-template <int N> __device__ __forceinline__ void stage_acc(float* dst, int stride, const float (&c)[4][N], int width, int ty, int tx) {
+template <int TX, int N> __device__ __forceinline__ void stage_acc(float* dst, int stride, const float (&c)[4][N], int width, Lay<TX> L) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const int col = tx * 4 + (m & 3) + 64 * (m >> 2);
-      if (col < width) dst[(ty * 4 + i) * stride + col] = c[i][m];
-    }
+    for (int m = 0; m < N; ++m)
+      if (L.col(m) < width) dst[(L.ty * 4 + i) * stride + L.col(m)] = c[i][m];
 }
 
 // dq: 64 query rows resident (Q', dO); streams K' and V tiles:  S, dP -> dS -> dQ' += dS K'
-template <int ND, int NK>
-__device__ __forceinline__ void bwd_dq_tiled(const TiledP& p, float* smem, uint64_t* bars, int qtile, int u) {
-  const int QF = p.KD * ST_ROWS, QA = NK * 16 * ST_ROWS, VF = p.DP * ST_ROWS;
+template <int TX, int ND, int NK>
+__device__ __forceinline__ void bwd_dq_tiled(const TiledP& p, float* smem, uint64_t* bars, int qtile, int u, int rank) {
+  constexpr int CS = 64 / TX;
+  const int QF = p.KD * ST_ROWS, QA = NK * TX * ST_ROWS, VF = p.DP * ST_ROWS;
   float *Qs = smem, *Gs = Qs + QF, *Ks = Gs + VF, *Vs = Ks + QA, *Ss = Vs + VF;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x;
+  const Lay<TX> L;
   const int b = u / p.H, h = u % p.H, hk = h % p.Hk, uk = b * p.Hk + hk, i0 = qtile * ST_ROWS;
   int n_end = p.Nk;
   if (p.causal) n_end = min(n_end, min(i0 + ST_ROWS, p.Nq));
-  const int T = (n_end + ST_ROWS - 1) / ST_ROWS;
-  const float* kimg = p.kimg + (int64_t)uk * p.kt * QF;
-  const float* vimg = p.vimg + (int64_t)uk * p.kt * VF;
+  const int tiles = (n_end + ST_ROWS - 1) / ST_ROWS, t0 = tiles * rank / p.split, T = tiles * (rank + 1) / p.split - t0;
+  const float* kimg = p.kimg + ((int64_t)uk * p.kt + t0) * QF;
+  const float* vimg = p.vimg + ((int64_t)uk * p.kt + t0) * VF;
   const uint8_t* mask = p.mask ? p.mask + b * p.msb : nullptr;
   if (tid == 0) {
     mbar_expect_tx(&bars[0], (QF + VF) * 4);
     bulk_load(Qs, p.qimg + ((int64_t)u * p.qt + qtile) * QF, QF * 4, &bars[0]);
     bulk_load(Gs, p.gimg + ((int64_t)u * p.qt + qtile) * VF, VF * 4, &bars[0]);
-    fetch(Ks, kimg, p.KD, &bars[1]);
-    fetch(Vs, vimg, p.DP, &bars[2]);
+    if (T > 0) fetch(Ks, kimg, p.KD, &bars[1]), fetch(Vs, vimg, p.DP, &bars[2]);
   }
   float lse2[4], dl[4], acc[4][NK];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int gi = i0 + ty * 4 + i;
+    const int gi = i0 + L.ty * 4 + i;
     const float l = gi < p.Nq ? p.lse_in[(int64_t)u * p.Nq + gi] : -CUDART_INF_F;
     lse2[i] = l == -CUDART_INF_F ? CUDART_INF_F : l * LOG2E;   // +inf: probabilities are exactly 0
     dl[i] = gi < p.Nq ? p.delta[(int64_t)u * p.Nq + gi] : 0.f;
@@ -331,130 +415,139 @@ __device__ __forceinline__ void bwd_dq_tiled(const TiledP& p, float* smem, uint6
   zero(acc);
   bool failed = !mbar_wait(&bars[0], 0, WAIT_LIMIT);
   for (int t = 0; t < T; ++t) {
-    const int j0 = t * ST_ROWS + tx * 4;
-    float s[4][4], dp[4][4];
+    const int n0 = (t0 + t) * ST_ROWS;
+    float s[4][CS], dp[4][CS];
     zero(s), zero(dp);
-    if (!failed) failed = !mbar_wait(&bars[2], t & 1, WAIT_LIMIT);
-    mm_features(dp, Gs, Vs, p.DP, ty, tx);
-    bool ok[4];
+    uint32_t ok = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ok[j] = j0 + j < p.Nk && (!mask || mask[(int64_t)(j0 + j) * p.msn] != 0);
+    for (int j = 0; j < CS; ++j) {
+      const int key = n0 + L.col(j);
+      ok |= (uint32_t)(key < p.Nk && (!mask || mask[(int64_t)key * p.msn] != 0)) << j;
+    }
+    if (!failed) failed = !mbar_wait(&bars[2], t & 1, WAIT_LIMIT);
+    mm_features<TX>(dp, Gs, Vs, p.DP, L);
     if (!failed) failed = !mbar_wait(&bars[1], t & 1, WAIT_LIMIT);
-    mm_features(s, Qs, Ks, p.KD, ty, tx);
+    mm_features<TX>(s, Qs, Ks, p.KD, L);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool vis = ok[j] && (!p.causal || j0 + j <= i0 + ty * 4 + i);
+      for (int j = 0; j < CS; ++j) {
+        const bool vis = ((ok >> j) & 1u) && (!p.causal || n0 + L.col(j) <= i0 + L.ty * 4 + i);
         s[i][j] = vis ? exp2f(s[i][j] * p.scale_log2 - lse2[i]) * (dp[i][j] - dl[i]) * p.scale : 0.f;
       }
-    put_scores(Ss, s, ty, tx);
+    put_scores<TX>(Ss, s, L);
     __syncthreads();   // dS is written, the V tile has been read
     if (tid == 0 && t + 1 < T) fetch(Vs, vimg + (int64_t)(t + 1) * VF, p.DP, &bars[2]);
-    mm_rows<NK>(acc, Ss, Ks, ty, tx);
+    mm_rows<TX, NK>(acc, Ss, Ks, L);
     __syncthreads();   // the K' tile and dS have been read
     if (tid == 0 && t + 1 < T) fetch(Ks, kimg + (int64_t)(t + 1) * QF, p.KD, &bars[1]);
   }
   const int astr = p.d + p.r + 1;
-  stage_acc<NK>(Gs, astr, acc, p.d + p.r, ty, tx);   // dO, K', V and dS are dead: [64][d + r + 1] fits them
-  __syncthreads();
+  stage_acc<TX, NK>(Gs, astr, acc, p.d + p.r, L);   // dO, K', V and dS are dead: [64][d + r + 1] fits them
+  split_sync(p.split);
   float* df = p.dfreqs ? p.dfreqs + b * p.sdf.b + h * p.sdf.h : nullptr;
-  chain_rule(p, Gs, astr, Qs, i0, p.Nq, p.dq, b * p.sdq.b + h * p.sdq.h, p.sdq.n, df, p.sdf.n, p.Nk - p.Nq, nullptr);
+  chain_rule(p, Gs, astr, Qs, i0, p.Nq, p.dq, b * p.sdq.b + h * p.sdq.h, p.sdq.n, df, p.sdf.n, p.Nk - p.Nq, nullptr, rank);
+  if (p.split > 1) split_sync(p.split);   // nobody leaves while its shared memory is read
   if (failed) atomicOr(p.status, 1u);
 }
 
 // dk / dv: 64 key rows resident (K', V); streams the Q' and dO tiles of every grouped query head:
 // S^T, dP^T -> P^T -> dV += P^T dO, dS^T -> dK' += dS^T Q'
-template <int ND, int NK>
-__device__ __forceinline__ void bwd_dkdv_tiled(const TiledP& p, float* smem, uint64_t* bars, int ktile, int uk) {
-  const int QF = p.KD * ST_ROWS, QA = NK * 16 * ST_ROWS, VF = p.DP * ST_ROWS, VA = ND * 16 * ST_ROWS;
+template <int TX, int ND, int NK>
+__device__ __forceinline__ void bwd_dkdv_tiled(const TiledP& p, float* smem, uint64_t* bars, int ktile, int uk, int rank) {
+  constexpr int CS = 64 / TX;
+  const int QF = p.KD * ST_ROWS, QA = NK * TX * ST_ROWS, VF = p.DP * ST_ROWS, VA = ND * TX * ST_ROWS;
   float *Ks = smem, *Vs = Ks + QF, *Qs = Vs + VF, *Gs = Qs + QA, *Ss = Gs + VA;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x;
+  const Lay<TX> L;
   const int b = uk / p.Hk, hk = uk % p.Hk, j0 = ktile * ST_ROWS, groups = p.H / p.Hk;
   const int t_first = p.causal ? ktile : 0;   // under the causal mask queries before this tile see none of its keys
-  const int per = p.qt > t_first ? p.qt - t_first : 0, T = per * groups;
+  const int per = p.qt > t_first ? p.qt - t_first : 0, total = per * groups;
+  const int s0 = total * rank / p.split, T = total * (rank + 1) / p.split - s0;   // this CTA's part of the stream
   const uint8_t* mask = p.mask ? p.mask + b * p.msb : nullptr;
-  auto unit = [&](int t) { return b * p.H + (t / per) * p.Hk + hk; };
-  auto qtile = [&](int t) { return t_first + t % per; };
+  auto unit = [&](int t) { return b * p.H + ((s0 + t) / per) * p.Hk + hk; };
+  auto qtile = [&](int t) { return t_first + (s0 + t) % per; };
   auto fetch_q = [&](int t) { fetch(Qs, p.qimg + ((int64_t)unit(t) * p.qt + qtile(t)) * QF, p.KD, &bars[1]); };
   auto fetch_g = [&](int t) { fetch(Gs, p.gimg + ((int64_t)unit(t) * p.qt + qtile(t)) * VF, p.DP, &bars[2]); };
-  if (tid == 0 && T > 0) {
+  if (tid == 0) {
     mbar_expect_tx(&bars[0], (QF + VF) * 4);
     bulk_load(Ks, p.kimg + ((int64_t)uk * p.kt + ktile) * QF, QF * 4, &bars[0]);
     bulk_load(Vs, p.vimg + ((int64_t)uk * p.kt + ktile) * VF, VF * 4, &bars[0]);
-    fetch_q(0), fetch_g(0);
+    if (T > 0) fetch_q(0), fetch_g(0);
   }
   float ak[4][NK], av[4][ND];
   zero(ak), zero(av);
   bool ok[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int gj = j0 + ty * 4 + i;
+    const int gj = j0 + L.ty * 4 + i;
     ok[i] = gj < p.Nk && (!mask || mask[(int64_t)gj * p.msn] != 0);
   }
-  bool failed = T > 0 && !mbar_wait(&bars[0], 0, WAIT_LIMIT);
+  bool failed = !mbar_wait(&bars[0], 0, WAIT_LIMIT);
   for (int t = 0; t < T; ++t) {
-    const int q0 = qtile(t) * ST_ROWS + tx * 4;
+    const int q0 = qtile(t) * ST_ROWS;
     const float *lse = p.lse_in + (int64_t)unit(t) * p.Nq, *delta = p.delta + (int64_t)unit(t) * p.Nq;
-    float lse2[4], dl[4], s[4][4], dp[4][4];
+    float lse2[CS], dl[CS], s[4][CS], dp[4][CS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float l = q0 + j < p.Nq ? __ldg(lse + q0 + j) : -CUDART_INF_F;
+    for (int j = 0; j < CS; ++j) {
+      const int i = q0 + L.col(j);
+      const float l = i < p.Nq ? __ldg(lse + i) : -CUDART_INF_F;
       lse2[j] = l == -CUDART_INF_F ? CUDART_INF_F : l * LOG2E;
-      dl[j] = q0 + j < p.Nq ? __ldg(delta + q0 + j) : 0.f;
+      dl[j] = i < p.Nq ? __ldg(delta + i) : 0.f;
     }
     zero(s), zero(dp);
     if (!failed) failed = !mbar_wait(&bars[1], t & 1, WAIT_LIMIT);
-    mm_features(s, Ks, Qs, p.KD, ty, tx);
+    mm_features<TX>(s, Ks, Qs, p.KD, L);
     if (!failed) failed = !mbar_wait(&bars[2], t & 1, WAIT_LIMIT);
-    mm_features(dp, Vs, Gs, p.DP, ty, tx);
+    mm_features<TX>(dp, Vs, Gs, p.DP, L);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool vis = ok[i] && (!p.causal || j0 + ty * 4 + i <= q0 + j);
+      for (int j = 0; j < CS; ++j) {
+        const bool vis = ok[i] && (!p.causal || j0 + L.ty * 4 + i <= q0 + L.col(j));
         s[i][j] = vis ? exp2f(s[i][j] * p.scale_log2 - lse2[j]) : 0.f;
         dp[i][j] = s[i][j] * (dp[i][j] - dl[j]) * p.scale;
       }
-    put_scores(Ss, s, ty, tx);
+    put_scores<TX>(Ss, s, L);
     __syncthreads();
-    mm_rows<ND>(av, Ss, Gs, ty, tx);
+    mm_rows<TX, ND>(av, Ss, Gs, L);
     __syncthreads();   // P^T and the dO tile have been read
     if (tid == 0 && t + 1 < T) fetch_g(t + 1);
-    put_scores(Ss, dp, ty, tx);
+    put_scores<TX>(Ss, dp, L);
     __syncthreads();
-    mm_rows<NK>(ak, Ss, Qs, ty, tx);
+    mm_rows<TX, NK>(ak, Ss, Qs, L);
     __syncthreads();   // dS^T and the Q' tile have been read
     if (tid == 0 && t + 1 < T) fetch_q(t + 1);
   }
   const int astr = p.d + p.r + 1;
-  stage_acc<NK>(Qs, astr, ak, p.d + p.r, ty, tx);   // Q', dO and the scores are dead: [64][d + r + 1] fits them
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gj = j0 + ty * 4 + i;
-    if (gj >= p.Nk) continue;
-    const int64_t base = b * p.sdv.b + hk * p.sdv.h + (int64_t)gj * p.sdv.n;
-#pragma unroll
-    for (int m = 0; m < ND; ++m) {
-      const int col = tx * 4 + (m & 3) + 64 * (m >> 2);
-      if (col < p.d) put(p.dv, base + col, av[i][m], p.dtype);
+  stage_acc<TX, NK>(Qs, astr, ak, p.d + p.r, L);   // Q', dO and the scores are dead: [64][d + r + 1] fits them
+  // dV: with one CTA per tile straight from the registers, else through the (dead) buffers behind the staged dK'
+  float* vs = Qs + ST_ROWS * astr;   // [64][d + 1]
+  if (p.split > 1) stage_acc<TX, ND>(vs, p.d + 1, av, p.d, L);
+  split_sync(p.split);
+  const int64_t vbase = b * p.sdv.b + hk * p.sdv.h + (int64_t)j0 * p.sdv.n;
+  if (p.split > 1) {
+    for (int idx = tid; idx < (ST_ROWS / p.split) * p.d; idx += Lay<TX>::THREADS) {
+      const int row = ST_ROWS / p.split * rank + idx / p.d, c = idx % p.d;
+      if (j0 + row < p.Nk) put(p.dv, vbase + row * p.sdv.n + c, over_split(vs + row * (p.d + 1) + c, p.split), p.dtype);
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int m = 0; m < ND; ++m)
+        if (L.col(m) < p.d && j0 + L.ty * 4 + i < p.Nk) put(p.dv, vbase + (L.ty * 4 + i) * p.sdv.n + L.col(m), av[i][m], p.dtype);
   }
-  __syncthreads();
   float* df = p.dfreqs ? p.dfreqs + b * p.sdf.b + hk * p.sdf.h : nullptr;
-  // (a tile that no query sees has zero gradients; its K' tile was never fetched, so zeros stand in for it)
-  if (T == 0) {
-    for (int i = tid; i < QF; i += ST_THREADS) Ks[i] = 0.f;
-    __syncthreads();
-  }
-  chain_rule(p, Qs, astr, Ks, j0, p.Nk, p.dk, b * p.sdk.b + hk * p.sdk.h, p.sdk.n, df, p.sdf.n, 0, p.dbias ? p.dbias + hk * p.dbias_sh : nullptr);
+  chain_rule(p, Qs, astr, Ks, j0, p.Nk, p.dk, b * p.sdk.b + hk * p.sdk.h, p.sdk.n, df, p.sdf.n, 0, p.dbias ? p.dbias + hk * p.dbias_sh : nullptr, rank);
+  if (p.split > 1) split_sync(p.split);   // nobody leaves while its shared memory is read
   if (failed) atomicOr(p.status, 1u);
 }
 
 // Both sides in one launch: the CTAs of one side fill what the other leaves idle.  Blocks come heaviest first (under the
 // causal mask: late query tiles, early key tiles).
-template <int ND, int NK>
-__global__ void __launch_bounds__(ST_THREADS, (ND == 4 && NK <= 8) ? 2 : 1) attn_bwd_tiled_kernel(TiledP p, int nq_units, int nk_units) {
+template <int TX, int ND, int NK>
+__global__ void __launch_bounds__(16 * TX, NK * TX <= 128 ? 2 : 1) attn_bwd_tiled_kernel(TiledP p, int nq_units, int nk_units) {
   extern __shared__ __align__(128) float st_smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(st_smem);
   if (threadIdx.x == 0) {
@@ -463,11 +556,11 @@ __global__ void __launch_bounds__(ST_THREADS, (ND == 4 && NK <= 8) ? 2 : 1) attn
   }
   __syncthreads();
   pdl_wait();
-  const int level = blockIdx.x / (nq_units + nk_units), w = blockIdx.x % (nq_units + nk_units);
+  const int rank = blockIdx.x % p.split, id = blockIdx.x / p.split, level = id / (nq_units + nk_units), w = id % (nq_units + nk_units);
   if (w < nk_units) {
-    if (level < p.kt) bwd_dkdv_tiled<ND, NK>(p, st_smem + 32, bars, level, w);
+    if (level < p.kt) bwd_dkdv_tiled<TX, ND, NK>(p, st_smem + 32, bars, level, w, rank);
   } else if (level < p.qt) {
-    bwd_dq_tiled<ND, NK>(p, st_smem + 32, bars, p.qt - 1 - level, w - nk_units);
+    bwd_dq_tiled<TX, ND, NK>(p, st_smem + 32, bars, p.qt - 1 - level, w - nk_units, rank);
   }
 }
 
@@ -476,10 +569,10 @@ static int up(int x, int m) { return (x + m - 1) / m * m; }
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 static size_t img_bytes(int units, int rows, int feats) { return up256((size_t)units * ((rows + ST_ROWS - 1) / ST_ROWS) * ST_ROWS * feats * 4); }
 
-static size_t fwd_smem(int KD, int ND) { return (size_t)(2 * KD + ND * 16 + ST_ROWS) * ST_ROWS * 4 + 64; }
+static size_t fwd_smem(int KD, int d_wide) { return (size_t)(2 * KD + d_wide + ST_ROWS + 2) * ST_ROWS * 4 + 64; }
 // dk / dv side: K', V resident, Q', dO streamed, one score tile (the dq side needs no more); the staged gradients,
-// 64 x (d + r + 1), fit the streamed buffers of either side
-static size_t bwd_smem(int KD, int DP, int ND, int NK) { return (size_t)(KD + DP + NK * 16 + ND * 16 + ST_ROWS) * ST_ROWS * 4 + 128; }
+// 64 x (2 d + r + 2), fit the streamed buffers and the score tile of either side
+static size_t bwd_smem(int KD, int DP, int d_wide, int k_wide) { return (size_t)(KD + DP + k_wide + d_wide + ST_ROWS) * ST_ROWS * 4 + 128; }
 
 // Tiles of 64 query rows: fewer than 32 leave most of a tile empty, and the key-split kernels of simt_attn.cu serve those.
 // Wider operands than these do not fit shared memory in tiles of 64 rows.
@@ -492,6 +585,13 @@ size_t attn_fwd_tiled_workspace(const PopeShape& s) {
 }
 size_t attn_bwd_tiled_workspace(const PopeShape& s) {
   return attn_fwd_tiled_workspace(s) + img_bytes(s.B * s.H, s.Nq, up(s.d, 8)) + up256((size_t)s.B * s.H * s.Nq * 4);
+}
+
+// CTAs per tile: until two per SM are there, as long as each keeps at least two streamed tiles
+static int tiled_split(int64_t ctas, int stream) {
+  int n = 1;
+  while (n < 4 && ctas * n < 2 * 148 && stream >= 4 * n) n *= 2;
+  return n;
 }
 
 static TiledP tiled_params(const PopeShape& s, int causal, float scale, const uint8_t* mask, int64_t msb, int64_t msn, float* ws) {
@@ -517,10 +617,10 @@ static TileJob tile_job(const void* x, const PopeStride3& sx, int batch, int hea
 
 template <int ND>
 static cudaError_t launch_fwd_tiled(const TiledP& p, const PopeShape& s, cudaStream_t st) {
-  const size_t smem = fwd_smem(p.KD, ND);
+  const size_t smem = fwd_smem(p.KD, ND * 8);
   cudaError_t e = ensure_max_smem<attn_fwd_tiled_kernel<ND>>();
   if (e != cudaSuccess) return e;
-  return launch_dependent(attn_fwd_tiled_kernel<ND>, dim3(p.qt, s.B * s.H), dim3(ST_THREADS), smem, st, p);
+  return launch_clusters(attn_fwd_tiled_kernel<ND>, p.split, dim3(p.qt * p.split, s.B * s.H), dim3(128), smem, st, p);
 }
 
 cudaError_t attn_fwd_tiled(const PopeAttnArgs& a, cudaStream_t st) {
@@ -535,16 +635,18 @@ cudaError_t attn_fwd_tiled(const PopeAttnArgs& a, cudaStream_t st) {
   jobs.job[2] = tile_job(a.v, a.sv, s.B, s.Hk, s.Nk, 0, 0, p.DP, p.vimg);
   const cudaError_t e = launch_tile_images(jobs, 3, s, a.embed, st);
   if (e != cudaSuccess) return e;
-  return s.d <= 64 ? launch_fwd_tiled<4>(p, s, st) : s.d <= 128 ? launch_fwd_tiled<8>(p, s, st) : launch_fwd_tiled<16>(p, s, st);
+  p.split = tiled_split((int64_t)p.qt * s.B * s.H, p.kt);
+  return s.d <= 64 ? launch_fwd_tiled<8>(p, s, st) : s.d <= 128 ? launch_fwd_tiled<16>(p, s, st) : launch_fwd_tiled<32>(p, s, st);
 }
 
-template <int ND, int NK>
+template <int TX, int ND, int NK>
 static cudaError_t launch_bwd_tiled(const TiledP& p, const PopeShape& s, cudaStream_t st) {
-  const size_t smem = bwd_smem(p.KD, p.DP, ND, NK);
-  cudaError_t e = ensure_max_smem<attn_bwd_tiled_kernel<ND, NK>>();
+  const size_t smem = bwd_smem(p.KD, p.DP, ND * TX, NK * TX);
+  cudaError_t e = ensure_max_smem<attn_bwd_tiled_kernel<TX, ND, NK>>();
   if (e != cudaSuccess) return e;
   const int nq = s.B * s.H, nk = s.B * s.Hk;
-  return launch_dependent(attn_bwd_tiled_kernel<ND, NK>, dim3((unsigned)((nq + nk) * std::max(p.qt, p.kt))), dim3(ST_THREADS), smem, st, p, nq, nk);
+  return launch_clusters(attn_bwd_tiled_kernel<TX, ND, NK>, p.split, dim3((unsigned)((nq + nk) * std::max(p.qt, p.kt) * p.split)), dim3(16 * TX), smem, st, p,
+                         nq, nk);
 }
 
 cudaError_t attn_bwd_tiled(const PopeAttnBwdArgs& a, cudaStream_t st) {
@@ -566,8 +668,9 @@ cudaError_t attn_bwd_tiled(const PopeAttnBwdArgs& a, cudaStream_t st) {
   jobs.job[3] = tile_job(a.dout, a.sdo, s.B, s.H, s.Nq, 0, 0, p.DP, p.gimg);
   if ((e = launch_tile_images(jobs, 4, s, a.embed, st)) != cudaSuccess) return e;
   const int kd = s.d + s.r;
-  if (s.d <= 64) return kd <= 64 ? launch_bwd_tiled<4, 4>(p, s, st) : launch_bwd_tiled<4, 8>(p, s, st);
-  return kd <= 128 ? launch_bwd_tiled<8, 8>(p, s, st) : kd <= 192 ? launch_bwd_tiled<8, 12>(p, s, st) : launch_bwd_tiled<8, 16>(p, s, st);
+  p.split = tiled_split((int64_t)p.qt * s.B * s.H + (int64_t)p.kt * s.B * s.Hk, std::min(p.qt, p.kt));
+  if (s.d <= 64) return kd <= 64 ? launch_bwd_tiled<8, 8, 8>(p, s, st) : launch_bwd_tiled<8, 8, 16>(p, s, st);
+  return kd <= 128 ? launch_bwd_tiled<8, 16, 16>(p, s, st) : kd <= 192 ? launch_bwd_tiled<16, 8, 12>(p, s, st) : launch_bwd_tiled<16, 8, 16>(p, s, st);
 }
 
 }  // namespace pope

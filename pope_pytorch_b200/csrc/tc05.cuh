@@ -75,6 +75,20 @@ __device__ __forceinline__ void drain_copies(uint64_t* full, int nst, int first,
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ---- thread-block clusters ---------------------------------------------------------------------------
+// every thread of every CTA of the cluster (whole warps)
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p in the shared memory of CTA `rank` of this cluster
+__device__ __forceinline__ float dsmem_ld(const float* p, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
 // ---- TMA: tiled bulk tensor load into this CTA's shared memory (no multicast) -------------------
 // `tmap` is the address of a CUtensorMap kernel parameter (__grid_constant__).  The innermost coordinate
 // times the element size must be a multiple of 16 bytes.  Rows outside the tensor arrive as zeros.
