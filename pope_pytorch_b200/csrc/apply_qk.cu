@@ -6,8 +6,10 @@
 // (:56); accurate sincosf and log1pf / expf, since the result IS the user-visible value here (no 16-bit rounding
 // follows).  The backward is the chain rule of the same map:
 //   dx = (g_c cos + g_s sin) sigmoid(x),  dphase = a (g_s cos - g_c sin)  -> dfreqs (query and key rows), dbias (key rows).
+#include <algorithm>
+
 #include "kernels.h"
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace pope {
 
@@ -35,78 +37,173 @@ struct ApplyP {
 };
 
 constexpr int AP_THREADS = 256;
-constexpr int AP_ROWS = 16;   // rows per block: the bias gradient of a block is reduced before it touches global memory
+constexpr int AP_ITEMS = 2;    // rotated items per thread and unit
+constexpr int AP_ROWS = 64;    // most rows per block
 
-// grid (row blocks, units, 2 sides); thread = (row within the block, feature): DP = features rounded up to a power of two
-template <typename T, bool BACKWARD>
-__global__ void __launch_bounds__(AP_THREADS) apply_qk_kernel(ApplyP p, int DP) {
-  const ApplySide& s = p.side[blockIdx.z];
-  const int u = blockIdx.y, b = u / s.heads, h = u % s.heads;
-  if (b >= p.B) return;
-  const int c = threadIdx.x % DP, lane_row = threadIdx.x / DP, rows_per_pass = AP_THREADS / DP;
-  const int row_begin = blockIdx.x * AP_ROWS;
-  if (row_begin >= s.rows) return;
-  const bool live = c < p.d;
-  const bool rot = c < p.r;
-  const float hb = (rot && s.bias) ? s.bias[h * s.bias_sh + c] : 0.f;
-  float dbias_acc = 0.f;
-  for (int rr = lane_row; rr < AP_ROWS; rr += rows_per_pass) {
-    const int i = row_begin + rr;
-    if (i >= s.rows || !live) continue;
-    const T* xr = static_cast<const T*>(s.x) + b * s.sx.b + h * s.sx.h + (int64_t)i * s.sx.n;
-    float* yr = s.y + b * s.sy.b + h * s.sy.h + (int64_t)i * s.sy.n;
-    const float x = to_f32<T>(xr[c]);
-    if (rot) {
-      const int pos = s.pos0 + i;
-      const float f = p.freqs[b * p.sf.b + h * p.sf.h + (int64_t)pos * p.sf.n + c];
-      float sn, cs;
-      sincosf(s.bias ? f + hb : f, &sn, &cs);
-      const float a = softplus_f(x);
-      if (!BACKWARD) {
-        *reinterpret_cast<float2*>(yr + 2 * c) = make_float2(a * cs, a * sn);
-      } else {
-        const float2 g = *reinterpret_cast<const float2*>(yr + 2 * c);
-        T* dxr = static_cast<T*>(s.dx) + b * s.sdx.b + h * s.sdx.h + (int64_t)i * s.sdx.n;
-        dxr[c] = from_f32<T>((g.x * cs + g.y * sn) * sigmoid_f(x));
-        const float dphase = a * (g.y * cs - g.x * sn);
-        if (p.dfreqs) atomicAdd(p.dfreqs + b * p.sdf.b + h * p.sdf.h + (int64_t)pos * p.sdf.n + c, dphase);
-        dbias_acc += dphase;
-      }
-    } else {
-      if (!BACKWARD) {
-        yr[p.r + c] = x;
-      } else {
-        T* dxr = static_cast<T*>(s.dx) + b * s.sdx.b + h * s.sdx.h + (int64_t)i * s.sdx.n;
-        dxr[c] = from_f32<T>(yr[p.r + c]);
-      }
-    }
+// N consecutive elements as fp32
+template <int N, typename T> __device__ __forceinline__ void ap_load(const T* src, float (&x)[N]) {
+  if constexpr (N == 1) {
+    x[0] = to_f32<T>(src[0]);
+  } else {
+    struct alignas(N * sizeof(T)) Pack { T v[N]; };
+    const Pack w = *reinterpret_cast<const Pack*>(src);
+#pragma unroll
+    for (int e = 0; e < N; ++e) x[e] = to_f32<T>(w.v[e]);
   }
-  if (BACKWARD && s.dbias) {
-    // one atomic per (block, feature): the row lanes of a feature are summed through shared memory first
-    __shared__ float red[AP_THREADS];
-    red[threadIdx.x] = dbias_acc;
-    __syncthreads();
-    if (lane_row == 0 && rot) {
-      float sum = 0.f;
-      for (int l = 0; l < rows_per_pass; ++l) sum += red[l * DP + c];
-      atomicAdd(s.dbias + h * s.dbias_sh + c, sum);
-    }
+}
+template <int N, typename T> __device__ __forceinline__ void ap_store(T* dst, const float (&x)[N]) {
+  if constexpr (N == 1) {
+    dst[0] = from_f32<T>(x[0]);
+  } else {
+    struct alignas(N * sizeof(T)) Pack { T v[N]; } w;
+#pragma unroll
+    for (int e = 0; e < N; ++e) w.v[e] = from_f32<T>(x[e]);
+    *reinterpret_cast<Pack*>(dst) = w;
   }
 }
 
-static int pow2_at_least(int x) {
-  int p = 1;
-  while (p < x) p <<= 1;
-  return p;
+// grid (row blocks, unit groups, 2 sides).  A block takes `rows_pb` rows of `group` units (u = head x B + batch entry, so that
+// the entries of a head are neighbours).  An item is RW rotated features of a row, or PW plain ones; rotated and plain items
+// are dealt out separately, so that no warp holds both, and a thread keeps its AP_ITEMS rotated items for all units of the
+// group: their cosines and sines (accurate sincosf, half of the arithmetic) are taken once per phase, not once per unit.
+// VEC: pairs of rotated features and quads of plain ones, every access of a warp in whole 16- to 4-byte pieces.
+//
+// Bytes = inputs + outputs: (4, 16, 2048, 64), r = 32, bf16 moves 134 MB forward and 168 MB backward, 21 and 26 us at the
+// copy rate.  One thread per feature and row, half of every warp rotated, a sincosf per unit: forward and backward of a
+// training step 228 us; as here 117 us, of which the kernels take 39 and 64: expf and log1pf keep the arithmetic at
+// about half of that time, more warps (40 registers) spill and are slower (54 + 73), four items per thread too (57 + 104).
+template <typename T, bool BACKWARD, bool VEC>
+__global__ void __launch_bounds__(AP_THREADS, 4) apply_qk_kernel(ApplyP p, int rows_pb, int group) {
+  constexpr int RW = VEC ? 2 : 1, PW = VEC ? 4 : 1;
+  __shared__ float red[BACKWARD ? AP_THREADS * AP_ITEMS * RW : 1];
+  pdl_wait();
+  const ApplySide& s = p.side[blockIdx.z];
+  const int units = p.B * s.heads, u0 = blockIdx.y * group, u1 = min(u0 + group, units);
+  const int row0 = blockIdx.x * rows_pb, nrow = min(rows_pb, s.rows - row0);
+  if (u0 >= units || nrow <= 0) return;
+  const int RP = p.r / RW, PP = (p.d - p.r) / PW;   // rotated and plain items of a row
+  int row[AP_ITEMS], c[AP_ITEMS];
+  bool act[AP_ITEMS];
+  float cs[AP_ITEMS][RW], sn[AP_ITEMS][RW], df[AP_ITEMS][RW], db[AP_ITEMS][RW];
+#pragma unroll
+  for (int k = 0; k < AP_ITEMS; ++k) {
+    const int item = threadIdx.x + AP_THREADS * k;
+    row[k] = RP > 0 ? item / RP : nrow, c[k] = (item - row[k] * RP) * RW, act[k] = row[k] < nrow;
+#pragma unroll
+    for (int e = 0; e < RW; ++e) cs[k][e] = sn[k][e] = df[k][e] = db[k][e] = 0.f;
+  }
+  int h = u0 / p.B, b = u0 - h * p.B;
+  auto flush_freqs = [&]() {   // the gradient of the phases of (b, h), summed over the units that shared them
+    if (!BACKWARD || !p.dfreqs) return;
+#pragma unroll
+    for (int k = 0; k < AP_ITEMS; ++k)
+#pragma unroll
+      for (int e = 0; e < RW; ++e) {
+        if (act[k]) atomicAdd(p.dfreqs + b * p.sdf.b + h * p.sdf.h + (int64_t)(s.pos0 + row0 + row[k]) * p.sdf.n + c[k] + e, df[k][e]);
+        df[k][e] = 0.f;
+      }
+  };
+  auto flush_bias = [&]() {    // one atomic per (block, head, feature); block-uniform
+    if (!BACKWARD || !s.dbias) return;
+#pragma unroll
+    for (int k = 0; k < AP_ITEMS; ++k)
+#pragma unroll
+      for (int e = 0; e < RW; ++e) red[(threadIdx.x + AP_THREADS * k) * RW + e] = db[k][e], db[k][e] = 0.f;
+    __syncthreads();
+    for (int f = threadIdx.x; f < p.r; f += AP_THREADS) {
+      float sum = 0.f;
+      for (int i = 0; i < nrow; ++i) sum += red[i * p.r + f];
+      atomicAdd(s.dbias + h * s.dbias_sh + f, sum);
+    }
+    __syncthreads();
+  };
+  bool fresh = true;
+  for (int u = u0; u < u1; ++u) {
+    const T* x = static_cast<const T*>(s.x) + b * s.sx.b + h * s.sx.h + (int64_t)row0 * s.sx.n;
+    float* y = s.y + b * s.sy.b + h * s.sy.h + (int64_t)row0 * s.sy.n;
+    T* dx = BACKWARD ? static_cast<T*>(s.dx) + b * s.sdx.b + h * s.sdx.h + (int64_t)row0 * s.sdx.n : nullptr;
+    float xv[AP_ITEMS][RW], g[AP_ITEMS][2 * RW];
+#pragma unroll
+    for (int k = 0; k < AP_ITEMS; ++k) {
+      if (!act[k]) continue;
+      ap_load<RW>(x + row[k] * s.sx.n + c[k], xv[k]);
+      if (BACKWARD) ap_load<2 * RW>(y + row[k] * s.sy.n + 2 * c[k], g[k]);
+    }
+    for (int i = threadIdx.x; i < nrow * PP; i += AP_THREADS) {
+      const int rr = i / PP, cc = p.r + (i - rr * PP) * PW;
+      float v[PW];
+      if (!BACKWARD) {
+        ap_load<PW>(x + rr * s.sx.n + cc, v);
+        ap_store<PW>(y + rr * s.sy.n + p.r + cc, v);
+      } else {
+        ap_load<PW>(y + rr * s.sy.n + p.r + cc, v);
+        ap_store<PW>(dx + rr * s.sdx.n + cc, v);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < AP_ITEMS; ++k) {
+      if (!act[k]) continue;
+      if (fresh) {
+        const float* f = p.freqs + b * p.sf.b + h * p.sf.h + (int64_t)(s.pos0 + row0 + row[k]) * p.sf.n + c[k];
+#pragma unroll
+        for (int e = 0; e < RW; ++e) sincosf(s.bias ? f[e] + s.bias[h * s.bias_sh + c[k] + e] : f[e], &sn[k][e], &cs[k][e]);
+      }
+      float out[BACKWARD ? RW : 2 * RW];
+#pragma unroll
+      for (int e = 0; e < RW; ++e) {
+        const float xe = xv[k][e], ex = expf(xe);          // (softplus_f and sigmoid_f with one exponential)
+        const float a = xe > 20.f ? xe : log1pf(ex);
+        if constexpr (BACKWARD) {
+          const float gc = g[k][2 * e], gs = g[k][2 * e + 1];
+          out[e] = (gc * cs[k][e] + gs * sn[k][e]) * (xe > 20.f ? 1.f : ex / (1.f + ex));
+          const float dphase = a * (gs * cs[k][e] - gc * sn[k][e]);
+          df[k][e] += dphase, db[k][e] += dphase;
+        } else {
+          out[2 * e] = a * cs[k][e], out[2 * e + 1] = a * sn[k][e];
+        }
+      }
+      if constexpr (BACKWARD) ap_store<RW>(dx + row[k] * s.sdx.n + c[k], out);
+      else ap_store<2 * RW>(y + row[k] * s.sy.n + 2 * c[k], out);
+    }
+    const int h2 = b + 1 == p.B ? h + 1 : h, b2 = b + 1 == p.B ? 0 : b + 1;
+    fresh = (h2 != h && (s.bias || p.sf.h != 0)) || (b2 != b && p.sf.b != 0);
+    if (BACKWARD && (fresh || u + 1 == u1)) flush_freqs();
+    if (BACKWARD && (h2 != h || u + 1 == u1)) flush_bias();
+    h = h2, b = b2;
+  }
+}
+
+// Whether every row of both sides can be read and written in pieces of 2 and 4 elements.
+template <typename T>
+static bool apply_vectors(const ApplyP& p) {
+  if (p.d % 4 != 0 || p.r % 4 != 0) return false;
+  auto ok = [](const void* ptr, const Strides& st, size_t esz) {
+    return reinterpret_cast<uintptr_t>(ptr) % (4 * esz) == 0 && st.b % 4 == 0 && st.h % 4 == 0 && st.n % 4 == 0;
+  };
+  for (const ApplySide& s : p.side)
+    if (!ok(s.x, s.sx, sizeof(T)) || !ok(s.y, s.sy, 4) || (s.dx && !ok(s.dx, s.sdx, sizeof(T)))) return false;
+  return true;
+}
+
+template <typename T, bool BACKWARD, bool VEC>
+static cudaError_t launch_apply_v(const ApplyP& p, int units_max, int rows_max, cudaStream_t st) {
+  if (p.d > AP_THREADS) return cudaErrorInvalidValue;
+  const int items = p.r / (VEC ? 2 : 1);
+  const int rows_pb = items > 0 ? std::min(AP_ROWS, AP_ITEMS * AP_THREADS / items) : AP_ROWS;
+  const int blocks = (rows_max + rows_pb - 1) / rows_pb;
+  // Units per block: up to 8, whole heads where possible, while six blocks per SM (one and a half times what is resident)
+  // are left.  At (4, 16, 2048, 64), r = 32: 1 unit 55 + 81 us (forward + backward), 2 units 44 + 68, 4 units 40 + 64,
+  // 8 units 39 + 64, 16 units 43 + 68.
+  int group = (int)std::min<int64_t>(8, std::max<int64_t>(1, (int64_t)blocks * units_max * 2 / (148 * 6)));
+  if (group > p.B) group -= group % p.B;
+  const dim3 grid((unsigned)blocks, (unsigned)((units_max + group - 1) / group), 2);
+  return launch_dependent(apply_qk_kernel<T, BACKWARD, VEC>, grid, dim3(AP_THREADS), 0, st, p, rows_pb, group);
 }
 
 template <typename T, bool BACKWARD>
 static cudaError_t launch_apply(const ApplyP& p, int units_max, int rows_max, cudaStream_t st) {
-  const int DP = pow2_at_least(p.d);
-  if (DP > AP_THREADS) return cudaErrorInvalidValue;
-  const dim3 grid((unsigned)((rows_max + AP_ROWS - 1) / AP_ROWS), (unsigned)units_max, 2);
-  apply_qk_kernel<T, BACKWARD><<<grid, AP_THREADS, 0, st>>>(p, DP);
-  return cudaGetLastError();
+  return apply_vectors<T>(p) ? launch_apply_v<T, BACKWARD, true>(p, units_max, rows_max, st)
+                             : launch_apply_v<T, BACKWARD, false>(p, units_max, rows_max, st);
 }
 
 static ApplyP apply_params(const PopeShape& s, const PopeEmbed& e) {
