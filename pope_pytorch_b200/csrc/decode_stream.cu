@@ -660,7 +660,7 @@ static cudaError_t launch_decode_stream(const PopeAttnArgs& a, cudaStream_t st, 
   const unsigned units = (unsigned)(s.B * s.H / G);
   const dim3 grid((unsigned)p.nsplit, units), block(32 * (NW + 1));
   if constexpr (SHORT) {
-    return launch_clusters(kernel, p.nsplit, grid, block, smem, st, p);
+    return launch_clusters(kernel, p.nsplit, grid, block, smem, st, true, p);
   }
   // behind the table kernel, which also zeroes the counters, the decode kernel starts as its programmatic dependent;
   // without rotated features it is the first launch of the call and an ordinary one

@@ -620,7 +620,7 @@ static cudaError_t launch_fwd_tiled(const TiledP& p, const PopeShape& s, cudaStr
   const size_t smem = fwd_smem(p.KD, ND * 8);
   cudaError_t e = ensure_max_smem<attn_fwd_tiled_kernel<ND>>();
   if (e != cudaSuccess) return e;
-  return launch_clusters(attn_fwd_tiled_kernel<ND>, p.split, dim3(p.qt * p.split, s.B * s.H), dim3(128), smem, st, p);
+  return launch_clusters(attn_fwd_tiled_kernel<ND>, p.split, dim3(p.qt * p.split, s.B * s.H), dim3(128), smem, st, true, p);
 }
 
 cudaError_t attn_fwd_tiled(const PopeAttnArgs& a, cudaStream_t st) {
@@ -645,7 +645,7 @@ static cudaError_t launch_bwd_tiled(const TiledP& p, const PopeShape& s, cudaStr
   cudaError_t e = ensure_max_smem<attn_bwd_tiled_kernel<TX, ND, NK>>();
   if (e != cudaSuccess) return e;
   const int nq = s.B * s.H, nk = s.B * s.Hk;
-  return launch_clusters(attn_bwd_tiled_kernel<TX, ND, NK>, p.split, dim3((unsigned)((nq + nk) * std::max(p.qt, p.kt) * p.split)), dim3(16 * TX), smem, st, p,
+  return launch_clusters(attn_bwd_tiled_kernel<TX, ND, NK>, p.split, dim3((unsigned)((nq + nk) * std::max(p.qt, p.kt) * p.split)), dim3(16 * TX), smem, st, true, p,
                          nq, nk);
 }
 

@@ -80,14 +80,18 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// *p in the shared memory of CTA `rank` of this cluster
-__device__ __forceinline__ float dsmem_ld(const float* p, uint32_t rank) {
+// the address of *p in the shared memory of CTA `rank` of this cluster, and a load from such an address
+__device__ __forceinline__ uint32_t dsmem_map(const float* p, uint32_t rank) {
   uint32_t a;
-  float v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float dsmem_ld(uint32_t a) {
+  float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
   return v;
 }
+__device__ __forceinline__ float dsmem_ld(const float* p, uint32_t rank) { return dsmem_ld(dsmem_map(p, rank)); }
 
 // ---- TMA: tiled bulk tensor load into this CTA's shared memory (no multicast) -------------------
 // `tmap` is the address of a CUtensorMap kernel parameter (__grid_constant__).  The innermost coordinate

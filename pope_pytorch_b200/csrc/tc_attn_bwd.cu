@@ -13,6 +13,7 @@
 // phase bias of the keys is part of the K' images.  A streamed tile in shared memory serves two MMAs: as the
 // K-major B operand of the score product and, re-described as MN-major, as the B operand of the gradient
 // product -- the 8x16-byte core-matrix layout is symmetric under that exchange.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -39,6 +40,7 @@ struct TcBwdP {
   int64_t msb, msn;
   float *dfreqs, *dbias;
   unsigned int* status;
+  int split;             // CTAs of a cluster that share the key rows of a dk / dv block
   int img_maps;          // 1: the resident 128-row operand arrives by one tensor-map copy of its image
 };
 

@@ -21,7 +21,9 @@ enum { KB_QFULL = 0,     // [3] Q' tile j (and its lse / delta rows) has landed 
        KB_COUNT = 20 };
 constexpr int KQ_NST = 3, KG_NST = 2;
 
-template <int D, typename T, bool VW>
+// SPLIT: the CTAs of a cluster (p.split of them) share a block of key rows.  (A variant of its own: as a run-time choice the tile
+// arithmetic and the second epilogue cost the unshared sweep 2 % of a training step at (4, 16, 4096, 128).)
+template <int D, typename T, bool VW, bool SPLIT>
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP p, const __grid_constant__ CUtensorMap tmap_v,
                                                                           const __grid_constant__ CUtensorMap tmap_g,
                                                                           const __grid_constant__ CUtensorMap tmap_kimg) {
@@ -39,7 +41,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int u = blockIdx.y, b = u / p.Hk, hk = u % p.Hk;
-  const int j0 = blockIdx.x * BQ;
+  const int split = SPLIT ? p.split : 1, rank = SPLIT ? blockIdx.x % split : 0, kblock = SPLIT ? blockIdx.x / split : blockIdx.x;
+  const int j0 = kblock * BQ;
   const int groups = p.H / p.Hk;
 
   if (warp == BWD_M_WARP) {
@@ -58,12 +61,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP
   // query tiles: under the causal mask rows i < j0 see none of this CTA's keys
   const int m_begin = p.causal ? (j0 / BT) * BT : 0;
   const int tiles_per_group = m_begin < p.Nq ? (p.Nq - m_begin + BT - 1) / BT : 0;
-  const int T_tiles = tiles_per_group * groups;
+  // this CTA's part of them
+  const int all_tiles = tiles_per_group * groups, j_first = SPLIT ? (int)((int64_t)all_tiles * rank / split) : 0;
+  const int T_tiles = SPLIT ? (int)((int64_t)all_tiles * (rank + 1) / split) - j_first : all_tiles;
   // tile j -> (query head of the group, first query row); rotated per CTA like the dq kernel's key order
-  const int rot = tiles_per_group > 0 ? (u * 5 + blockIdx.x * 3) % tiles_per_group : 0;
-  auto tile_head = [&](int j) { return (j / tiles_per_group) * p.Hk + hk; };
+  const int rot = tiles_per_group > 0 ? (u * 5 + kblock * 3) % tiles_per_group : 0;
+  auto tile_head = [&](int j) { return ((j + j_first) / tiles_per_group) * p.Hk + hk; };
   auto tile_start = [&](int j) {
-    int t = j % tiles_per_group + rot;
+    int t = (j + j_first) % tiles_per_group + rot;
     if (t >= tiles_per_group) t -= tiles_per_group;
     return m_begin + t * BT;
   };
@@ -81,7 +86,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP
     // =============================== copies: resident K' / V, then Q' and dO image tiles ==========
     {   // resident K' (phase bias folded in) and V: two image tiles each, one 1 KB copy per chunk column and 64 rows
       const int64_t t0 = (int64_t)u * (int64_t)image_tiles(p.Nk) + j0 / BT;
-      if (T_tiles > 0) {   // (a CTA without any visible query row would leave with these copies in flight)
+      if (all_tiles > 0) {   // (a CTA without any visible query row would leave with these copies in flight)
         if (lane == 0) mbar_expect_tx(&bars[KB_RESIDENT], BQ * KD * 2 + BQ * D * 2);
         __syncwarp();
         if (p.img_maps) {
@@ -207,6 +212,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP
     __syncwarp();
   }
   if (warp >= BWD_E_WARPS) {
+    if constexpr (SPLIT) cluster_sync(), cluster_sync();
     fence_before_sync();
     __syncthreads();
     if (warp == BWD_M_WARP) tmem_dealloc(tmem, 512);
@@ -296,6 +302,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP
   if (T_tiles > 0 && !failed)
     failed = !mbar_wait(&bars[KB_ACCG + (T_tiles - 1) % KG_NST], ((T_tiles - 1) / KG_NST) & 1, WAIT_LIMIT) ||
              !mbar_wait(&bars[KB_ACCQ + (T_tiles - 1) % KQ_NST], ((T_tiles - 1) / KQ_NST) & 1, WAIT_LIMIT);
+  if (SPLIT && all_tiles > 0 && !failed) failed = !mbar_wait(&bars[KB_RESIDENT], 0, WAIT_LIMIT);   // (K' is read below, also without tiles of one's own)
   fence_after_sync();
   asm volatile("bar.sync 1, 256;" ::: "memory");   // every MMA is done: the streamed buffers can be reused
   // Everything below reuses dead shared memory behind the resident K' tile (V and the streamed buffers): row-major
@@ -306,75 +313,150 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP
   //   dk = (dKc kc + dKs ks) / a * sigmoid(k),   dphase = a (dKs cos - dKc sin) = dKs kc - dKc ks,
   // so the epilogue reads neither k nor the phase tables from global memory.  The 16-bit rounding of K' costs the
   // cosine a relative 2^-8 sin^2 at most.  Rows past Nk are zero in the image and produce zeros.
-  constexpr int OSTR = D * 2 + 16;             // bytes of a staged output row (16 bytes of padding: conflict-free)
-  uint8_t* dk_stage = Vs;
-  uint8_t* dv_stage = Vs + BQ * OSTR;
-  float* dmat = reinterpret_cast<float*>(Vs + 2 * BQ * OSTR);   // [128 rows][r + 1]: a thread writes its row, the column sums
-  const int DSTR = p.r + 1;                                     // read along a row; the odd stride keeps both off bank conflicts
-  {
-    constexpr int HW = D / 2;
-    const uint32_t accv = tmem + lane_base + TK_DV, acck = tmem + lane_base + TK_DK;
-    float* dfrow = p.dfreqs ? p.dfreqs + b * p.sdf.b + hk * p.sdf.h + (int64_t)gj * p.sdf.n : nullptr;
-    const bool live = gj < p.Nk;
+  const uint32_t accv = tmem + lane_base + TK_DV, acck = tmem + lane_base + TK_DK;
+  float* dfrow = p.dfreqs ? p.dfreqs + b * p.sdf.b + hk * p.sdf.h + (int64_t)gj * p.sdf.n : nullptr;
+  const bool live = gj < p.Nk;
+  // accumulator columns [cbase, cbase + 16) of this thread's row: dV, and the cosine (or plain) and sine parts of dK'
+  auto load_acc = [&](int cbase, bool rot, float (&gv)[16], float (&gc)[16], float (&gs)[16]) {
+    uint32_t v[16], c[16], n[16];
+    if (T_tiles > 0) {
+      tmem_ld16(accv + cbase, v);
+      tmem_ld16(acck + cbase, c);
+      if (rot) tmem_ld16(acck + D + cbase, n);
+      tmem_ld_wait();
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {   // (no visible query row: zero gradients)
+      gv[e] = T_tiles > 0 ? __uint_as_float(v[e]) : 0.f, gc[e] = T_tiles > 0 ? __uint_as_float(c[e]) : 0.f;
+      gs[e] = T_tiles > 0 && rot ? __uint_as_float(n[e]) : 0.f;
+    }
+  };
+  // dk of the 16 columns, packed, and the phase gradients (zero where nothing is rotated)
+  auto chain_rule = [&](int cbase, bool rot, const float (&gc)[16], const float (&gs)[16], uint32_t (&wk)[8], float (&dph)[16]) {
+    if (rot) {
+      uint32_t cw[8], sw[8];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint4 kcw = *reinterpret_cast<const uint4*>(Ks + (cbase / 8 + i) * (BQ * 16) + row * 16);
+        const uint4 ksw = *reinterpret_cast<const uint4*>(Ks + (D / 8 + cbase / 8 + i) * (BQ * 16) + row * 16);
+        cw[4 * i] = kcw.x, cw[4 * i + 1] = kcw.y, cw[4 * i + 2] = kcw.z, cw[4 * i + 3] = kcw.w;
+        sw[4 * i] = ksw.x, sw[4 * i + 1] = ksw.y, sw[4 * i + 2] = ksw.z, sw[4 * i + 3] = ksw.w;
+      }
+#pragma unroll
+      for (int e = 0; e < 16; e += 2) {
+        const float2 kc = unpack2<T>(cw[e >> 1]), ks = unpack2<T>(sw[e >> 1]);
+        const float m0 = kc.x * kc.x + ks.x * ks.x, m1 = kc.y * kc.y + ks.y * ks.y;   // a^2
+        const float r0 = m0 > 0.f ? rsqrtf(m0) : 0.f, r1 = m1 > 0.f ? rsqrtf(m1) : 0.f;
+        const float sg0 = 1.f - ex2_approx(-m0 * r0 * LOG2E), sg1 = 1.f - ex2_approx(-m1 * r1 * LOG2E);
+        dph[e] = gs[e] * kc.x - gc[e] * ks.x, dph[e + 1] = gs[e + 1] * kc.y - gc[e + 1] * ks.y;
+        if (dfrow && live) atomicAdd(dfrow + cbase + e, dph[e]), atomicAdd(dfrow + cbase + e + 1, dph[e + 1]);
+        wk[e >> 1] = pack2<T>((gc[e] * kc.x + gs[e] * ks.x) * r0 * sg0, (gc[e + 1] * kc.y + gs[e + 1] * ks.y) * r1 * sg1);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) dph[e] = 0.f;
+#pragma unroll
+      for (int e = 0; e < 16; e += 2) wk[e >> 1] = pack2<T>(gc[e], gc[e + 1]);
+    }
+  };
+  constexpr int HW = D / 2;
+  T* dkbase = (T*)p.dk + b * p.sdk.b + hk * p.sdk.h;
+  T* dvbase = (T*)p.dv + b * p.sdv.b + hk * p.sdv.h;
+  if constexpr (SPLIT) {
+    // The parts of the query range meet.  The accumulators are cut into chunks of 16 columns (dV, and both parts of dK'); a
+    // CTA leaves the chunks that another one finishes in its shared memory, [chunk slot][48][128 rows] fp32, and finishes the
+    // chunks c % split == rank itself: its own accumulator plus the others' out of theirs, 32-byte pieces of dk and dv
+    // straight to global memory.
+    float* dump = reinterpret_cast<float*>(Vs);
+    auto slot = [&](int chunk, int r) { return chunk - (chunk - r + split - 1) / split; };   // chunks before it that r does not own
 #pragma unroll
     for (int c0 = 0; c0 < HW; c0 += 16) {
-      const int cbase = half * HW + c0;
-      uint32_t gv[16], gc[16], gs[16];
-      const bool rot = cbase < p.r && T_tiles > 0;
-      if (T_tiles > 0) {
-        tmem_ld16(accv + cbase, gv);
-        tmem_ld16(acck + cbase, gc);
-        if (rot) tmem_ld16(acck + D + cbase, gs);
-        tmem_ld_wait();
-      } else {   // no visible query row: zero gradients (the resident tiles were never loaded)
+      const int cbase = half * HW + c0, chunk = cbase / 16;
+      if (chunk % split == rank) continue;
+      float gv[16], gc[16], gs[16];
+      load_acc(cbase, cbase < p.r, gv, gc, gs);
+      float* dst = dump + slot(chunk, rank) * (48 * BQ) + row;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) gv[e] = gc[e] = gs[e] = 0u;
+      for (int e = 0; e < 16; ++e) dst[e * BQ] = gv[e], dst[(16 + e) * BQ] = gc[e];
+      if (cbase < p.r) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) dst[(32 + e) * BQ] = gs[e];
+      }
+    }
+    __syncwarp();
+    cluster_sync();
+#pragma unroll
+    for (int c0 = 0; c0 < HW; c0 += 16) {
+      const int cbase = half * HW + c0, chunk = cbase / 16;
+      if (chunk % split != rank) continue;
+      const bool rot = cbase < p.r;
+      float gv[16], gc[16], gs[16], dph[16];
+      load_acc(cbase, rot, gv, gc, gs);
+      for (int i = 1; i < split; ++i) {
+        const int r = rank + i < split ? rank + i : rank + i - split;
+        const uint32_t src = dsmem_map(dump + slot(chunk, r) * (48 * BQ) + row, r);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) gv[e] += dsmem_ld(src + e * BQ * 4), gc[e] += dsmem_ld(src + (16 + e) * BQ * 4);
+        if (rot) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) gs[e] += dsmem_ld(src + (32 + e) * BQ * 4);
+        }
       }
       uint32_t wv[8], wk[8];
 #pragma unroll
-      for (int e = 0; e < 16; e += 2) wv[e >> 1] = pack2<T>(__uint_as_float(gv[e]), __uint_as_float(gv[e + 1]));
-      if (rot) {
-        uint32_t cw[8], sw[8];
+      for (int e = 0; e < 16; e += 2) wv[e >> 1] = pack2<T>(gv[e], gv[e + 1]);
+      chain_rule(cbase, rot && all_tiles > 0, gc, gs, wk, dph);
+      if (live) {
+        uint4* dv4 = reinterpret_cast<uint4*>(dvbase + (int64_t)gj * p.sdv.n + cbase);
+        uint4* dk4 = reinterpret_cast<uint4*>(dkbase + (int64_t)gj * p.sdk.n + cbase);
+        dv4[0] = make_uint4(wv[0], wv[1], wv[2], wv[3]), dv4[1] = make_uint4(wv[4], wv[5], wv[6], wv[7]);
+        dk4[0] = make_uint4(wk[0], wk[1], wk[2], wk[3]), dk4[1] = make_uint4(wk[4], wk[5], wk[6], wk[7]);
+      }
+      if (p.dbias && rot) {
+        // sums over the warp's rows, halving the columns a lane carries with every step; lane l ends up with column l / 2
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const uint4 kcw = *reinterpret_cast<const uint4*>(Ks + (cbase / 8 + i) * (BQ * 16) + row * 16);
-          const uint4 ksw = *reinterpret_cast<const uint4*>(Ks + (D / 8 + cbase / 8 + i) * (BQ * 16) + row * 16);
-          cw[4 * i] = kcw.x, cw[4 * i + 1] = kcw.y, cw[4 * i + 2] = kcw.z, cw[4 * i + 3] = kcw.w;
-          sw[4 * i] = ksw.x, sw[4 * i + 1] = ksw.y, sw[4 * i + 2] = ksw.z, sw[4 * i + 3] = ksw.w;
+        for (int n = 8; n >= 1; n /= 2) {
+          const bool hi = (lane & (2 * n)) != 0;
+#pragma unroll
+          for (int e = 0; e < n; ++e) {
+            const float give = hi ? dph[e] : dph[e + n], keep = hi ? dph[e + n] : dph[e];
+            dph[e] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * n);
+          }
         }
+        dph[0] += __shfl_xor_sync(0xffffffffu, dph[0], 1);
+        if ((lane & 1) == 0) atomicAdd(p.dbias + hk * p.dbias_sh + cbase + (lane >> 1), dph[0]);
+      }
+    }
+    __syncwarp();
+    cluster_sync();   // nobody leaves while its shared memory is read
+  } else {
+    constexpr int OSTR = D * 2 + 16;             // bytes of a staged output row (16 bytes of padding: conflict-free)
+    uint8_t* dk_stage = Vs;
+    uint8_t* dv_stage = Vs + BQ * OSTR;
+    float* dmat = reinterpret_cast<float*>(Vs + 2 * BQ * OSTR);   // [128 rows][r + 1]: a thread writes its row, the column sums
+    const int DSTR = p.r + 1;                                     // read along a row; the odd stride keeps both off bank conflicts
 #pragma unroll
-        for (int e = 0; e < 16; e += 2) {
-          const float2 kc = unpack2<T>(cw[e >> 1]), ks = unpack2<T>(sw[e >> 1]);
-          const float g0 = __uint_as_float(gc[e]), g1 = __uint_as_float(gc[e + 1]);
-          const float h0 = __uint_as_float(gs[e]), h1 = __uint_as_float(gs[e + 1]);
-          const float m0 = kc.x * kc.x + ks.x * ks.x, m1 = kc.y * kc.y + ks.y * ks.y;   // a^2
-          const float r0 = m0 > 0.f ? rsqrtf(m0) : 0.f, r1 = m1 > 0.f ? rsqrtf(m1) : 0.f;
-          const float sg0 = 1.f - ex2_approx(-m0 * r0 * LOG2E), sg1 = 1.f - ex2_approx(-m1 * r1 * LOG2E);
-          const float d0 = h0 * kc.x - g0 * ks.x, d1 = h1 * kc.y - g1 * ks.y;
-          if (dfrow && live) atomicAdd(dfrow + cbase + e, d0), atomicAdd(dfrow + cbase + e + 1, d1);
-          if (p.dbias) dmat[row * DSTR + cbase + e] = d0, dmat[row * DSTR + cbase + e + 1] = d1;
-          wk[e >> 1] = pack2<T>((g0 * kc.x + h0 * ks.x) * r0 * sg0, (g1 * kc.y + h1 * ks.y) * r1 * sg1);
-        }
-      } else {
-        if (p.dbias && cbase < p.r) {
+    for (int c0 = 0; c0 < HW; c0 += 16) {
+      const int cbase = half * HW + c0;
+      float gv[16], gc[16], gs[16], dph[16];
+      const bool rot = cbase < p.r && T_tiles > 0;
+      load_acc(cbase, rot, gv, gc, gs);
+      uint32_t wv[8], wk[8];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) dmat[row * DSTR + cbase + e] = 0.f;
-        }
+      for (int e = 0; e < 16; e += 2) wv[e >> 1] = pack2<T>(gv[e], gv[e + 1]);
+      chain_rule(cbase, rot, gc, gs, wk, dph);
+      if (p.dbias && cbase < p.r) {
 #pragma unroll
-        for (int e = 0; e < 16; e += 2) wk[e >> 1] = pack2<T>(__uint_as_float(gc[e]), __uint_as_float(gc[e + 1]));
+        for (int e = 0; e < 16; ++e) dmat[row * DSTR + cbase + e] = dph[e];
       }
       *reinterpret_cast<uint4*>(dv_stage + row * OSTR + cbase * 2) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
       *reinterpret_cast<uint4*>(dv_stage + row * OSTR + cbase * 2 + 16) = make_uint4(wv[4], wv[5], wv[6], wv[7]);
       *reinterpret_cast<uint4*>(dk_stage + row * OSTR + cbase * 2) = make_uint4(wk[0], wk[1], wk[2], wk[3]);
       *reinterpret_cast<uint4*>(dk_stage + row * OSTR + cbase * 2 + 16) = make_uint4(wk[4], wk[5], wk[6], wk[7]);
     }
-  }
-  asm volatile("bar.sync 1, 256;" ::: "memory");
-  {
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     // dk / dv rows leave 16 bytes per thread: consecutive threads cover one 2 D-byte row after the other
     constexpr int GPR = D / 8;   // 16-byte groups per row
-    T* dkbase = (T*)p.dk + b * p.sdk.b + hk * p.sdk.h;
-    T* dvbase = (T*)p.dv + b * p.sdv.b + hk * p.sdv.h;
     for (int idx = tid; idx < BQ * GPR; idx += 256) {
       const int rr = idx / GPR, g = idx - rr * GPR;
       if (j0 + rr < p.Nk) {
@@ -534,16 +616,34 @@ class ForkGuard {
   std::unique_lock<std::mutex> lock_;
 };
 
+// CTAs that share a 128-key block of dk / dv.  With grouped heads a block sweeps the query tiles of all heads of its group, one
+// after the other, while few blocks are there to fill the chip: the sweep is what the call waits for, and is cut until it is no
+// longer than that of a dq block, which runs beside it.  Whole training steps as a graph, d = 64 to 128, on 1 / 2 / 4 CTAs:
+// (1, 8 / 2, 2048) 242 / 172 / 140 us, (2, 8 / 2, 1024) 178 / 138 / 123, (1, 32 / 4, 500) 144 / 113 / 94, and the kernel of
+// (3, 8 / 2, 777) 68 / 43 / 42.  Without groups the sweep is no longer than dq's and the merge costs more than it gives:
+// (1, 8, 1024) 71 / 74 / 81, (2, 8, 600) 61 / 62 / 75.  Above 172 CTAs the blocks fill the chip by themselves.
+static int dkdv_split(const PopeShape& s) {
+  const int64_t ctas = (int64_t)((s.Nk + BQ - 1) / BQ) * s.B * s.Hk;
+  int split = 1;
+  while (split < 4 && s.H / s.Hk >= 2 * split && ctas * 2 * split <= 172) split *= 2;
+  return split;
+}
+
 template <int D, typename T, bool VW>
 static cudaError_t launch_bwd_kernels(const TcBwdP& p, const PopeShape& s, size_t smem_q, size_t smem_k, const CUtensorMap& tv64,
                                       const CUtensorMap& tv128, const CUtensorMap& tg64, const CUtensorMap& tqi,
                                       const CUtensorMap& tki, cudaStream_t st, cudaStream_t sk) {
   cudaError_t e;
   if ((e = ensure_max_smem<attn_bwd_dq_tc_kernel<D, T, VW>>()) != cudaSuccess) return e;
-  if ((e = ensure_max_smem<attn_bwd_dkdv_tc_kernel<D, T, VW>>()) != cudaSuccess) return e;
   attn_bwd_dq_tc_kernel<D, T, VW><<<dim3((s.Nq + BQ - 1) / BQ, s.B * s.H), BWD_THREADS, smem_q, st>>>(p, tv64, tqi);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  attn_bwd_dkdv_tc_kernel<D, T, VW><<<dim3((s.Nk + BQ - 1) / BQ, s.B * s.Hk), BWD_THREADS, smem_k, sk>>>(p, tv128, tg64, tki);
+  const dim3 grid((unsigned)((s.Nk + BQ - 1) / BQ * p.split), (unsigned)(s.B * s.Hk));
+  if (p.split > 1) {
+    if ((e = ensure_max_smem<attn_bwd_dkdv_tc_kernel<D, T, VW, true>>()) != cudaSuccess) return e;
+    return launch_clusters(attn_bwd_dkdv_tc_kernel<D, T, VW, true>, p.split, grid, dim3(BWD_THREADS), smem_k, sk, false, p, tv128, tg64, tki);
+  }
+  if ((e = ensure_max_smem<attn_bwd_dkdv_tc_kernel<D, T, VW, false>>()) != cudaSuccess) return e;
+  attn_bwd_dkdv_tc_kernel<D, T, VW, false><<<grid, BWD_THREADS, smem_k, sk>>>(p, tv128, tg64, tki);
   return cudaGetLastError();
 }
 
@@ -599,6 +699,7 @@ static cudaError_t launch_bwd_tc(const PopeAttnBwdArgs& a, cudaStream_t st) {
   p.sfn = a.embed.sf.n, p.bias_sh = a.embed.bias_stride_h, p.dbias_sh = a.dbias_stride_h;
   p.kimg = kimg, p.qimg = qimg, p.vimg = vimg, p.gimg = gimg, p.rowstat = rowstat;
   p.mask = a.mask, p.msb = a.mask_stride_b, p.msn = a.mask_stride_n;
+  p.split = dkdv_split(s);
   p.dfreqs = s.r > 0 ? a.dfreqs : nullptr, p.dbias = s.r > 0 ? a.dbias : nullptr;
   p.status = tc_status_ptr();
   if (!p.status) return cudaErrorInvalidSymbol;
@@ -613,6 +714,10 @@ static cudaError_t launch_bwd_tc(const PopeAttnBwdArgs& a, cudaStream_t st) {
   // every CTA allocates all 512 TMEM columns: keep two CTAs from sharing an SM
   if (smem_q < 120 * 1024) smem_q = 120 * 1024;
   if (smem_k < 120 * 1024) smem_k = 120 * 1024;
+  if (p.split > 1) {   // the chunks a CTA leaves to the others, behind K'; at most 64 + 144 + 1 KB
+    const size_t chunks = (size_t)D / 16, dump = (chunks - chunks / p.split) * 48 * BQ * 4;
+    smem_k = std::max(smem_k, (size_t)BQ * KD * 2 + dump + 1024);
+  }
   if (fork) {   // images -> side stream (dk/dv); row statistics -> caller's stream (dq reads delta)
     if ((e = cudaEventRecord(fk->ready, st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(fk->side, fk->ready, 0)) != cudaSuccess) return e;
