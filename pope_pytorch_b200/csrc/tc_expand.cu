@@ -19,15 +19,14 @@
 
 namespace pope {
 
-// grid (tiles / 4, units, jobs), 256 threads; dynamic shared memory (d+r)/8 * CS64 bytes + 2 r floats.  One launch
+// grid (tiles / tpc, units, jobs), 256 threads; dynamic shared memory (d+r)/8 * CS64 bytes + 2 r floats.  One launch
 // builds the images of up to four operands (blockIdx.z picks the job); CTAs outside a job's tile / unit range leave.
-// A CTA builds EXPAND_TPC consecutive tiles of one unit.  A thread keeps the same 16-byte feature group (chunk) for
+// A CTA builds tpc (1, 2 or 4) consecutive tiles of one unit.  A thread keeps the same 16-byte feature group (chunk) for
 // every row it touches, so whether it rotates at all, and the cos / sin of the head's phase offset for its eight
 // features, are fixed for its lifetime (registers instead of 16 shared-memory loads per group); the raw rows of the
 // next tile are requested before the current tile is worked on.
-constexpr int EXPAND_TPC = 4;
 template <typename T, int D>
-__global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, const __half* __restrict__ ctab,
+__global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, int tpc, const __half* __restrict__ ctab,
                                                             const __half* __restrict__ stab) {
   // (ctab / stab are advanced to the unit's table slice below)
   extern __shared__ __align__(16) uint8_t stage[];
@@ -35,8 +34,8 @@ __global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, c
   pdl_trigger();   // the attention kernel behind this one may set itself up, and read the caller's V
   const ExpandJob& jb = jobs.job[blockIdx.z];
   const int tid = threadIdx.x, u = blockIdx.y;
-  const int tiles = (int)image_tiles(jb.rows);   // a multiple of EXPAND_TPC
-  const int tile0 = blockIdx.x * EXPAND_TPC;
+  const int tiles = (int)image_tiles(jb.rows);   // a multiple of 4
+  const int tile0 = blockIdx.x * tpc;
   if (tile0 >= tiles || u >= jb.units) return;
   const int r = jb.r, rows = jb.rows;
   constexpr int DC = D >> 3;
@@ -71,7 +70,7 @@ __global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, c
       if (active && row < IMAGE_ROWS && jrow < rows) raw[it] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)jrow * sx.n));
     }
   };
-  for (int tt = 0; tt < EXPAND_TPC; ++tt) {
+  for (int tt = 0; tt < tpc; ++tt) {
     const int tile = tile0 + tt;
     uint4 raw[NIT];
     load_raw(tile, raw);
@@ -135,7 +134,7 @@ __global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, c
         out[g] = *reinterpret_cast<const uint4*>(stage + cc * CS64 + row * 16);
       }
     }
-    if (tt + 1 < EXPAND_TPC) __syncthreads();   // the stage is rewritten by the next tile
+    if (tt + 1 < tpc) __syncthreads();   // the stage is rewritten by the next tile
   }
 }
 
@@ -143,17 +142,25 @@ template <typename T>
 static cudaError_t launch_expand_t(const ExpandJobs& jobs, int njobs, int d, const __half* ctab, const __half* stab,
                                    cudaStream_t st) {
   int tiles = 0, units = 0, rmax = 0;
+  int64_t total = 0;
   for (int i = 0; i < njobs; ++i) {
-    tiles = std::max(tiles, (int)image_tiles(jobs.job[i].rows));
+    const int t = (int)image_tiles(jobs.job[i].rows);
+    tiles = std::max(tiles, t), total += (int64_t)t * jobs.job[i].units;
     units = std::max(units, jobs.job[i].units);
     rmax = std::max(rmax, jobs.job[i].r);
   }
-  const dim3 grid((unsigned)(tiles / EXPAND_TPC), (unsigned)units, (unsigned)njobs);
+  // Tiles per CTA: four, which share what a CTA sets up, while that leaves every SM the three CTAs it holds, fewer for less
+  // work, where four in a row are only four times the latency.  Forward calls as a graph, four tiles / by this rule:
+  // (2, 8, 1024, 64) 26.6 / 20.6 us, (1, 16, 2048, 128) 63.7 / 55.4, (2, 16, 2048, 128) 110.7 / 107.1, (1, 4, 200, 64) 16.5 / 14.5.
+  // (Taking the cosines and sines here as well, without a table kernel, gave nothing at the smallest call, 14.4, and lost from
+  // 0.5 million rotated elements on: 22.6 against 20.6.)
+  const int tpc = total >= 4 * 3 * 148 ? 4 : total >= 2 * 3 * 148 ? 2 : 1;
+  const dim3 grid((unsigned)(tiles / tpc), (unsigned)units, (unsigned)njobs);
   const size_t smem = (size_t)((d + rmax) / 8) * CS64 + 2 * (size_t)rmax * sizeof(float);
   switch (d) {
-    case 64: return launch_dependent(expand_image_kernel<T, 64>, grid, dim3(256), smem, st, jobs, ctab, stab);
-    case 96: return launch_dependent(expand_image_kernel<T, 96>, grid, dim3(256), smem, st, jobs, ctab, stab);
-    case 128: return launch_dependent(expand_image_kernel<T, 128>, grid, dim3(256), smem, st, jobs, ctab, stab);
+    case 64: return launch_dependent(expand_image_kernel<T, 64>, grid, dim3(256), smem, st, jobs, tpc, ctab, stab);
+    case 96: return launch_dependent(expand_image_kernel<T, 96>, grid, dim3(256), smem, st, jobs, tpc, ctab, stab);
+    case 128: return launch_dependent(expand_image_kernel<T, 128>, grid, dim3(256), smem, st, jobs, tpc, ctab, stab);
     default: return cudaErrorInvalidValue;
   }
 }
