@@ -12,7 +12,8 @@
 // With q' = (a_q cos fq, a_q sin fq) and k' = (a_k cos(fk + b), a_k sin(fk + b)) the score term of a rotated feature
 // is a_q a_k cos(fq - fk - b) = a_k (Qc cos fk + Qs sin fk), Qc = a_q cos(fq - b), Qs = a_q sin(fq - b): the head's bias
 // is folded into the query once per CTA and the key side needs only the bias-free table shared by all units.
-// Key ranges are split over CTAs; each CTA writes a partial (o, max, sum) that the split combine merges.
+// Key ranges are split over CTAs; their partial (o, max, sum) meet in the kernel: in a cluster's shared
+// memory, or in the workspace, where the CTA that finishes last merges its unit.
 //
 // Semantics: PoPE_pytorch/triton_pope_flash_attn.py:52-57,73-80 (transform), :89-91 (mask, True = keep), :96-117
 // (softmax, empty rows); the query sits at the LAST table row (PoPE_pytorch/pope.py:64).
@@ -734,7 +735,7 @@ size_t decode_paged_workspace(const PopePagedDecodeArgs& g) {
 }
 
 cudaError_t decode_paged(const PopePagedDecodeArgs& g, cudaStream_t st) {
-  // the row statistics of the split combine go to the caller's lse or, without one, to the end of the workspace
+  // the row statistics go to the caller's lse or, without one, to the end of the workspace
   float* lse = g.lse;
   if (!lse) lse = reinterpret_cast<float*>(static_cast<uint8_t*>(g.workspace) + decode_stream_workspace(paged_as_attn(g, nullptr)));
   const PopeAttnArgs a = paged_as_attn(g, lse);
