@@ -332,9 +332,32 @@ def apply_qk_supported(q, k, freqs, bias) -> bool:
             and freqs.ndim in (2, 3, 4) and bias.ndim == 2 and is_available())
 
 
+class _Recorded(torch.autograd.Function):
+    """An operator as one node of a ``torch.jit.trace`` recording, which does not see into the extension module (the result
+    would be recorded as a constant); the gradients run the operator again."""
+
+    @staticmethod
+    def forward(ctx, name, count, *args):
+        ctx.name, ctx.rest = name, args[count:]
+        ctx.save_for_backward(*args[:count])
+        return getattr(_ops(), name)(*args)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        ins = [t.detach().requires_grad_(t.requires_grad) for t in ctx.saved_tensors]
+        with torch.enable_grad():
+            out = getattr(_ops(), ctx.name)(*ins, *ctx.rest)
+        out = out if isinstance(out, tuple) else (out,)
+        wanted = [t for t in ins if t.requires_grad]
+        got = iter(torch.autograd.grad(out, wanted, grads))
+        return None, None, *(next(got) if t.requires_grad else None for t in ins), *(None for _ in ctx.rest)
+
+
 def apply_qk(q, k, freqs, bias):
     """Differentiable fused transform on head-first (b,h,n,d) tensors -> fp32 (q', k') in the
     reference's interleaved layout."""
+    if torch._C._is_tracing():
+        return _Recorded.apply("apply_qk", 4, q, k, freqs, bias)
     return _ops().apply_qk(q, k, freqs, bias)
 
 
@@ -372,6 +395,8 @@ def flash_attn(q, k, v, freqs=None, bias=None, mask=None, causal=False, softmax_
         head, row = (2, 1) if seq_first else (1, 2)
         freqs = torch.empty(k.shape[row], 0, dtype=torch.float32, device=q.device)
         bias = torch.empty(k.shape[head], 0, dtype=torch.float32, device=q.device)
+    if torch._C._is_tracing():
+        return _Recorded.apply("flash_attn", 5, q, k, v, freqs, bias, mask, causal, scale, None, seq_first)
     return _ops().flash_attn(q, k, v, freqs, bias, mask, causal, scale, _attached(freqs), seq_first)
 
 

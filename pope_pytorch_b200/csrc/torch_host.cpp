@@ -5,6 +5,7 @@
 // 351 us per (3, 8 / 2, 777, 64) training step whose kernels take 159 us; here they take 27 and 148 us.  The kernels themselves stay behind
 // the C ABI (include/pope_b200.h): this file only fills its structs.  No arithmetic happens here and nothing is kept from one
 // call to the next.
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -208,9 +209,11 @@ struct FlashAttn : torch::autograd::Function<FlashAttn> {
   }
 };
 
+// Whether the call goes through its autograd node: for gradients, and for tangents of forward mode, which the node refuses
+// (a call past it would drop them).
 template <typename... Ts>
 bool wants_graph(const Ts&... ts) {
-  return at::GradMode::is_enabled() && (ts.requires_grad() || ...);
+  return (at::GradMode::is_enabled() && (ts.requires_grad() || ...)) || (ts._fw_grad(0).defined() || ...);
 }
 
 Tensor flash_attn(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask,
@@ -381,9 +384,12 @@ struct Table : torch::autograd::Function<Table> {
   }
 };
 
-// None when the module's tensors are not what the kernel takes (another type or device, frequencies that train, ...)
+// None when the module's tensors are not what the kernel takes (another type or device, frequencies that train, tensors of a
+// function transform or of a dispatch mode, forward mode): the module's own PyTorch operations serve those
 optional<std::vector<Tensor>> table(const Tensor& bias, const std::vector<Tensor>& inv, const std::vector<int64_t>& dims, double offset) {
-  auto plain = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous(); };
+  auto plain = [](const Tensor& t) {
+    return !at::isTensorSubclassLike(t) && t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && !t._fw_grad(0).defined();
+  };
   if (inv.empty() || inv.size() != dims.size() || inv.size() > POPE_MAX_AXES || bias.dim() != 2 || !plain(bias)) return std::nullopt;
   int64_t n = 1, r = 0;
   for (const int64_t d : dims) {

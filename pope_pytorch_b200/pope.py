@@ -87,6 +87,11 @@ def _apply_pope_to_qk_torch(freqs, bias, q, k, to_magnitude, return_complex):
     return q_out, k_out
 
 
+def _traced() -> bool:
+    """Whether a compiler or ``torch.jit.trace`` is recording: it sees PyTorch operations only."""
+    return torch._C._is_tracing() or torch.compiler.is_compiling()
+
+
 class PoPE(nn.Module):
     """Polar positional embedding: one frequency per rotated feature, theta^(-c/dim), and a
     learned per-head key phase kept in [-2pi, 0]."""
@@ -111,7 +116,8 @@ class PoPE(nn.Module):
         return self.inv_freqs.device
 
     def forward(self, pos_or_seq_len: Union[Tensor, int], offset=0) -> PolarEmbedReturn:
-        if self.bias.is_cuda and isinstance(pos_or_seq_len, int) and isinstance(offset, (int, float)):
+        if self.bias.is_cuda and isinstance(pos_or_seq_len, int) and isinstance(offset, (int, float)) \
+                and not _traced():
             from . import _native          # one launch instead of a chain of elementwise kernels
             made = _native.embed_table(self.bias, [self.inv_freqs], [pos_or_seq_len], offset)
             if made is not None:

@@ -12,7 +12,7 @@ from typing import Optional, Tuple, Union
 import torch
 from torch import Tensor, nn
 
-from .pope import TWO_PI, FactoredPolarEmbed, PolarEmbedReturn, apply_pope_to_qk
+from .pope import TWO_PI, FactoredPolarEmbed, PolarEmbedReturn, _traced, apply_pope_to_qk
 
 
 class AxialPoPE(nn.Module):
@@ -44,7 +44,7 @@ class AxialPoPE(nn.Module):
         return coords.flip(-1)
 
     def forward(self, pos_or_dims: Union[Tensor, Tuple[int, ...]]) -> PolarEmbedReturn:
-        if self.bias.is_cuda and isinstance(pos_or_dims, tuple) and len(pos_or_dims) == len(self.axial_dims) > 1:
+        if self.bias.is_cuda and isinstance(pos_or_dims, tuple) and len(pos_or_dims) == len(self.axial_dims) > 1 and not _traced():
             from . import _native          # one launch instead of a chain of elementwise kernels
             made = _native.embed_table(self.bias, list(self.inv_freqs), list(pos_or_dims))
             if made is not None:
