@@ -17,8 +17,9 @@
 //                   G = hi + lo and writes them as 16-byte chunks of 8 keys; that one layout serves both sides -- as the
 //                   K-major A operand of G K' and, re-described as MN-major, as the A operand of G^T Q'
 //   issuing warps : two, taking the even and the odd steps: three MMA chains per step, hi*hi' + hi*lo' + lo*hi' (fp32
-//                   accuracy from bf16 products, as in the forward), accumulating in TMEM over the whole sweep
-// and the epilogue applies the chain rule with accurate sincosf / softplus on the rows it owns.
+//                   accuracy from bf16 products, as in the forward), each accumulating in TMEM columns of its own over the
+//                   whole sweep
+// and the epilogue adds the two accumulators and applies the chain rule with accurate sincosf / softplus on the rows it owns.
 #include <algorithm>
 #include <cstring>
 
@@ -57,8 +58,8 @@ enum { WB_GFULL = 0,     // [3] the G tile of step s has landed in staging buffe
        WB_CONV = 6,      // [2] 8 worker warps: the converted tile of step s is in buffer s & 1
        WB_IFULL = 8,     // [2] the operand tile of step s has landed in buffer s & 1 (transaction bytes)
        WB_DONE = 10,     // [2] tcgen05.commit: the chains of step s have completed: both buffers s & 1 are free
-       WB_HEAD = 12,     // the first instruction of step 0 (the one that overwrites the accumulator) has been issued
-       WB_COUNT = 13 };
+       WB_COUNT = 12 };
+constexpr uint32_t SBW_ACC = 128;    // TMEM columns of one accumulator (shared memory holds no d + r above that): even steps, odd steps
 
 // One side of the backward for one CTA: resident block `blk` (128 rows) of unit `u` (batch x query heads on the query
 // side, batch x key heads on the key side).
@@ -90,7 +91,7 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
   const int S = steps_per_head * groups;
 
   if (warp == SBW_MMA_WARP) {
-    tmem_alloc(tmem_slot, 256);
+    tmem_alloc(tmem_slot, 2 * SBW_ACC);
     tmem_relinquish();
   }
   if (tid == 0) {
@@ -98,7 +99,6 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[WB_CONV + i], 8), mbar_init(&bars[WB_IFULL + i], 1), mbar_init(&bars[WB_DONE + i], 1);
     }
-    mbar_init(&bars[WB_HEAD], 1);
     mbar_init_fence();
   }
   fence_before_sync();
@@ -161,11 +161,11 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
     // =============================== MMA issue ====================================================
     // Two issuing threads take the even and the odd steps.  Around the 12 instructions of a step (about 630 clocks of
     // issue) one thread spends as long again on its waits, fences and commits, and it alone set the pace of the loop;
-    // alternating, each has two steps' time for one step's work.  Every instruction accumulates into the same columns
-    // except the first of step 0, so the odd thread starts once that one has been issued.
+    // alternating, each has two steps' time for one step's work.  Products into one accumulator are ordered only when ONE
+    // thread issues them, so each has columns of its own.
     if (lane == 0) {
       const int first = warp == SBW_MMA_WARP ? 0 : 1;
-      if (first == 1 && S > 1) failed = !mbar_wait(&bars[WB_HEAD], 0, WAIT_LIMIT);
+      const uint32_t acc = tmem + first * SBW_ACC;
       // query side: A = G (K-major: 128 query rows x 16 keys per step); key side: A = G^T (MN-major: 128 keys x 16 query rows)
       const uint32_t idesc = instr_desc(FMT_BF16, 128, KD, KEY_SIDE, true);
       const uint32_t g_addr = smem_u32(Gbf), i_addr = smem_u32(Img);
@@ -185,9 +185,8 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {   // 16 swept rows per instruction
             const uint32_t astep = KEY_SIDE ? ks * ((2 * 128) >> 4) : ks * ((2 * GCS) >> 4);
-            mma_ss_lh(tmem, desc_lo(ad) + astep, desc_hi(ad), desc_lo(bd) + ks * ((2 * 128) >> 4), desc_hi(bd), idesc,
-                      (s > 0 || ch > 0 || ks > 0) ? 1u : 0u);
-            if (s == 0 && ch == 0 && ks == 0) mbar_arrive(&bars[WB_HEAD]);
+            mma_ss_lh(acc, desc_lo(ad) + astep, desc_hi(ad), desc_lo(bd) + ks * ((2 * 128) >> 4), desc_hi(bd), idesc,
+                      (s > first || ch > 0 || ks > 0) ? 1u : 0u);
           }
         }
         mma_commit(&bars[WB_DONE + buf]);
@@ -246,14 +245,14 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
       const int row = tid & 127, grp = tid >> 7;
       const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16);
       for (int cg = grp; cg * 16 < KD; cg += 2) {
-        uint32_t w[16];
-        if (S > 0) {
-          tmem_ld16(acc + cg * 16, w);
-          tmem_ld_wait();
-        } else {
+        uint32_t w[16], w1[16];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) w[e] = 0u;
-        }
+        for (int e = 0; e < 16; ++e) w[e] = w1[e] = 0u;
+        if (S > 0) tmem_ld16(acc + cg * 16, w);
+        if (S > 1) tmem_ld16(acc + SBW_ACC + cg * 16, w1);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(__uint_as_float(w[e]) + __uint_as_float(w1[e]));
         uint4* dst = reinterpret_cast<uint4*>(accs + row * ASTR + cg * 64);
 #pragma unroll
         for (int e = 0; e < 4; ++e) dst[e] = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
@@ -335,7 +334,7 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
   }
   fence_before_sync();
   __syncthreads();
-  if (warp == SBW_MMA_WARP) tmem_dealloc(tmem, 256);
+  if (warp == SBW_MMA_WARP) tmem_dealloc(tmem, 2 * SBW_ACC);
 }
 
 // Both sides in ONE launch, 1-D grid.  Blocks are numbered so that the CTAs of one (batch, key head) group are
@@ -371,7 +370,7 @@ cudaError_t sim_launch_prepass(const PopeShape& s, const PopeEmbed& e, const voi
 bool sim_bwd_tc_supported(const PopeSimBwdArgs& a) {
   const PopeShape& s = a.shape;
   if (s.dtype != POPE_F32) return false;
-  if (s.d % 16 != 0 || s.r % 8 != 0 || (s.d + s.r) % 16 != 0 || s.d + s.r > 256) return false;
+  if (s.d % 16 != 0 || s.r % 8 != 0 || (s.d + s.r) % 16 != 0 || s.d + s.r > (int)SBW_ACC) return false;
   if (s.r > 0 && (a.embed.sf.b != 0 || a.embed.sf.h != 0)) return false;
   if (a.dfreqs && (a.sdf.b != 0 || a.sdf.h != 0)) return false;
   auto ok = [&](const void* ptr, const PopeStride3& st) {
