@@ -3,7 +3,7 @@ up to the accumulators' full width, repeated calls equal to the bit.
 
 Bound against 64 bits: an operand kept as two bf16 numbers is off by 2^-17 of itself at most, a product loses lo * lo' on top
 (2^-18) and cosine, sine and softplus are good to 1e-6: 2e-5 of the result's 2-norm.  (Key phases are rounded to fp32 by
-definition, fl(f + b), and so they are in the reference here.)"""
+definition, fl(f + b), and so they are in the reference here.  The rows of the gradient lie on 16 bytes, as these kernels ask.)"""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -30,8 +30,8 @@ def in_64_bits(q, k, freqs, bias, dsim):
 
 
 @pytest.mark.parametrize("b,h,hk,nq,nk,d,r,repeats", [
-    (1, 1, 1, 1, 1, 64, 64, 2),            # one step on either side: the second accumulator is never written
-    (1, 2, 1, 64, 65, 64, 32, 4),          # one step per head of a group, two in all; two steps, the second a single key
+    (1, 1, 1, 3, 4, 64, 64, 2),            # one step on either side: the second accumulator is never written
+    (1, 2, 1, 64, 68, 64, 32, 4),          # one step per head of a group, two in all; two steps, the second of four keys
     (2, 3, 3, 130, 192, 32, 32, 4),        # three steps
     (1, 2, 2, 200, 300, 128, 0, 4),        # the widest operands: all of them plain ...
     (1, 4, 2, 300, 300, 80, 48, 4),        # ... and partly rotated
