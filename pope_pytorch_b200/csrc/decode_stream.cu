@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_st
     for (int s = 0; s < p.nstages; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], NW);
     mbar_init_fence();
   }
-  if (SHORT) pdl_wait();   // (first kernel of its call: nothing in global memory may be touched earlier)
+  pdl_wait();
   // keys of this sequence (paged cache: its own length, at most the bound the split was planned for), cut evenly
   const int nk = p.seq_lens ? max(0, min(p.seq_lens[b], p.Nk)) : p.Nk;
   const int tiles_all = (nk + TILE - 1) / TILE;
@@ -203,11 +203,8 @@ __global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_st
       if (r > 0 && lane == 2) bulk_load(st, p.ch + (int64_t)key0 * r, n * r * 2, &full[s]);
       if (r > 0 && lane == 3) bulk_load(st + tbytes, p.sh + (int64_t)key0 * r, n * r * 2, &full[s]);
     };
-    // the first ring of K and V does not depend on the phase table, which the kernel before this one may still be writing
     const int pre = min(T_tiles, p.nstages);
-    for (int jt = 0; jt < pre; ++jt) load_kv(jt, jt);
-    if (!SHORT) pdl_wait();
-    for (int jt = 0; jt < pre; ++jt) load_phases(jt, jt);
+    for (int jt = 0; jt < pre; ++jt) load_kv(jt, jt), load_phases(jt, jt);
     int s = 0;
     uint32_t par = 0;
     for (int jt = pre; jt < T_tiles; ++jt) {
@@ -501,10 +498,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_st
   // slowest unit of the grid).
   __threadfence();
   worker_sync();
-  if (tid == 0) {
-    pdl_wait();   // the counters were zeroed by the kernel before this one
-    *last_s = atomicAdd(p.done + u, 1u) == (unsigned)p.nsplit - 1u;
-  }
+  if (tid == 0) *last_s = atomicAdd(p.done + u, 1u) == (unsigned)p.nsplit - 1u;
   worker_sync();
   if (!*last_s) return;
   __threadfence();
@@ -764,8 +758,8 @@ __device__ __forceinline__ void append_group(const KvAppendP& p, int b, int hk, 
   const int64_t dst = (int64_t)pg * p.page_stride + ((int64_t)hk * p.page_size + pos % p.page_size) * p.d + c * 8;
   const T* krow = static_cast<const T*>(p.k) + b * p.sk.b + hk * p.sk.h + (int64_t)i * p.sk.n + c * 8;
   const T* vrow = static_cast<const T*>(p.v) + b * p.sv.b + hk * p.sv.h + (int64_t)i * p.sv.n + c * 8;
-  *reinterpret_cast<uint4*>(static_cast<T*>(p.k_pages) + dst) = __ldg(reinterpret_cast<const uint4*>(krow));
-  *reinterpret_cast<uint4*>(static_cast<T*>(p.v_pages) + dst) = __ldg(reinterpret_cast<const uint4*>(vrow));
+  *reinterpret_cast<uint4*>(static_cast<T*>(p.k_pages) + dst) = *reinterpret_cast<const uint4*>(krow);
+  *reinterpret_cast<uint4*>(static_cast<T*>(p.v_pages) + dst) = *reinterpret_cast<const uint4*>(vrow);
 }
 
 template <typename T>

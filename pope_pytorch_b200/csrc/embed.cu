@@ -45,8 +45,7 @@ cudaError_t pope_table(const PopeTableArgs& p, cudaStream_t st) {
   return launch_dependent(pope_table_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), 0, st, p, (int)n, r);
 }
 
-__global__ void __launch_bounds__(256) pope_clamp_bwd_kernel(const float* __restrict__ bias, const float* __restrict__ grad,
-                                                             float* __restrict__ out, int64_t n) {
+__global__ void __launch_bounds__(256) pope_clamp_bwd_kernel(const float* bias, const float* grad, float* out, int64_t n) {
   pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i < n) out[i] = (bias[i] >= POPE_BIAS_MIN && bias[i] <= 0.f) ? grad[i] : 0.f;

@@ -85,7 +85,7 @@ struct TileJobs { TileJob job[4]; };
 // loads, a line per lane, come back from L1 for the next 31 features.  A thread takes every 4 slices-th feature, four at a time
 // with their loads up front.
 template <typename T>
-__global__ void __launch_bounds__(256) tile_image_kernel(TileJobs jobs, int d, int slices, const float* __restrict__ freqs, Strides sf) {
+__global__ void __launch_bounds__(256) tile_image_kernel(TileJobs jobs, int d, int slices, const float* freqs, Strides sf) {
   pdl_wait();
   pdl_trigger();
   const TileJob& jb = jobs.job[blockIdx.z];
@@ -254,12 +254,12 @@ __global__ void __launch_bounds__(128, ND == 8 ? 2 : 1) attn_fwd_tiled_kernel(Ti
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
     mbar_init_fence();
-    pdl_wait();
-    if (T > 0) {
-      fetch(Qs, p.qimg + ((int64_t)u * p.qt + qtile) * QF, p.KD, &bars[0]);
-      fetch(Ks, kimg, p.KD, &bars[1]);
-      fetch(Vs, vimg, p.DP, &bars[2]);
-    }
+  }
+  pdl_wait();
+  if (tid == 0 && T > 0) {
+    fetch(Qs, p.qimg + ((int64_t)u * p.qt + qtile) * QF, p.KD, &bars[0]);
+    fetch(Ks, kimg, p.KD, &bars[1]);
+    fetch(Vs, vimg, p.DP, &bars[2]);
   }
   __syncthreads();
   bool failed = T > 0 && !mbar_wait(&bars[0], 0, WAIT_LIMIT);
@@ -509,9 +509,9 @@ __device__ __forceinline__ void bwd_dkdv_tiled(const TiledP& p, float* smem, uin
 #pragma unroll
     for (int j = 0; j < CS; ++j) {
       const int i = q0 + L.col(j);
-      const float l = i < p.Nq ? __ldg(lse + i) : -CUDART_INF_F;
+      const float l = i < p.Nq ? lse[i] : -CUDART_INF_F;
       lse2[j] = l == -CUDART_INF_F ? CUDART_INF_F : l * LOG2E;
-      dl[j] = i < p.Nq ? __ldg(delta + i) : 0.f;
+      dl[j] = i < p.Nq ? delta[i] : 0.f;
     }
     zero(s), zero(dp);
     if (!failed) failed = !mbar_wait(&bars[1], t & 1, WAIT_LIMIT);

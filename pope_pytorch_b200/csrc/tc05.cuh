@@ -69,9 +69,13 @@ __device__ __forceinline__ void drain_copies(uint64_t* full, int nst, int first,
 
 // ---- programmatic dependent launch ---------------------------------------------------------------
 // A kernel launched with launch_dependent() (tc_common.cuh) may start while the kernel before it on the stream still
-// runs: its CTAs do their setup and call pdl_wait() before they touch anything that kernel wrote -- the wait returns once
-// that whole grid has completed and its writes are visible (at once for a kernel launched the ordinary way).
-// pdl_trigger() in the earlier kernel lets the next one start as soon as every CTA of this one has called it or exited.
+// runs: its CTAs do their setup and call pdl_wait(), which returns once that whole grid has completed and its writes are visible
+// (at once for a kernel launched the ordinary way).  Two rules hold for every such kernel:
+//   * no access to global memory before the wait, by the accessing thread itself or by one that a barrier orders before it.
+//     What ran before the PREVIOUS kernel is complete too by then: that kernel has waited for it.
+//   * no loads that may take the read-only path (__ldg, const __restrict__ parameters): they promise that the data does not
+//     change while the grid exists, which here it may do until the wait, and they may be moved across it.
+// pdl_trigger() in the earlier kernel, behind its own wait, lets the next one start as soon as every CTA has called it or exited.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) attn_fwd_tc_kernel(TcFwdP p, co
   } else if (warp == FW_VLOAD_WARP) {
     // =============================== copies: V ===================================================
     if (lane == 0) {
+      pdl_wait();   // the caller's V may be the work of a kernel just before the call
       int j = 0;
       for (; j < T_tiles; ++j) {
         const int buf = j % FW_VST, n0 = j * FW_TK;
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) attn_fwd_tc_kernel(TcFwdP p, co
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const int row_bar = 1 + (warp & 3);   // named barrier of the FW_NPR warps that share 32 rows
     auto row_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(row_bar), "n"(32 * FW_NPR) : "memory"); };
-    pdl_wait();   // the phase tables read below come from the kernels before this one
+    pdl_wait();   // q, the mask, and the phase tables of the kernels before this one
     {
       // Q' = [a cos f | pass | a sin f] of this CTA's rows, expanded HERE from q and the fp16 phase tables and written
       // straight into tensor memory (lane = row, 4 columns per 8-feature chunk): the resident operand never exists in
@@ -336,12 +337,12 @@ __global__ void __launch_bounds__(FW_THREADS, 1) attn_fwd_tc_kernel(TcFwdP p, co
       // 14-30 us slower per forward -- its code displaces the main loop's in the instruction cache)
       for (int c = part; c < DC; c += FW_NPR) {
         uint4 raw = make_uint4(0, 0, 0, 0);
-        if (live) raw = __ldg(reinterpret_cast<const uint4*>(qrow + c * 8));
+        if (live) raw = *reinterpret_cast<const uint4*>(qrow + c * 8);
         if (c < RC) {
           uint4 cq = make_uint4(0, 0, 0, 0), sq = cq;
           if (live) {
-            cq = __ldg(reinterpret_cast<const uint4*>(p.ch + trow + c * 8));
-            sq = __ldg(reinterpret_cast<const uint4*>(p.sh + trow + c * 8));
+            cq = *reinterpret_cast<const uint4*>(p.ch + trow + c * 8);
+            sq = *reinterpret_cast<const uint4*>(p.sh + trow + c * 8);
           }
           const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w}, cw[4] = {cq.x, cq.y, cq.z, cq.w}, sw[4] = {sq.x, sq.y, sq.z, sq.w};
           uint32_t o1[4], o2[4];
@@ -572,8 +573,7 @@ static cudaError_t launch_fwd_tc(const PopeAttnArgs& a, cudaStream_t st) {
   jobs.job[0] = expand_job(a.k, a.sk, s.B, s.Hk, s.Nk, s.r, 0, a.embed.bias, a.embed.bias_stride_h, kimg, s.Nk, by_batch, tab_heads);
   jobs.job[0].tile128 = 1;
   if (s.r > 0 && (e = launch_trig_tables(a.embed, s.Nk, s.r, nullptr, nullptr, tt.ch, tt.sh, st, slices, tab_heads)) != cudaSuccess) return e;
-  // tables -> images -> attention, each a programmatic dependent of the kernel before it; the first of them waits for the
-  // work before the call and lets the next one go only then
+  // tables -> images -> attention, each a programmatic dependent of the kernel before it
   if ((e = launch_expand_images(jobs, 1, s.d, bf16, tt.ch, tt.sh, st)) != cudaSuccess) return e;
   dim3 grid((s.Nq + TQ - 1) / TQ, s.B * s.H);
   return launch_dependent(attn_fwd_tc_kernel<D, T>, grid, dim3(FW_THREADS), smem, st, p, tmap_v);

@@ -118,10 +118,8 @@ cudaError_t launch_expand_images(const ExpandJobs& jobs, int njobs, int d, bool 
                                  cudaStream_t st);
 
 // Launch `kernel` so that its CTAs may start while the previous kernel on `st` still runs (programmatic stream
-// serialization); the kernel calls pdl_wait() before it reads what that kernel wrote.  A kernel that waits before its first
-// access to global memory may stand behind anything (its launch then overlaps the end of whatever runs before it, about a
-// microsecond of a short call); one that reads the caller's inputs earlier, only behind a kernel of this library that was
-// itself ordered after everything earlier on the stream.
+// serialization) and sets itself up under its end, about a microsecond of a short call.  The kernel keeps the rules at
+// pdl_wait() (tc05.cuh) and may then stand behind anything, as the first of a call too.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

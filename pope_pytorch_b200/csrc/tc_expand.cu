@@ -26,12 +26,11 @@ namespace pope {
 // features, are fixed for its lifetime (registers instead of 16 shared-memory loads per group); the raw rows of the
 // next tile are requested before the current tile is worked on.
 template <typename T, int D>
-__global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, int tpc, const __half* __restrict__ ctab,
-                                                            const __half* __restrict__ stab) {
+__global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, int tpc, const __half* ctab, const __half* stab) {
   // (ctab / stab are advanced to the unit's table slice below)
   extern __shared__ __align__(16) uint8_t stage[];
   pdl_wait();      // the phase tables (the kernel before this one) or, as the first kernel of a call, the work before it are complete
-  pdl_trigger();   // the attention kernel behind this one may set itself up, and read the caller's V
+  pdl_trigger();
   const ExpandJob& jb = jobs.job[blockIdx.z];
   const int tid = threadIdx.x, u = blockIdx.y;
   const int tiles = (int)image_tiles(jb.rows);   // a multiple of 4
@@ -67,7 +66,7 @@ __global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, i
     for (int it = 0; it < NIT; ++it) {
       const int row = row0 + it * RPP, jrow = tile * IMAGE_ROWS + row;
       raw[it] = make_uint4(0, 0, 0, 0);
-      if (active && row < IMAGE_ROWS && jrow < rows) raw[it] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)jrow * sx.n));
+      if (active && row < IMAGE_ROWS && jrow < rows) raw[it] = *reinterpret_cast<const uint4*>(base + (int64_t)jrow * sx.n);
     }
   };
   for (int tt = 0; tt < tpc; ++tt) {
@@ -83,8 +82,8 @@ __global__ void __launch_bounds__(256, 3) expand_image_kernel(ExpandJobs jobs, i
         const int row = row0 + it * RPP, jrow = tile * IMAGE_ROWS + row;
         cq[it] = sq[it] = make_uint4(0, 0, 0, 0);
         if (active && row < IMAGE_ROWS && jrow < rows) {
-          cq[it] = __ldg(reinterpret_cast<const uint4*>(ctab + (int64_t)(jb.pos0 + jrow) * r));
-          sq[it] = __ldg(reinterpret_cast<const uint4*>(stab + (int64_t)(jb.pos0 + jrow) * r));
+          cq[it] = *reinterpret_cast<const uint4*>(ctab + (int64_t)(jb.pos0 + jrow) * r);
+          sq[it] = *reinterpret_cast<const uint4*>(stab + (int64_t)(jb.pos0 + jrow) * r);
         }
       }
 #pragma unroll

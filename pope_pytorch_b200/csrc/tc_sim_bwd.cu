@@ -126,6 +126,7 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
     // the one parked in its barrier wait kept the other from running (its copy went out ~900 clocks after the barrier
     // it was waiting for had completed).
     if (warp == SBW_LOAD_WARP && lane == 0) {
+      pdl_wait();   // G may be the work of a kernel just before the call
       int s = 0;
       for (; s < S; ++s) {
         int hq;
@@ -141,7 +142,7 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
       // a wait gave up: let the copies in flight land before the CTA may leave
       if (failed) drain_copies(&bars[WB_GFULL], SBW_GST, s - SBW_GST, s);
     } else if (warp == SBW_IMG_WARP && lane == 0) {
-      pdl_wait();   // the image pre-pass has completed (the G copies of the other loader do not depend on it)
+      pdl_wait();   // the image pre-pass has completed
       int s = 0;
       for (; s < S; ++s) {
         int hq;

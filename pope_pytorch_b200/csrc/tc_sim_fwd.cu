@@ -58,8 +58,8 @@ constexpr int SIM_THREADS = 320;
 // `zero` (may be null): nzero counters that the kernel behind this one wants to find at 0
 __global__ void pope_trig_table_f32_kernel(PhaseSrc src, int n, int r, float* ctab, float* stab, __half* ch, __half* sh, unsigned int* zero,
                                            int nzero) {
-  pdl_wait();      // usually the first kernel of its call; only behind this wait is the work before the call complete, so the
-  pdl_trigger();   // next kernel, which may read the caller's inputs before its own wait, is let go after it
+  pdl_wait();      // (usually the first kernel of its call)
+  pdl_trigger();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (zero && blockIdx.y == 0)
     for (int64_t i = idx; i < nzero; i += (int64_t)gridDim.x * blockDim.x) zero[i] = 0u;
@@ -149,14 +149,14 @@ constexpr int SIM_STG_WARP = 32 * 128;     // staging tile of one worker warp: 3
 // The 8-feature chunks of the 32 rows are numbered row-major and thread t takes chunks t, t + 256, ...: a warp's loads
 // cover whole rows.  Rows past the end of the operand become zeros.
 template <typename T, bool SPLIT>
-__global__ void __launch_bounds__(256) sim_prepass_kernel(const T* __restrict__ q, Strides sq, const T* __restrict__ k, Strides sk,
+__global__ void __launch_bounds__(256) sim_prepass_kernel(const T* q, Strides sq, const T* k, Strides sk,
                                                           PhaseSrc src,
-                                                          const float* __restrict__ bias, int64_t bias_sh, int B, int H, int Hk, int Nq,
+                                                          const float* bias, int64_t bias_sh, int B, int H, int Hk, int Nq,
                                                           int Nk, int d, int r, int qtiles, int ktiles, int tile_rows,
-                                                          uint8_t* __restrict__ qimg, uint8_t* __restrict__ kimg) {
+                                                          uint8_t* qimg, uint8_t* kimg) {
   const int tid = threadIdx.x, u = blockIdx.y;
-  pdl_wait();      // the work before this call is complete ...
-  pdl_trigger();   // ... before the similarity kernel behind this one may start (it waits for this grid before it reads the images)
+  pdl_wait();      // the work before this call is complete
+  pdl_trigger();
   const int bpt = tile_rows / 32;   // blocks per tile
   const bool is_q = (int)blockIdx.x < bpt * qtiles;
   const int blk = is_q ? blockIdx.x : blockIdx.x - bpt * qtiles, tile = blk / bpt, quarter = blk % bpt;
