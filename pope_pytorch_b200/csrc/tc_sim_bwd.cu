@@ -54,7 +54,7 @@ struct TcSimBwdP {
 };
 
 enum { WB_GFULL = 0,     // [3] the G tile of step s has landed in staging buffer s % 3 (transaction bytes)
-       WB_GFREE = 3,     // [3] 8 worker warps: staging buffer s % 3 has been read
+       WB_GFREE = 3,     // [3] 8 worker warps: staging buffer s % 3 has been read, and its values used
        WB_CONV = 6,      // [2] 8 worker warps: the converted tile of step s is in buffer s & 1
        WB_IFULL = 8,     // [2] the operand tile of step s has landed in buffer s & 1 (transaction bytes)
        WB_DONE = 10,     // [2] tcgen05.commit: the chains of step s have completed: both buffers s & 1 are free
@@ -206,8 +206,10 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
       uint4 v[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const uint4*>(src + ((i ^ (grow & 7)) << 4));
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[WB_GFREE + gst]);
+      // The staging buffer is given back only behind the conversion.  A load whose value nothing has used yet may still be on its
+      // way when a barrier arrives, and the copy that refills the buffer writes through another proxy: with the arrival straight
+      // behind the loads (and no fence) one call in 600 at (1, 8, 4096, 64) had rows of dq whose last 16 bytes of a tile were
+      // those of the tile three steps on.  The later arrival costs nothing: 449 to 462 us for the whole step either way.
       // the converted buffer was last read by the chains of step s - 2
       if (s >= 2 && !failed) failed = !mbar_wait(&bars[WB_DONE + buf], ((s - 2) >> 1) & 1, WAIT_LIMIT);
       uint8_t* dst = Gbf + buf * SBW_STG + (gbox * 4) * GCS + grow * 16;
@@ -228,9 +230,9 @@ __device__ __forceinline__ void sim_bwd_side(const TcSimBwdP& p, const CUtensorM
         *reinterpret_cast<uint4*>(dst + c * GCS) = make_uint4(h[0], h[1], h[2], h[3]);
         *reinterpret_cast<uint4*>(dst + c * GCS + GPART) = make_uint4(l[0], l[1], l[2], l[3]);
       }
-      fence_async_smem();
+      fence_async_smem();   // the converted tile is visible to the tensor core, the reads of the staged one are done
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[WB_CONV + buf]);
+      if (lane == 0) mbar_arrive(&bars[WB_CONV + buf]), mbar_arrive(&bars[WB_GFREE + gst]);
     }
     // ---- epilogue -----------------------------------------------------------------------------------
     // TMEM hands every thread one ROW of the accumulator, but x, the phase table and the outputs are row-major in
