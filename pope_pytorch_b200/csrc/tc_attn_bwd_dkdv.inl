@@ -21,6 +21,26 @@ enum { KB_QFULL = 0,     // [3] Q' tile j (and its lse / delta rows) has landed 
        KB_COUNT = 20 };
 constexpr int KQ_NST = 3, KG_NST = 2;
 
+// Shared memory, from a 1 KB boundary: resident K' [d + r][128], V [d][128], KQ_NST Q' and KG_NST dO tiles, the row statistics
+// that come with the Q' tiles, the barriers.  At the end of a shared sweep (split > 1) a CTA leaves its partial sums behind K',
+// over everything but the barriers, which keep their last waiters and arrivals: they sit behind the longer of the two.
+__host__ __device__ constexpr int dkdv_dump_bytes(int d, int split) { return split > 1 ? (d / 16 - d / 16 / split) * 48 * BQ * 4 : 0; }
+__host__ __device__ constexpr int dkdv_bars_offset(int d, int kd, int split) {
+  const int tiles = BQ * d * 2 + KQ_NST * BT * kd * 2 + KG_NST * BT * d * 2 + KQ_NST * 512, dump = dkdv_dump_bytes(d, split);
+  return BQ * kd * 2 + (dump > tiles ? dump : tiles);
+}
+constexpr int dkdv_smem_bytes(int d, int kd, int split) { return dkdv_bars_offset(d, kd, split) + (KB_COUNT + 1) * 8 + 16 + 1024; }
+constexpr bool dkdv_smem_fits() {
+  for (int d = 64; d <= 128; d += 32)
+    for (int r = 0; r <= d; r += 16)
+      for (int split = 1; split <= 4; split *= 2) {
+        const int bars = dkdv_bars_offset(d, d + r, split);
+        if (bars < BQ * (d + r) * 2 + dkdv_dump_bytes(d, split) || bars % 8 != 0 || dkdv_smem_bytes(d, d + r, split) > kMaxDynamicSmem) return false;
+      }
+  return true;
+}
+static_assert(dkdv_smem_fits(), "the partial sums of a shared sweep must stay off the barriers, and all of it must fit");
+
 // SPLIT: the CTAs of a cluster (p.split of them) share a block of key rows.  (A variant of its own: as a run-time choice the tile
 // arithmetic and the second epilogue cost the unshared sweep 2 % of a training step at (4, 16, 4096, 128).)
 template <int D, typename T, bool VW, bool SPLIT>
@@ -36,7 +56,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_dkdv_tc_kernel(TcBwdP
   uint8_t* Qb = Vs + BQ * D * 2;               // 3 x [KD/8][64][16 B] streamed Q'
   uint8_t* Gb = Qb + KQ_NST * KBUF;            // 2 x [D/8][64][16 B]  streamed dO
   float* rowstat = reinterpret_cast<float*>(Gb + KG_NST * VBUF);  // 3 x (64 lse*log2e, 64 delta), with the Q' stages
-  uint64_t* bars = reinterpret_cast<uint64_t*>(rowstat + KQ_NST * 128);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + dkdv_bars_offset(D, KD, SPLIT ? p.split : 1));
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + KB_COUNT + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -709,15 +729,10 @@ static cudaError_t launch_bwd_tc(const PopeAttnBwdArgs& a, cudaStream_t st) {
                make_image_tmap(&tki, kimg, (int64_t)s.B * s.Hk * (int64_t)image_tiles(s.Nk), KD / 8);
   const size_t stage = (size_t)BT * KD * 2 + (size_t)BT * D * 2;
   size_t smem_q = (size_t)BQ * KD * 2 + DQ_NST * stage + (BB_COUNT + 1) * 8 + 16 + 1024;
-  size_t smem_k = (size_t)BQ * KD * 2 + BQ * D * 2 + KQ_NST * (size_t)BT * KD * 2 + KG_NST * (size_t)BT * D * 2 + KQ_NST * 512 +
-                  (KB_COUNT + 1) * 8 + 16 + 1024;   // 232.2 KB at d = r = 128 (1 KB of it to put the base on a 1 KB boundary)
+  size_t smem_k = dkdv_smem_bytes(D, KD, p.split);   // 232.2 KB at d = r = 128 (1 KB of it to put the base on a 1 KB boundary)
   // every CTA allocates all 512 TMEM columns: keep two CTAs from sharing an SM
   if (smem_q < 120 * 1024) smem_q = 120 * 1024;
   if (smem_k < 120 * 1024) smem_k = 120 * 1024;
-  if (p.split > 1) {   // the chunks a CTA leaves to the others, behind K'; at most 64 + 144 + 1 KB
-    const size_t chunks = (size_t)D / 16, dump = (chunks - chunks / p.split) * 48 * BQ * 4;
-    smem_k = std::max(smem_k, (size_t)BQ * KD * 2 + dump + 1024);
-  }
   if (fork) {   // images -> side stream (dk/dv); row statistics -> caller's stream (dq reads delta)
     if ((e = cudaEventRecord(fk->ready, st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(fk->side, fk->ready, 0)) != cudaSuccess) return e;
