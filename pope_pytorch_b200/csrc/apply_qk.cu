@@ -196,7 +196,8 @@ __global__ void __launch_bounds__(AP_THREADS, 4) apply_qk_kernel(ApplyP p, int r
     }
     const int h2 = b + 1 == p.B ? h + 1 : h, b2 = b + 1 == p.B ? 0 : b + 1;
     fresh = (h2 != h && (s.bias || p.sf.h != 0)) || (b2 != b && p.sf.b != 0);
-    if (BACKWARD && (fresh || u + 1 == u1)) flush_freqs();
+    // (a table that is broadcast by a stride of 0 has a gradient with a slice for every unit: its own strides decide)
+    if (BACKWARD && ((h2 != h && p.sdf.h != 0) || (b2 != b && p.sdf.b != 0) || u + 1 == u1)) flush_freqs();
     if (BACKWARD && (h2 != h || u + 1 == u1)) flush_bias();
     h = h2, b = b2;
   }
