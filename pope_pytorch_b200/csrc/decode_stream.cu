@@ -400,6 +400,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_st
           for (int e = 0; e < 4; ++e) o[g][e] = fma2(make_float2(pk[g], pk[g]), vv[e], o[g][e]);
       }
     }
+    fence_async_smem();   // the tile has been read: the loader's next copy may write over it
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
     if (++s == p.nstages) s = 0, par ^= 1;

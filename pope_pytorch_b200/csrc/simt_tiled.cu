@@ -224,7 +224,10 @@ __device__ __forceinline__ void split_sync(int split) {
   else __syncwarp(), cluster_sync();
 }
 
-// one image tile by bulk copy; a thread of the CTA calls it after every thread is done with the buffer
+// every thread is done with a buffer that a copy is about to refill
+__device__ __forceinline__ void release_sync() { fence_async_smem(), __syncthreads(); }
+
+// one image tile by bulk copy; a thread of the CTA calls it behind release_sync()
 __device__ __forceinline__ void fetch(float* dst, const float* img, int feats, uint64_t* bar) {
   mbar_expect_tx(bar, feats * ST_ROWS * 4);
   bulk_load(dst, img, feats * ST_ROWS * 4, bar);
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(128, ND == 8 ? 2 : 1) attn_fwd_tiled_kernel(Ti
     }
     if (!failed) failed = !mbar_wait(&bars[1], t & 1, WAIT_LIMIT);
     mm_features<TX>(s, Qs, Ks, p.KD, L);
-    __syncthreads();   // the K' tile and (from the last round) P have been read
+    release_sync();   // the K' tile and (from the last round) P have been read
     if (tid == 0 && t + 1 < T) fetch(Ks, kimg + (int64_t)(t + 1) * QF, p.KD, &bars[1]);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -307,7 +310,7 @@ __global__ void __launch_bounds__(128, ND == 8 ? 2 : 1) attn_fwd_tiled_kernel(Ti
     if (!failed) failed = !mbar_wait(&bars[2], t & 1, WAIT_LIMIT);
     mm_rows<TX, ND>(o, Ps, Vs, L);
     if (t + 1 < T) {
-      __syncthreads();   // the V tile has been read
+      release_sync();   // the V tile has been read
       if (tid == 0) fetch(Vs, vimg + (int64_t)(t + 1) * p.DP * ST_ROWS, p.DP, &bars[2]);
     }
   }
@@ -454,10 +457,10 @@ __device__ __forceinline__ void bwd_dq_tiled(const TiledP& p, float* smem, uint6
         s[i][j] = vis ? exp2f(s[i][j] * p.scale_log2 - lse2[i]) * (dp[i][j] - dl[i]) * p.scale : 0.f;
       }
     put_scores<TX>(Ss, s, L);
-    __syncthreads();   // dS is written, the V tile has been read
+    release_sync();   // dS is written, the V tile has been read
     if (tid == 0 && t + 1 < T) fetch(Vs, vimg + (int64_t)(t + 1) * VF, p.DP, &bars[2]);
     mm_rows<TX, NK>(acc, Ss, Ks, L);
-    __syncthreads();   // the K' tile and dS have been read
+    release_sync();   // the K' tile and dS have been read
     if (tid == 0 && t + 1 < T) fetch(Ks, kimg + (int64_t)(t + 1) * QF, p.KD, &bars[1]);
   }
   const int astr = p.d + p.r + 1;
@@ -529,12 +532,12 @@ __device__ __forceinline__ void bwd_dkdv_tiled(const TiledP& p, float* smem, uin
     put_scores<TX>(Ss, s, L);
     __syncthreads();
     mm_rows<TX, ND>(av, Ss, Gs, L);
-    __syncthreads();   // P^T and the dO tile have been read
+    release_sync();   // P^T and the dO tile have been read
     if (tid == 0 && t + 1 < T) fetch_g(t + 1);
     put_scores<TX>(Ss, dp, L);
     __syncthreads();
     mm_rows<TX, NK>(ak, Ss, Qs, L);
-    __syncthreads();   // dS^T and the Q' tile have been read
+    release_sync();   // dS^T and the Q' tile have been read
     if (tid == 0 && t + 1 < T) fetch_q(t + 1);
   }
   const int astr = p.d + p.r + 1;

@@ -141,7 +141,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int bytes) {
 }
 
 // ---- fences ----------------------------------------------------------------------------------
-// generic-proxy shared-memory writes -> visible to the async proxy (tensor core / TMA reads)
+// Between generic and asynchronous accesses to shared memory, in front of the barrier that orders them: generic writes are
+// visible to the tensor core and the copy engine, and generic reads are done before a copy refills what they read.
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
