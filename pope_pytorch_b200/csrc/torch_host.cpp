@@ -340,6 +340,11 @@ std::tuple<Tensor, Tensor> apply_qk(const Tensor& q, const Tensor& k, const Tens
 }
 
 // ---- the embedding tables ------------------------------------------------------------------------------------------
+// a tensor whose memory a kernel may be given: fp32, contiguous, of no function transform or dispatch mode, without a tangent
+bool plain(const Tensor& t) {
+  return !at::isTensorSubclassLike(t) && t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && !t._fw_grad(0).defined();
+}
+
 // (freqs, clamped bias, positions, flat inverse frequencies, axis of a feature) of a sequence or a grid; a sequence has no
 // last two.  bias may carry a gradient, the frequencies do not (the Python modules see to that).
 struct Table : torch::autograd::Function<Table> {
@@ -373,7 +378,13 @@ struct Table : torch::autograd::Function<Table> {
   }
   static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad) {
     if (!grad[1].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
-    const Tensor bias = ctx->get_saved_variables()[0], g = grad[1].contiguous();
+    const Tensor bias = ctx->get_saved_variables()[0];
+    // a gradient that is differentiated itself (create_graph), or a batch of them: the clamp's gradient as PyTorch operations
+    if (at::GradMode::is_enabled() || at::isTensorSubclassLike(grad[1])) {
+      const Tensor passes = bias.ge(POPE_BIAS_MIN).logical_and_(bias.le(0.f));
+      return {at::where(passes, grad[1], at::zeros({}, bias.options())), Tensor(), Tensor(), Tensor()};
+    }
+    const Tensor g = grad[1].contiguous();
     c10::cuda::OptionalCUDAGuard guard(bias.device());
     Tensor out = at::empty_like(bias);
     PopeClampBwdArgs a = {};
@@ -387,9 +398,6 @@ struct Table : torch::autograd::Function<Table> {
 // None when the module's tensors are not what the kernel takes (another type or device, frequencies that train, tensors of a
 // function transform or of a dispatch mode, forward mode): the module's own PyTorch operations serve those
 optional<std::vector<Tensor>> table(const Tensor& bias, const std::vector<Tensor>& inv, const std::vector<int64_t>& dims, double offset) {
-  auto plain = [](const Tensor& t) {
-    return !at::isTensorSubclassLike(t) && t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && !t._fw_grad(0).defined();
-  };
   if (inv.empty() || inv.size() != dims.size() || inv.size() > POPE_MAX_AXES || bias.dim() != 2 || !plain(bias)) return std::nullopt;
   int64_t n = 1, r = 0;
   for (const int64_t d : dims) {
