@@ -115,6 +115,9 @@ class PagedKVCache:
             self._held = held = (*tensors, N._ops().Pages(*tensors))
         return held[4]
 
+    def __getstate__(self):
+        return {**self.__dict__, "_held": None}   # (the binding's object is made again; copies have tensors of their own)
+
     def _push_table(self, new_entries) -> None:
         if new_entries:
             width = self.alloc.max_pages_per_seq
