@@ -118,15 +118,22 @@ class PagedKVCache:
     def __getstate__(self):
         return {**self.__dict__, "_held": None}   # (the binding's object is made again; copies have tensors of their own)
 
+    def _row(self, b: int) -> int:
+        """Sequence ``b``, counted from the end when negative, as an index of the tables."""
+        if not -self.batch <= b < self.batch:
+            raise IndexError(f"sequence {b} is not in the cache")
+        return b % self.batch
+
     def _push_table(self, new_entries) -> None:
-        if new_entries:
+        if new_entries:      # (entries >= 0; a negative index would be a length)
             width = self.alloc.max_pages_per_seq
             N._ops().kv_map(self._pages(), [b * width + lp for b, lp, _ in new_entries], [pg for _, _, pg in new_entries])
 
     def release(self, b: int) -> None:
         """Forget sequence ``b`` and free its pages."""
+        b = self._row(b)
         self.alloc.release(b)
-        N._ops().kv_map(self._pages(), [-1 - (b % self.batch)], [0])
+        N._ops().kv_map(self._pages(), [-1 - b], [0])
 
     # ---- the two operators -------------------------------------------------------------------------
     def append(self, k: torch.Tensor, v: torch.Tensor) -> None:
@@ -144,6 +151,7 @@ class PagedKVCache:
 
     def append_to(self, b: int, k: torch.Tensor, v: torch.Tensor) -> None:
         """k, v: (kv_heads, n_new, head_dim) appended to sequence ``b`` only (ragged prompts)."""
+        b = self._row(b)
         if k.shape != v.shape or k.ndim != 3 or k.shape[0] != self.kv_heads or k.shape[2] != self.head_dim:
             raise ValueError("k and v must be (kv_heads, n_new, head_dim)")
         if k.dtype != self.dtype or v.dtype != self.dtype or k.device != self.device or v.device != self.device:

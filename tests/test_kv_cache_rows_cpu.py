@@ -1,4 +1,5 @@
-"""The paged cache as a Python object (no GPU; a recorder stands where the binding is called): copies of a cache in use."""
+"""The paged cache as a Python object (no GPU; a recorder stands where the binding is called): copies of a cache in use, and rows
+counted from the end or out of range."""
 import copy
 import pickle
 
@@ -49,3 +50,20 @@ def test_a_cache_in_use_can_be_copied(ops, again):
     twin.append_to(0, rows(1), rows(1))
     assert twin._pages()()[0] is twin.k_pages and cache._pages()()[0] is cache.k_pages
     assert twin.lens == [1, 70, 0] and cache.lens == [0, 70, 0]
+
+
+def test_negative_rows_count_from_the_end(ops):
+    cache = make()
+    cache.append_to(-1, rows(70), rows(70))
+    assert cache.lens == [0, 0, 70] and ops.maps == [([2 * 4, 2 * 4 + 1], [0, 1])] and ops.appends == [2]
+    cache.release(-1)
+    assert cache.lens == [0, 0, 0] and ops.maps[1] == ([-3], [0])
+
+
+@pytest.mark.parametrize("b", [3, -4])
+def test_rows_outside_the_cache_change_nothing(ops, b):
+    cache = make()
+    for call in (lambda: cache.append_to(b, rows(70), rows(70)), lambda: cache.release(b)):
+        with pytest.raises(IndexError):
+            call()
+    assert cache.lens == [0, 0, 0] and len(cache.alloc.free) == 8 and ops.maps == [] and ops.appends == []
