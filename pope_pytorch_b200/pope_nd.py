@@ -44,7 +44,8 @@ class AxialPoPE(nn.Module):
         return coords.flip(-1)
 
     def forward(self, pos_or_dims: Union[Tensor, Tuple[int, ...]]) -> PolarEmbedReturn:
-        if self.bias.is_cuda and isinstance(pos_or_dims, tuple) and len(pos_or_dims) == len(self.axial_dims) > 1 and not _traced():
+        if self.bias.is_cuda and isinstance(pos_or_dims, tuple) and len(pos_or_dims) == len(self.axial_dims) > 1 and not _traced() \
+                and all(isinstance(n, int) for n in pos_or_dims):      # (torch.arange takes other numbers too)
             from . import _native          # one launch instead of a chain of elementwise kernels
             made = _native.embed_table(self.bias, list(self.inv_freqs), list(pos_or_dims))
             if made is not None:
