@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(128, ND == 8 ? 2 : 1) attn_fwd_tiled_kernel(Ti
 
 // ---- backward ----------------------------------------------------------------------------------------------------------
 // Epilogue: X' gradients of rows [r0, r1) of a tile, staged as [64][astr] by every CTA that shares it -> dx, dphase.  Everything the chain rule needs is in the resident
-// image tile: with xc = a cos, xs = a sin,  a = sqrt(xc^2 + xs^2),  sigmoid(x) = 1 - exp(-a),
+// image tile: with xc = a cos, xs = a sin,  a = hypot(xc, xs),  sigmoid(x) = 1 - exp(-a),
 //   dx = (gc xc + gs xs) / a * sigmoid(x),  dphase = gs xc - gc xs.
 __device__ __forceinline__ void chain_rule(const TiledP& p, const float* acc, int astr, const float* X, int row0, int rows, void* dx, int64_t base,
                                            int64_t sn, float* df, int64_t sfn, int pos0, float* dbias, int rank) {
@@ -384,7 +384,7 @@ __device__ __forceinline__ void chain_rule(const TiledP& p, const float* acc, in
         const float gs = over_split(acc + row * astr + p.d + c, p.split);
         const float xc = X[c * ST_ROWS + (((grp ^ (c >> 2)) & 15) << 2) + e];
         const float xs = X[(p.d + c) * ST_ROWS + (((grp ^ ((p.d + c) >> 2)) & 15) << 2) + e];
-        const float a = sqrtf(xc * xc + xs * xs), dph = gs * xc - g * xs;
+        const float a = hypotf(xc, xs), dph = gs * xc - g * xs;   // (the squares leave the range of fp32 below x = -44 and above 1e19)
         g = a > 0.f ? (g * xc + gs * xs) / a * -expm1f(-a) : 0.f;
         sum += dph;
         if (df) atomicAdd(df + (int64_t)(pos0 + row0 + row) * sfn + c, dph);
