@@ -324,12 +324,8 @@ def _mask_u8(mask: Optional[torch.Tensor]):
 # ----------------------------------------------------------------------------------------------
 
 def apply_qk_supported(q, k, freqs, bias) -> bool:
-    """CUDA 4-D head-first q / k of one supported dtype, fp32 table, even expanded width."""
-    if not (q.is_cuda and k.is_cuda and freqs.is_cuda and bias.is_cuda and q.ndim == 4 and k.ndim == 4):
-        return False
-    d, r = q.shape[-1], freqs.shape[-1]
-    return (q.dtype in _DTYPES and k.dtype == q.dtype and d <= 256 and (d + r) % 2 == 0 and q.shape[1] % k.shape[1] == 0
-            and freqs.ndim in (2, 3, 4) and bias.ndim == 2 and is_available())
+    """Whether the fused transform takes the call (CUDA tensors that fit together, see ``apply_qk_takes`` in torch_host.cpp)."""
+    return q.is_cuda and (_host is not None or is_available()) and _host.apply_qk_takes(q, k, freqs, bias)
 
 
 class _Recorded(torch.autograd.Function):

@@ -99,8 +99,24 @@ Tensor workspace(int op, Args& a, const Tensor& like) {
 
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
+// The library sees pointers only: what a kernel reads has to be on q's device and reach as far as the kernel reads.  (Tensors
+// that reach further are read in part.)
+void same_device(const Tensor& t, const Tensor& q, const char* what) {
+  TORCH_CHECK(t.device() == q.device(), what, " is on ", t.device(), ", q on ", q.device());
+}
+
+void validate_embed(const Tensor& q, int64_t batch, int64_t heads, int64_t key_heads, const Tensor& freqs, const Tensor& bias) {
+  const int64_t r = freqs.size(-1);
+  if (r == 0) return;   // (nothing of either is read)
+  same_device(freqs, q, "freqs"), same_device(bias, q, "bias");
+  if (freqs.dim() >= 3) TORCH_CHECK_VALUE(freqs.size(0) == 1 || freqs.size(0) >= batch, "freqs must have one table, or one per batch entry");
+  if (freqs.dim() == 4) TORCH_CHECK_VALUE(freqs.size(1) == 1 || freqs.size(1) >= heads, "freqs must have one table, or one per head");
+  TORCH_CHECK_VALUE(bias.dim() >= 1 && bias.size(-1) >= r && bias.numel() > 0 && (key_heads == 1 || (bias.dim() == 2 && bias.size(0) >= key_heads)),
+                    "bias must have one row of rotated features per key head");
+}
+
 // the checks every operator makes on q, k and the pair (freqs, bias); GIL held
-void validate(const Tensor& q, const Tensor& k, const Tensor& freqs, bool seq_first) {
+void validate(const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias, bool seq_first) {
   if (!(q.is_cuda() && k.is_cuda())) TORCH_CHECK(false, "the native PoPE kernels need CUDA tensors");
   if (dtype_of(q) < 0 || k.scalar_type() != q.scalar_type())
     TORCH_CHECK_TYPE(false, "q and k must share a dtype among fp32/bf16/fp16, got ", q.scalar_type(), ", ", k.scalar_type());
@@ -109,6 +125,28 @@ void validate(const Tensor& q, const Tensor& k, const Tensor& freqs, bool seq_fi
   if (q.size(ha) % k.size(ha) != 0) assertion("query heads must be a multiple of key heads");
   if (q.size(na) > k.size(na) || freqs.size(-1) > q.size(-1)) assertion("queries must not outnumber keys, nor rotated features the head dim");
   if (freqs.dim() < 2 || (freqs.size(-2) != k.size(na) && freqs.size(-1) != 0)) assertion("freqs must have one row per key position");
+  same_device(k, q, "k");
+  TORCH_CHECK_VALUE(k.size(0) >= q.size(0) && k.size(3) >= q.size(3), "q and k must have the same batch size and head dim");
+  validate_embed(q, q.size(0), q.size(ha), k.size(ha), freqs, bias);
+}
+
+// ... and the attention on v and the mask
+void validate_attn(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask,
+                   bool seq_first) {
+  validate(q, k, freqs, bias, seq_first);
+  same_device(v, q, "v");
+  if (v.scalar_type() != q.scalar_type()) TORCH_CHECK_TYPE(false, "v must have the dtype of q and k, got ", v.scalar_type(), ", ", q.scalar_type());
+  const int ha = seq_first ? 2 : 1, na = seq_first ? 1 : 2;
+  TORCH_CHECK_VALUE(v.dim() == 4 && v.size(0) >= q.size(0) && v.size(ha) >= k.size(ha) && v.size(na) >= k.size(na) && v.size(3) >= q.size(3),
+                    "v must have the shape of k");
+  if (!mask || !mask->defined()) return;
+  same_device(*mask, q, "mask");
+  TORCH_CHECK_VALUE(mask->dim() == 2 && mask->size(0) >= q.size(0) && mask->size(1) >= k.size(na), "mask must be (batch, keys)");
+}
+
+// The buffer of the gradient of t = k or v.  The kernels write as far as they read: of a tensor that reaches further the rest is zero.
+Tensor grad_of_keys(const Tensor& t, const Tensor& k, const Tensor& q) {
+  return t.sizes() == k.sizes() && k.size(0) == q.size(0) && k.size(3) == q.size(3) ? at::empty_like(t) : at::zeros_like(t);
 }
 
 // ---- attention -------------------------------------------------------------------------------------------------
@@ -165,7 +203,7 @@ Grads attn_backward(const Tensor& dout_, const Tensor& q_, const Tensor& k_, con
   const Tensor q = inner_contig(q_), k = inner_contig(k_), v = inner_contig(v_), out = inner_contig(out_), dout = inner_contig(dout_);
   const Tensor freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
   const int r = (int)freqs.size(-1);
-  Grads g{at::empty_like(q), at::empty_like(k), at::empty_like(v), Tensor(), Tensor()};
+  Grads g{at::empty_like(q), grad_of_keys(k, k, q), grad_of_keys(v, k, q), Tensor(), Tensor()};
   const Mask m(mask);
   PopeAttnBwdArgs a = {};
   a.struct_bytes = sizeof(a), a.causal = causal, a.softmax_scale = (float)scale;
@@ -218,7 +256,7 @@ bool wants_graph(const Ts&... ts) {
 
 Tensor flash_attn(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask,
                   bool causal, double scale, const Factors& factors, bool seq_first) {
-  validate(q, k, freqs, seq_first);
+  validate_attn(q, k, v, freqs, bias, mask, seq_first);
   py::gil_scoped_release nogil;
   if (!wants_graph(q, k, v, freqs, bias)) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -249,7 +287,7 @@ Grads sim_backward(const Tensor& dsim_, const Tensor& q_, const Tensor& k_, cons
   c10::cuda::OptionalCUDAGuard guard(q_.device());
   const Tensor q = inner_contig(q_), k = inner_contig(k_), dsim = inner_contig(dsim_), freqs = fp32_rows(freqs_), bias = fp32_rows(bias_);
   const int r = (int)freqs.size(-1);
-  Grads g{at::empty_like(q), at::empty_like(k), Tensor(), Tensor(), Tensor()};
+  Grads g{at::empty_like(q), grad_of_keys(k, k, q), Tensor(), Tensor(), Tensor()};
   PopeSimBwdArgs a = {};
   a.struct_bytes = sizeof(a), a.allow_tf32 = allow_tf32;
   a.shape = shape_of(q, k, r, sf), a.embed = embed_of(freqs, bias, r);
@@ -278,7 +316,7 @@ struct Similarity : torch::autograd::Function<Similarity> {
 
 Tensor similarity(const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias, bool allow_tf32, const Factors& factors,
                   bool seq_first) {
-  validate(q, k, freqs, seq_first);
+  validate(q, k, freqs, bias, seq_first);
   py::gil_scoped_release nogil;
   if (!wants_graph(q, k, freqs, bias)) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -327,6 +365,17 @@ struct ApplyQK : torch::autograd::Function<ApplyQK> {
     return {g.dq, g.dk, to_dtype_of(g.dfreqs, s[2]), to_dtype_of(g.dbias, s[3])};
   }
 };
+
+// Whether the kernel takes the call: one supported dtype, batch size, head dim and device, a table and a bias that reach as far, an
+// even expanded width.  (The PyTorch operations take the rest, or say what is wrong with it.)
+bool apply_qk_takes(const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias) {
+  if (!q.is_cuda() || q.dim() != 4 || k.dim() != 4 || freqs.dim() < 2 || freqs.dim() > 4 || bias.dim() != 2) return false;
+  if (k.device() != q.device() || freqs.device() != q.device() || bias.device() != q.device()) return false;
+  if (dtype_of(q) < 0 || k.scalar_type() != q.scalar_type()) return false;
+  const int64_t b = q.size(0), h = q.size(1), hk = k.size(1), d = q.size(3), r = freqs.size(-1);
+  return hk > 0 && h % hk == 0 && k.size(0) == b && k.size(3) == d && d <= 256 && (d + r) % 2 == 0 && bias.size(0) >= hk && bias.size(1) >= r &&
+         (freqs.dim() == 2 || freqs.size(0) == 1 || freqs.size(0) >= b) && (freqs.dim() < 4 || freqs.size(1) == 1 || freqs.size(1) >= h);
+}
 
 std::tuple<Tensor, Tensor> apply_qk(const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias) {
   if (freqs.size(-1) != 0 && freqs.size(-2) != k.size(2)) assertion("freqs must have one row per key position");
@@ -454,6 +503,7 @@ void kv_append(const Pages& p, const Tensor& k_, const Tensor& v_, int64_t row) 
 }
 
 std::tuple<Tensor, Tensor> kv_decode(const Pages& p, const Tensor& q_, const Tensor& freqs_, const Tensor& bias_, double scale, int64_t nk) {
+  validate_embed(q_, q_.size(0), q_.size(1), p.k.size(1), freqs_, bias_);
   py::gil_scoped_release nogil;
   c10::cuda::OptionalCUDAGuard guard(p.k.device());
   at::NoGradGuard off;
@@ -476,6 +526,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flash_attn", &flash_attn);
   m.def("similarity", &similarity);
   m.def("apply_qk", &apply_qk);
+  m.def("apply_qk_takes", &apply_qk_takes);
   m.def("table", &table);
   py::class_<Pages>(m, "Pages").def(py::init([](Tensor k, Tensor v, Tensor table, Tensor lens) { return Pages{k, v, table, lens}; }));
   m.def("kv_map", &kv_map);
@@ -483,24 +534,35 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("kv_decode", &kv_decode);
   m.def("attn_forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask,
                            bool causal, double scale, const Factors& factors) {
-    validate(q, k, freqs, false);
+    validate_attn(q, k, v, freqs, bias, mask, false);
     at::NoGradGuard off;
     return attn_forward(q, k, v, freqs, bias, mask, causal, scale, factors, false);
   });
   m.def("attn_backward", [](const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
                             const Tensor& freqs, const Tensor& bias, const optional<Tensor>& mask, bool causal, double scale, bool need_df,
                             bool need_db, const Factors& factors) {
+    validate_attn(q, k, v, freqs, bias, mask, false);
+    same_device(out, q, "out"), same_device(dout, q, "dout"), same_device(lse, q, "lse");
+    TORCH_CHECK_VALUE(out.sizes() == q.sizes() && dout.sizes() == q.sizes() && lse.sizes() == q.sizes().slice(0, 3) && lse.is_contiguous(),
+                      "out and dout must have the shape of q, lse its rows");
+    if (out.scalar_type() != q.scalar_type() || dout.scalar_type() != q.scalar_type() || lse.scalar_type() != at::kFloat)
+      TORCH_CHECK_TYPE(false, "out and dout must have the dtype of q, lse fp32");
     at::NoGradGuard off;
     Grads g = attn_backward(dout, q, k, v, out, lse, freqs, bias, mask, causal, scale, need_df, need_db, factors, false);
     return std::make_tuple(g.dq, g.dk, g.dv, need_df ? optional<Tensor>(g.dfreqs) : std::nullopt, need_db ? optional<Tensor>(g.dbias) : std::nullopt);
   });
   m.def("sim_forward", [](const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias, bool allow_tf32, const Factors& factors) {
-    validate(q, k, freqs, false);
+    validate(q, k, freqs, bias, false);
     at::NoGradGuard off;
     return sim_forward(q, k, freqs, bias, allow_tf32, factors, false);
   });
   m.def("sim_backward", [](const Tensor& dsim, const Tensor& q, const Tensor& k, const Tensor& freqs, const Tensor& bias, bool need_df, bool need_db,
                            bool allow_tf32) {
+    validate(q, k, freqs, bias, false);
+    same_device(dsim, q, "dsim");
+    TORCH_CHECK_VALUE(dsim.dim() == 4 && dsim.size(0) >= q.size(0) && dsim.size(1) >= q.size(1) && dsim.size(2) >= q.size(2) && dsim.size(3) >= k.size(2),
+                      "dsim must have the shape of the similarity");
+    if (dsim.scalar_type() != q.scalar_type()) TORCH_CHECK_TYPE(false, "dsim must have the dtype of q");
     at::NoGradGuard off;
     Grads g = sim_backward(dsim, q, k, freqs, bias, need_df, need_db, allow_tf32, false);
     return std::make_tuple(g.dq, g.dk, need_df ? optional<Tensor>(g.dfreqs) : std::nullopt, need_db ? optional<Tensor>(g.dbias) : std::nullopt);
