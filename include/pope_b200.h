@@ -274,7 +274,7 @@ typedef struct PopeKvMapArgs {
  * table; freqs must have at least that many rows and no batch / head axes).  A sequence without keys
  * gives out = 0, lse = -inf.  lse (B, H) fp32 may be NULL.  Workspace: pope_b200_workspace_bytes(
  * POPE_OP_DECODE_PAGED, &args).  Kernel: the streaming decode kernel (copy-engine ring of 64-key tiles,
- * key ranges split over CTAs, split combine), tile addresses taken from the page table. */
+ * key ranges split over CTAs, partial results merged inside the kernel), tile addresses taken from the page table. */
 typedef struct PopePagedDecodeArgs {
   uint32_t struct_bytes;
   float softmax_scale;
@@ -325,8 +325,9 @@ typedef struct PopeClampBwdArgs {
 POPE_API int pope_b200_abi_version(void);
 POPE_API const char* pope_b200_status_str(int status);
 
-/* Name of the kernel family the last successful call ON THIS THREAD dispatched to
- * ("simt", "tcgen05", ...).  Diagnostic only. */
+/* Name of the kernel family the last successful call ON THIS THREAD dispatched to: "tcgen05" (tensor
+ * cores), "decode_stream" / "decode_stream_paged" (one 16-bit query row, streamed keys), "kv_append", "simt"
+ * (the exact-arithmetic kernels).  Diagnostic only. */
 POPE_API const char* pope_b200_last_path(void);
 
 /* Sticky device-side status of the tensor-core kernels on the current device: 0 = healthy,

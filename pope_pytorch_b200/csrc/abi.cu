@@ -169,7 +169,7 @@ int pope_b200_attn_fwd(const PopeAttnArgs* a, void* stream) {
                         : tiled ? pope::attn_fwd_tiled(*a, st)
                                 : pope::attn_fwd_simt(*a, st);
   if (e != cudaSuccess) return POPE_ERR_CUDA;
-  g_last_path = tc ? "tcgen05" : dec && !pope::decode_is_exact(*a) ? "decode_stream" : "simt";
+  g_last_path = tc ? "tcgen05" : dec ? "decode_stream" : "simt";
   return POPE_OK;
 }
 

@@ -97,7 +97,7 @@ template <typename T, int N2> __device__ __forceinline__ void unpack_words(const
   for (int e = 0; e < N2; ++e) x[e] = unpack2<T>(u[e]);
 }
 
-constexpr int DS_EXACT_KEYS = 1024;   // shorter contiguous key ranges keep fp32 phases
+constexpr int DS_FP32_KEYS = 1024;   // shorter contiguous key ranges keep fp32 phases
 constexpr int DS_TILE = 64;       // keys per tile
 constexpr int DS_MAX_SPLIT = 64;  // key ranges per unit
 
@@ -227,8 +227,17 @@ __global__ void __launch_bounds__(32 * (NW + 1), NW == 8 ? 2 : 1) attn_decode_st
     const float x = to_f32<T>(qrow[c]);
     float qc = x, qs = 0.f;
     if (c < r) {
-      float sn, cs;
-      sincosf(p.freqs[(int64_t)(max(nk, 1) - 1) * p.sfn + c] - p.bias[hk * p.bias_sh + c], &sn, &cs);
+      // Cosine and sine of position phase minus bias, each angle by itself: rounded to fp32 the difference would be off by up to
+      // 2^-15 rad at a few hundred rad, for every key alike.  (A loop, not two calls in a row: half the code to fetch.)
+      const float f = p.freqs[(int64_t)(max(nk, 1) - 1) * p.sfn + c], b_ = p.bias[hk * p.bias_sh + c];
+      float cs = 1.f, sn = 0.f;
+#pragma unroll 1
+      for (int i = 0; i < 2; ++i) {
+        float s1, c1;
+        sincosf(i == 0 ? f : -b_, &s1, &c1);
+        const float t = cs * c1 - sn * s1;
+        sn = fmaf(sn, c1, cs * s1), cs = t;
+      }
       const float a = softplus_f(x) * LN2;   // (the keys' magnitudes come in units of ln 2)
       qc = a * cs, qs = a * sn;
     }
@@ -564,15 +573,17 @@ static int decode_stream_split(const PopeShape& s, bool shrt) {
 // The SHORT flavour saves a launch and the trip of the partials through L2, about 2 us, and pays for its own cosines and sines
 // with every tile of a CTA, the less the more heads share them: (2, 16, 4000, 128) with 8 tiles per CTA takes 21.6 us
 // against 18.9, (4, 32 / 8, 2000, 128) with 8 tiles of four heads 19.9 against 20.7, (2, 16 / 4, 777, 128) 10.0 against 11.8.
-// It copies rows of the phase table, which therefore has to be contiguous.  Below DS_EXACT_KEYS keys every call takes it: those
-// calls are promised fp32 phases (they belong to the exact-arithmetic family; a call without a usable table goes to its
-// other kernels).
+// It copies rows of the phase table, which therefore has to be contiguous.  Below DS_FP32_KEYS keys every call takes it, with
+// fp32 phases but approximate functions (ex2, lg2, sine and cosine of the special-function unit, 2^-21 absolute and better); a
+// call without a usable table goes to the exact family, which took them all before.  Against 64 bits both are off by the rounding
+// of the output, 2.066e-4 in fp16 at (2, 16 / 4, 777, 128); the nearest fp16 value is missed in 0.05 % of the outputs here and
+// in 1.1 % there.  (Accurate softplus, sine and cosine of the keys changed neither figure and took 11.5 instead of 10.3 us.)
 static bool decode_short_possible(const PopeShape& s, const PopeEmbed& e) {
   return s.r == 0 || (e.sf.n == s.r && (reinterpret_cast<uintptr_t>(e.freqs) & 15) == 0);
 }
 static bool decode_short(const PopeShape& s, const PopeEmbed& e) {
   if (!decode_short_possible(s, e)) return false;
-  if (s.Nk < DS_EXACT_KEYS) return true;
+  if (s.Nk < DS_FP32_KEYS) return true;
   const int tiles = (s.Nk + DS_TILE - 1) / DS_TILE, n = decode_stream_split(s, true), g = decode_heads(s);
   const int64_t ctas = (int64_t)s.B * s.H / g * n, slots = decode_slots(s);
   return (ctas + slots - 1) / slots * ((tiles + n - 1) / n) <= 4 + g;
@@ -581,7 +592,7 @@ static bool decode_short(const PopeShape& s, const PopeEmbed& e) {
 bool decode_stream_supported(const PopeAttnArgs& a) {
   const PopeShape& s = a.shape;
   if (s.Nq != 1 || a.causal) return false;
-  if (s.Nk < DS_EXACT_KEYS && !decode_short_possible(s, a.embed)) return false;
+  if (s.Nk < DS_FP32_KEYS && !decode_short_possible(s, a.embed)) return false;
   if (s.dtype != POPE_BF16 && s.dtype != POPE_F16) return false;
   if (s.d != 64 && s.d != 96 && s.d != 128) return false;
   if (s.r % 8 != 0) return false;
@@ -691,8 +702,6 @@ template <typename T>
 static cudaError_t decode_stream_d(const PopeAttnArgs& a, cudaStream_t st, const PopePagedKV* kv) {
   return decode_short(a.shape, a.embed) ? decode_stream_g<T, true>(a, st, kv) : decode_stream_g<T, false>(a, st, kv);
 }
-
-bool decode_is_exact(const PopeAttnArgs& a) { return a.shape.Nk < DS_EXACT_KEYS; }
 
 cudaError_t decode_stream(const PopeAttnArgs& a, cudaStream_t st) {
   return a.shape.dtype == POPE_BF16 ? decode_stream_d<__nv_bfloat16>(a, st, nullptr) : decode_stream_d<__half>(a, st, nullptr);

@@ -32,7 +32,6 @@ cudaError_t apply_qk_bwd(const PopeApplyBwdArgs& a, cudaStream_t st);
 // streaming decode (one query row, 16-bit inputs): copy-engine ring + shared-memory transform, HBM-bound
 bool decode_stream_supported(const PopeAttnArgs& a);
 size_t decode_stream_workspace(const PopeAttnArgs& a);
-bool decode_is_exact(const PopeAttnArgs& a);   // fp32 phases throughout: reported as the exact-arithmetic family
 cudaError_t decode_stream(const PopeAttnArgs& a, cudaStream_t st);
 // the same kernel over a paged key / value cache, and the append into the pages
 bool decode_paged_supported(const PopePagedDecodeArgs& a);

@@ -36,7 +36,7 @@ def test_decode_edges(b, h, hk, nk, d, r, dtype, masked, seq_first, monkeypatch)
         v[-1, :, ~mask[-1]] = float("nan")
     ins = [t.transpose(1, 2).contiguous() for t in (q, k, v)] if seq_first else [q, k, v]
     out = flash_attn_with_pope(*ins, pos_emb=emb, mask=mask, head_dimension_at_first=not seq_first)
-    assert _native.last_path() == ("decode_stream" if nk >= 1024 else "simt") and _native.device_status() == 0
+    assert _native.last_path() == "decode_stream" and _native.device_status() == 0
     out = out.transpose(1, 2) if seq_first else out
     monkeypatch.setenv("POPE_B200_FORCE_SIMT", "1")
     kc, vc = (torch.nan_to_num(t.float()) for t in (k, v))

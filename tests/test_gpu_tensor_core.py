@@ -54,11 +54,15 @@ def test_forward_tc_matches_exact_family(b, h, n, d, r, causal, masked, dtype):
 
 
 def test_short_query_blocks_take_the_exact_family():
-    q = torch.randn(1, 2, 1, 64, device=DEV, dtype=torch.bfloat16)
+    """... of two rows and more; a single row streams the keys, unless its phase table cannot be copied row by row."""
+    q = torch.randn(1, 2, 5, 64, device=DEV, dtype=torch.bfloat16)
     k = torch.randn(1, 2, 512, 64, device=DEV, dtype=torch.bfloat16)
     e = PoPE(32, heads=2)(512)
-    _native.attn_forward(q, k, k, e.freqs.to(DEV), e.bias.detach().to(DEV), None, False, 0.125)
-    assert _native.last_path() == "simt"
+    freqs, bias = e.freqs.to(DEV), e.bias.detach().to(DEV)
+    apart = torch.empty(512, 40, device=DEV)[:, :32].copy_(freqs)
+    for rows, table, path in ((5, freqs, "simt"), (2, freqs, "simt"), (1, apart, "simt"), (1, freqs, "decode_stream")):
+        _native.attn_forward(q[:, :, :rows], k, k, table, bias, None, False, 0.125)
+        assert _native.last_path() == path, (rows, path)
 
 
 def _bwd(do, q, k, v, out, lse, emb, mask, causal, force_simt, want_dfreqs=True):
