@@ -244,10 +244,6 @@ def _s3(t: torch.Tensor) -> Stride3:
     return Stride3(s[0], s[1], s[2])
 
 
-def _inner_contig(t: torch.Tensor) -> torch.Tensor:
-    return t if t.shape[-1] <= 1 or t.stride(-1) == 1 else t.contiguous()
-
-
 def _freq_strides(freqs: torch.Tensor) -> Stride3:
     """(batch, head, row) strides with 0 = broadcast.  A 4-D table is (b, h, n, r), the layout
     apply_pope_to_qk and the similarity kernel of the reference use
@@ -262,28 +258,15 @@ def _freq_strides(freqs: torch.Tensor) -> Stride3:
     raise ValueError("freqs must have 2, 3 or 4 dimensions")
 
 
-def _prep_embed(freqs: torch.Tensor, bias: torch.Tensor, nk: int, r: int):
-    freqs = _inner_contig(freqs.float()) if freqs.dtype != torch.float32 else _inner_contig(freqs)
-    bias = _inner_contig(bias.float()) if bias.dtype != torch.float32 else _inner_contig(bias)
-    assert freqs.shape[-2] == nk or r == 0, "freqs must have one row per key position"
-    return freqs, bias
-
-
 def _attached(freqs):
     """The factors riding on a table built by PoPE / AxialPoPE, unchecked (the binding looks at them)."""
     return getattr(freqs, "_pope_factored", None)
 
 
 def _factors_of(freqs):
-    """(positions, inv_freqs, axis_of) riding on a table built by PoPE / AxialPoPE, when usable as is."""
+    """(positions, inv_freqs, axis_of) riding on a table, when the binding uses them in its place."""
     f = _attached(freqs)
-    if f is None or freqs.ndim != 2:
-        return None
-    pos, inv, axis = f
-    ok = (pos.device == freqs.device and inv.device == freqs.device and pos.dtype == torch.float32 and inv.dtype == torch.float32
-          and pos.shape[0] == freqs.shape[0] and inv.numel() == freqs.shape[1] and pos.stride(-1) == 1 and inv.is_contiguous()
-          and (axis is None or (axis.device == freqs.device and axis.dtype == torch.int32 and axis.is_contiguous())))
-    return f if ok else None
+    return f if f is not None and _ops().factors_usable(f, freqs) else None
 
 
 def _embed_struct(freqs, bias, r, factors=None) -> Embed:
@@ -300,15 +283,6 @@ def _shape(q, k, r) -> Shape:
     b, h, nq, d = q.shape
     hk, nk = k.shape[1], k.shape[2]
     return Shape(b, h, hk, nq, nk, d, r, _DTYPES[q.dtype])
-
-
-def _workspace(op: int, args, device) -> Optional[torch.Tensor]:
-    need = load_library().pope_b200_workspace_bytes(op, C.addressof(args))
-    if need == 0:
-        return None
-    ws = torch.empty(need, dtype=torch.uint8, device=device)
-    args.workspace, args.workspace_bytes = ws.data_ptr(), need
-    return ws
 
 
 def _mask_u8(mask: Optional[torch.Tensor]):

@@ -15,7 +15,9 @@
 //     shared memory set the pace.)
 //   * small grids are cut along the streamed operand: a cluster of 2 or 4 CTAs shares a tile, each takes a part of the
 //     stream, and the partial accumulators meet in distributed shared memory.
-// Measured at (1, 8, 1024, 64), r = 64, causal, fp32: see the table at the launch functions.
+// Measured at (1, 8, 1024, 64), r = 64, causal, fp32, a whole training step: 1131 us with the kernels of simt_attn.cu, 609 in tiles
+// with 4 x 4 scores per thread, 341 with 4 x 8 and clusters, 337 with the images of a tile dealt over several CTAs (80 us at the
+// nominal fp32 rate).
 //
 // Semantics: PoPE_pytorch/triton_pope_flash_attn.py:23-218 (top-left causal mask, bottom-right positions, mask True = keep,
 // zero output and -inf LSE for empty rows).

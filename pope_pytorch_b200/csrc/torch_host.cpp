@@ -1,8 +1,9 @@
 // torch binding of libpope_b200.so: output and workspace allocation, argument structs and the autograd nodes.
 //
 // What a call costs on the host decides the small shapes.  The same layer written in Python over ctypes took 45 us per
-// (2, 8, 1024, 64) forward whose kernels take 26 us and, with its backward in a Python autograd node on the engine's thread,
-// 351 us per (3, 8 / 2, 777, 64) training step whose kernels take 159 us; here they take 27 and 148 us.  The kernels themselves stay behind
+// (2, 8, 1024, 64) forward whose kernels then took 26 us and, with its backward in a Python autograd node on the engine's thread,
+// 351 us per (3, 8 / 2, 777, 64) training step whose kernels took 159 us; here they took 27 and 148 us (with the kernels since
+// then: 21 us, bound by the GPU, and 142 us around about 100 us of kernels).  The kernels themselves stay behind
 // the C ABI (include/pope_b200.h): this file only fills its structs.  No arithmetic happens here and nothing is kept from one
 // call to the next.
 #include <ATen/TensorSubclassLikeUtils.h>
@@ -523,6 +524,7 @@ std::tuple<Tensor, Tensor> kv_decode(const Pages& p, const Tensor& q_, const Ten
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("factors_usable", &factors_usable);
   m.def("flash_attn", &flash_attn);
   m.def("similarity", &similarity);
   m.def("apply_qk", &apply_qk);
