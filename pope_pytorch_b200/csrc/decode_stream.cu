@@ -551,8 +551,20 @@ static int decode_heads(const PopeShape& s) {
   return groups % 4 == 0 && s.d != 96 ? 4 : groups % 2 == 0 ? 2 : 1;
 }
 
-// CTAs resident at a time: two per SM with 8 worker warps, one with 16 (four heads per CTA)
-static int64_t decode_slots(const PopeShape& s) { return (decode_heads(s) == 4 ? 1 : 2) * 148; }
+// Shared memory of a CTA: a ring stage, and everything beside the ring (but the paged cache's page indices)
+static size_t decode_stage_bytes(const PopeShape& s) { return (size_t)DS_TILE * (2 * s.d * 2 + 2 * s.r * 2); }
+static size_t decode_fixed_bytes(const PopeShape& s, int g, int nw) {
+  return ((2 + nw) * g * s.d + nw * g * 2 + g * DS_MAX_SPLIT) * sizeof(float) + 2 * 3 * 8 + 64;
+}
+constexpr size_t DS_HALF_SM = 112 * 1024;   // what a CTA may take where two share an SM
+
+// CTAs resident at a time: two per SM with 8 worker warps, one with 16 (four heads per CTA), and one where two stages of wide
+// rotations do not fit half of the shared memory (counted as two, (1, 8, 30000, 128), r = 128 took 76 us instead of 69,
+// (2, 16, 700, 128) 18.5 instead of 12.4)
+static int64_t decode_slots(const PopeShape& s) {
+  const bool two = decode_heads(s) < 4 && 2 * decode_stage_bytes(s) + decode_fixed_bytes(s, decode_heads(s), 8) <= DS_HALF_SM;
+  return (two ? 2 : 1) * 148;
+}
 
 // Key ranges per unit.  The time of a grid in units of one 64-key tile: whole waves of resident CTAs times the tiles of a CTA
 // plus what a CTA costs beside its tiles (start, ring fill, merge: about four tiles' time); the smallest wins.  SHORT: at
@@ -651,11 +663,9 @@ static cudaError_t launch_decode_stream(const PopeAttnArgs& a, cudaStream_t st, 
   p.ch = ch, p.sh = sh;
   p.status = tc_status_ptr();
   if (!p.status) return cudaErrorInvalidSymbol;
-  const size_t stage = (size_t)DS_TILE * (2 * D * 2 + 2 * s.r * 2);
-  const size_t fixed = ((2 + NW) * G * D + NW * G * 2 + G * DS_MAX_SPLIT) * sizeof(float) + 2 * 3 * 8 + 64 +
-                       (size_t)p.npg_smem * sizeof(int);
+  const size_t stage = decode_stage_bytes(s), fixed = decode_fixed_bytes(s, G, NW) + (size_t)p.npg_smem * sizeof(int);
   // two CTAs per SM: the ring of each takes what half of the shared memory leaves, at most 3 stages
-  int nst = (int)(((NW == 8 ? 112 : 224) * 1024 - (int64_t)fixed) / (int64_t)stage);
+  int nst = (int)(((NW == 8 ? 1 : 2) * (int64_t)DS_HALF_SM - (int64_t)fixed) / (int64_t)stage);
   if (nst < 2) nst = (int)((kMaxDynamicSmem - 1024 - (int64_t)fixed) / (int64_t)stage);   // wide rotations (r = d = 128): one CTA per SM
   nst = nst > 3 ? 3 : nst;
   if (nst < 2) return cudaErrorInvalidValue;

@@ -641,7 +641,10 @@ class ForkGuard {
 // longer than that of a dq block, which runs beside it.  Whole training steps as a graph, d = 64 to 128, on 1 / 2 / 4 CTAs:
 // (1, 8 / 2, 2048) 242 / 172 / 140 us, (2, 8 / 2, 1024) 178 / 138 / 123, (1, 32 / 4, 500) 144 / 113 / 94, and the kernel of
 // (3, 8 / 2, 777) 68 / 43 / 42.  Without groups the sweep is no longer than dq's and the merge costs more than it gives:
-// (1, 8, 1024) 71 / 74 / 81, (2, 8, 600) 61 / 62 / 75.  Above 172 CTAs the blocks fill the chip by themselves.
+// (1, 8, 1024) 71 / 74 / 81, (2, 8, 600) 61 / 62 / 75.  Up to 172 CTAs, a little over one round of 148 SMs, a further cut does
+// not cost a second round.  Beyond that it depends on the length of a sweep, which this rule does not look at: backward calls with
+// the sweep cut once more against the rule, (4, 8 / 2, 777) 74 / 70 us, (2, 16 / 4, 1024, 128) 111 / 107, (4, 8 / 2, 1024) 89 / 88,
+// but (2, 8 / 2, 2048, 128) 170 / 182 and (1, 16 / 4, 4096, 128) 419 / 500.
 static int dkdv_split(const PopeShape& s) {
   const int64_t ctas = (int64_t)((s.Nk + BQ - 1) / BQ) * s.B * s.Hk;
   int split = 1;
